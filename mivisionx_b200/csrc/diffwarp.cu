@@ -12,9 +12,10 @@
 // floor(xs), floor(ys); each of the four taps outside the source reads the border value.
 //
 // Adjoint: d/dsrc scatters gout times the tap weights (red.global.add on the source
-// gradient); d/dtheta sums gout * (dout/dxs * dxs/dtheta + dout/dys * dys/dtheta) with
-// double sums per warp and block (atomicAdd double per block and image).
+// gradient); d/dtheta sums gout * (dout/dxs * dxs/dtheta + dout/dys * dys/dtheta) in double
+// per thread, warp and block (atomicAdd double per block and image).
 #include "agocuda_internal.cuh"
+#include <limits.h>
 
 uint64_t agocuda_count_launch(unsigned n);
 
@@ -50,36 +51,120 @@ __device__ __forceinline__ Taps taps(const float *src, int stride, int W, int H,
     return t;
 }
 
+// floor(v) of a position inside a source of n columns (or rows) without the double-to-int
+// conversions and FRND: v + 1.5 * 2^52 rounded down holds floor(v) in its low word, and its
+// high word is 0x43380000 exactly for 0 <= floor(v) < 2^32 (any other value, an infinity or
+// a NaN has another one).  Returns whether both taps floor(v), floor(v) + 1 lie inside.
+__device__ __forceinline__ bool floor_inside(double v, int n, int &i, float &f)
+{
+    const double magic = 6755399441055744.0;
+    const double t = __dadd_rd(v, magic);
+    i = __double2loint(t);
+    f = (float)(v - (t - magic));
+    return __double2hiint(t) == 0x43380000 && (unsigned)i < (unsigned)(n - 1);
+}
+
+// One sample: the taps, and in `key` the element index of the first tap where all four lie
+// inside a source of fewer than 2^31 elements (`wide` is false), else kNoKey with the tap
+// flags in t.
+constexpr int kNoKey = INT_MIN;
+struct Sample { Taps t; int key; };
+
+__device__ __forceinline__ Sample sample(const float *src, int stride, int W, int H, double xs, double ys, float border,
+                                         bool wide)
+{
+    Sample s;
+    const bool inx = floor_inside(xs, W, s.t.x0, s.t.fx), iny = floor_inside(ys, H, s.t.y0, s.t.fy);
+    if (inx && iny && !wide) {
+        s.key = s.t.y0 * stride + s.t.x0;
+        const float *p = src + s.key;
+        s.t.p00 = __ldg(p); s.t.p01 = __ldg(p + 1);
+        s.t.p10 = __ldg(p + stride); s.t.p11 = __ldg(p + stride + 1);
+        s.t.k00 = s.t.k01 = s.t.k10 = s.t.k11 = true;
+    } else {
+        s.t = taps(src, stride, W, H, xs, ys, border);
+        s.key = kNoKey;
+    }
+    return s;
+}
+
+// The scatter of a warp that walks down the rows of a 32-column strip.  One atomic per tap is
+// what bounds the adjoint (4 per pixel); neighbouring samples mostly share taps, so a lane
+// keeps its lower two contributions until the next row, where they join the upper two if the
+// addresses agree, and hands its right-hand contribution to the lane whose left-hand one has
+// that address.  Near a unit-scale map about 1.7 atomics per pixel are left.  Any map is
+// right: contributions join only where their addresses are equal.
+struct Scatter {
+    int key = kNoKey;          // address of the contributions kept from the row above
+    float v0 = 0.f, v1 = 0.f;
+
+    // all lanes of the warp take part; a lane without a sample passes key kNoKey and g 0
+    __device__ __forceinline__ void row(float *gsrc, int stride, const Sample &s, float g, bool has)
+    {
+        const Taps &t = s.t;
+        const float gu = g * (1.f - t.fx), gr = g * t.fx;
+        float c00 = gu * (1.f - t.fy), c01 = gr * (1.f - t.fy);
+        const float c10 = gu * t.fy, c11 = gr * t.fy;
+        const int k = s.key;
+        if (key != kNoKey) {
+            if (key == k) {
+                c00 += v0;
+                c01 += v1;
+            } else {
+                atomicAdd(gsrc + key, v0);
+                atomicAdd(gsrc + key + 1, v1);
+            }
+        }
+        const int lane = threadIdx.x & 31;
+        const int ku = __shfl_up_sync(0xffffffffu, k, 1), kd = __shfl_down_sync(0xffffffffu, k, 1);
+        const float cu = __shfl_up_sync(0xffffffffu, c01, 1);
+        key = kNoKey;
+        if (k != kNoKey) {
+            if (lane > 0 && ku == k - 1) c00 += cu;
+            atomicAdd(gsrc + k, c00);
+            if (lane == 31 || kd != k + 1) atomicAdd(gsrc + k + 1, c01);
+            key = k + stride;
+            v0 = c10;
+            v1 = c11;
+        } else if (has) {
+            float *p = gsrc + (long long)t.y0 * stride + t.x0;
+            if (t.k00) atomicAdd(p, c00);
+            if (t.k01) atomicAdd(p + 1, c01);
+            if (t.k10) atomicAdd(p + stride, c10);
+            if (t.k11) atomicAdd(p + stride + 1, c11);
+        }
+    }
+    __device__ __forceinline__ void flush(float *gsrc)
+    {
+        const int lane = threadIdx.x & 31;
+        const int ku = __shfl_up_sync(0xffffffffu, key, 1), kd = __shfl_down_sync(0xffffffffu, key, 1);
+        const float cu = __shfl_up_sync(0xffffffffu, v1, 1);
+        if (key == kNoKey) return;
+        atomicAdd(gsrc + key, lane > 0 && ku == key - 1 ? v0 + cu : v0);
+        if (lane == 31 || kd != key + 1) atomicAdd(gsrc + key + 1, v1);
+    }
+};
+
 __device__ __forceinline__ float interp(const Taps &t)
 {
     return (t.p00 * (1.f - t.fx) + t.p01 * t.fx) * (1.f - t.fy) + (t.p10 * (1.f - t.fx) + t.p11 * t.fx) * t.fy;
 }
 
-// scatter g times the tap weights into the source gradient
-__device__ __forceinline__ void scatter(float *gsrc, int stride, const Taps &t, float g)
-{
-    if (t.k00) atomicAdd(gsrc + (size_t)t.y0 * stride + t.x0, g * (1.f - t.fx) * (1.f - t.fy));
-    if (t.k01) atomicAdd(gsrc + (size_t)t.y0 * stride + t.x0 + 1, g * t.fx * (1.f - t.fy));
-    if (t.k10) atomicAdd(gsrc + (size_t)(t.y0 + 1) * stride + t.x0, g * (1.f - t.fx) * t.fy);
-    if (t.k11) atomicAdd(gsrc + (size_t)(t.y0 + 1) * stride + t.x0 + 1, g * t.fx * t.fy);
-}
-
 __device__ __forceinline__ float dout_dxs(const Taps &t) { return (1.f - t.fy) * (t.p01 - t.p00) + t.fy * (t.p11 - t.p10); }
 __device__ __forceinline__ float dout_dys(const Taps &t) { return (1.f - t.fx) * (t.p10 - t.p00) + t.fx * (t.p11 - t.p01); }
 
-// block reduction of N per-thread terms into double atomics at dst[0..N), summed in double
-// from the first addition (the theta gradient cancels strongly across pixels)
+// block reduction of N per-thread double sums into double atomics at dst[0..N)
 template <int N>
-__device__ __forceinline__ void block_add(const float (&v)[N], double *dst)
+__device__ __forceinline__ void block_add(const double (&v)[N], double *dst)
 {
     __shared__ double red[N][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int k = 0; k < N; k++) {
-        double s = (double)v[k];
+        double s = v[k];
 #pragma unroll
         for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) red[k][warp] = (double)s;
+        if (lane == 0) red[k][warp] = s;
     }
     __syncthreads();
     if (threadIdx.x < N) {
@@ -97,85 +182,138 @@ struct Img32 {
 
 enum Mode { kForward = 0, kAdjoint = 1, kFusedL2 = 2 };
 
-// One thread per output pixel of image blockIdx.z.  Modes: forward (out), adjoint (gout ->
-// gsrc, gtheta), fused L2 step (target -> gsrc, gtheta and loss with gout = 2 (out - target)).
-// NT = 6: affine; NT = 9: perspective.  Per image the adjoint adds NT theta gradients, the
-// fused step NT gradients and then the loss.
+// Warps of image blockIdx.z.  Modes: forward (out), adjoint (gout -> gsrc, parameter
+// gradient), fused L2 step (target -> gsrc, gtheta and loss with gout = 2 (out - target)).
+// NT = 6: affine; NT = 9: perspective; NT = 2: displacement field (the gradient is a field).
+// Per image the adjoint adds NT theta gradients, the fused step NT gradients and then the loss.
+//
+// A warp owns a strip of 32 columns and `rows` rows and walks down it, the taps of the next
+// row loaded while a row is worked on.  Per pixel a thread adds 2 (affine) or 6 terms to
+// double sums of its own; x is fixed per thread, so sum(g x) is x sum(g), and the sums meet
+// across lanes once per strip instead of once per pixel (7 double butterflies per pixel were
+// the larger half of the fused step).  Affine L2 step of 32 x 1024^2: 573 us with one pixel per
+// thread, 278 us so; issue-bound (77 % of the issue slots).  `rows` is 16 where the batch fills the device with
+// such strips and less where it does not (warp_rows).
 template <int MODE, int NT>
 __global__ void __launch_bounds__(256)
-k_warp_f32(int W, int H, Img32 src, Img32 out, Img32 aux, const float *theta, float border, Img32 gsrc, double *gtheta)
+k_warp_f32(int W, int H, int rows, Img32 src, Img32 out, Img32 aux, const float *par, long long parBatch, int parStride,
+           float border, Img32 gsrc, void *gpar)
 {
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5), n = blockIdx.z;
-    const float *th = theta + NT * n;
-    float acc[NT + 1];
+    const int x = blockIdx.x * 32 + (threadIdx.x & 31), n = blockIdx.z;
+    const int yA = (blockIdx.y * 8 + (threadIdx.x >> 5)) * rows, yB = min(yA + rows, H);
+    const bool act = x < W;
+    const float *sp = src.p + src.batch * n;
+    float *gp = MODE == kForward ? nullptr : gsrc.p + gsrc.batch * n;
+    const bool wide = (long long)src.stride * src.H > 0x7fffffffll;
+    const float *th = NT == 2 ? nullptr : par + NT * n;
+    const float2 *field = NT == 2 ? (const float2 *)par + parBatch * n : nullptr;
+    float2 *gfield = NT == 2 && MODE == kAdjoint ? (float2 *)gpar + parBatch * n : nullptr;
+    // the parts of the map that do not depend on y (products of 24-bit factors: exact)
+    double mx[3] = {}, my[3] = {}, m0[3] = {};
+    if (NT != 2) {
+        constexpr int D = NT == 9 ? 3 : 2;
 #pragma unroll
-    for (int k = 0; k <= NT; k++) acc[k] = 0.f;
-    if (x < W && y < H) {
-        const float fx = (float)x, fy = (float)y;
-        double xs, ys, iz = 1.0;
-        if (NT == 6) {
-            xs = (double)th[0] * x + (double)th[2] * y + (double)th[4];
-            ys = (double)th[1] * x + (double)th[3] * y + (double)th[5];
-        } else {
-            const double z = (double)th[2] * x + (double)th[5] * y + (double)th[8];
-            iz = z != 0.0 ? 1.0 / z : 0.0;
-            xs = z != 0.0 ? ((double)th[0] * x + (double)th[3] * y + (double)th[6]) * iz : __longlong_as_double(0x7ff8000000000000ll);
-            ys = z != 0.0 ? ((double)th[1] * x + (double)th[4] * y + (double)th[7]) * iz : xs;
-        }
-        const Taps t = taps(src.p + src.batch * n, src.stride, src.W, src.H, xs, ys, border);
-        if (MODE == kForward) {
-            out.p[out.batch * n + (size_t)y * out.stride + x] = interp(t);
-        } else {
-            float g;
-            if (MODE == kAdjoint) {
-                g = aux.p[aux.batch * n + (size_t)y * aux.stride + x];
-            } else {
-                const float r = interp(t) - aux.p[aux.batch * n + (size_t)y * aux.stride + x];
-                acc[NT] = r * r;
-                g = 2.f * r;
-            }
-            scatter(gsrc.p + gsrc.batch * n, gsrc.stride, t, g);
-            const float gx = g * dout_dxs(t), gy = g * dout_dys(t);
-            if (NT == 6) {
-                acc[0] = gx * fx; acc[1] = gy * fx; acc[2] = gx * fy; acc[3] = gy * fy; acc[4] = gx; acc[5] = gy;
-            } else if (iz != 0.0 && (gx != 0.f || gy != 0.f)) {   // a sample on the border has no theta term
-                // d(xs)/d(m00, m10, m20) = (x, y, 1) / z; d(xs)/d(m02, m12, m22) = -xs (x, y, 1) / z; same for ys
-                const double gxz = gx * iz, gyz = gy * iz, q = -((double)gx * xs + (double)gy * ys) * iz;
-                acc[0] = (float)(gxz * x); acc[1] = (float)(gyz * x); acc[2] = (float)(q * x);
-                acc[3] = (float)(gxz * y); acc[4] = (float)(gyz * y); acc[5] = (float)(q * y);
-                acc[6] = (float)gxz; acc[7] = (float)gyz; acc[8] = (float)q;
-            }
+        for (int k = 0; k < D; k++) {
+            mx[k] = (double)th[k] * x;
+            my[k] = (double)th[D + k];
+            m0[k] = (double)th[2 * D + k];
         }
     }
-    if (MODE == kAdjoint) {
-        float v[NT];
+    struct Pos { double xs, ys, iz; };
+    auto position = [&](int y) -> Pos {
+        if (NT == 2) {
+            const float2 d = act ? field[(size_t)y * parStride + x] : make_float2(0.f, 0.f);
+            return {(double)x + d.x, (double)y + d.y, 1.0};
+        }
+        const double xn = mx[0] + my[0] * y + m0[0], yn = mx[1] + my[1] * y + m0[1];
+        if (NT == 6) return {xn, yn, 1.0};
+        const double z = mx[2] + my[2] * y + m0[2];
+        if (z == 0.0) { const double nan = __longlong_as_double(0x7ff8000000000000ll); return {nan, nan, 0.0}; }
+        const double iz = 1.0 / z;
+        return {xn * iz, yn * iz, iz};
+    };
+    if constexpr (MODE == kForward) {
+        if (!act) return;
+        float *o = out.p + out.batch * n + x;
+        for (int y = yA; y < yB; y += 2) {                 // two rows at a time: their loads overlap
+            const Pos p = position(y), q = position(min(y + 1, yB - 1));
+            const Sample a = sample(sp, src.stride, src.W, src.H, p.xs, p.ys, border, wide);
+            const Sample b = sample(sp, src.stride, src.W, src.H, q.xs, q.ys, border, wide);
+            o[(size_t)y * out.stride] = interp(a.t);
+            if (y + 1 < yB) o[(size_t)(y + 1) * out.stride] = interp(b.t);
+        }
+        return;
+    }
+    constexpr int NS = NT == 2 ? 1 : NT + (MODE == kFusedL2 ? 1 : 0);
+    double sum[NS] = {};
+    Scatter sc;
+    const float *ap = aux.p + aux.batch * n + x;
+    auto load = [&](int y, Pos &p, Sample &s, float &a) {
+        if (act && y < yB) {
+            p = position(y);
+            a = __ldg(ap + (size_t)y * aux.stride);
+            s = sample(sp, src.stride, src.W, src.H, p.xs, p.ys, border, wide);
+        } else {
+            s = Sample{};
+            s.key = kNoKey;
+            a = 0.f;
+        }
+    };
+    Pos p, pn;
+    Sample s, sn;
+    float a, an;
+    load(yA, p, s, a);
+    for (int y = yA; y < yB; y++) {
+        load(y + 1, pn, sn, an);
+        const Taps &t = s.t;
+        float g = a;
+        if (MODE == kFusedL2) {
+            const float r = act ? interp(t) - a : 0.f;
+            sum[NS - 1] += (double)r * r;
+            g = 2.f * r;
+        }
+        sc.row(gp, gsrc.stride, s, g, act);
+        const float gx = g * dout_dxs(t), gy = g * dout_dys(t);
+        if (NT == 2) {
+            if (act) gfield[(size_t)y * parStride + x] = make_float2(gx, gy);
+        } else if (NT == 6) {
+            const double dx = gx, dy = gy;
+            sum[4 % NS] += dx;
+            sum[5 % NS] += dy;
+            sum[2 % NS] += dx * y;
+            sum[3 % NS] += dy * y;
+        } else if (act && p.iz != 0.0 && (gx != 0.f || gy != 0.f)) {   // a sample on the border has no theta term
+            // d(xs)/d(m00, m10, m20) = (x, y, 1) / z; d(xs)/d(m02, m12, m22) = -xs (x, y, 1) / z; same for ys
+            const double gxz = gx * p.iz, gyz = gy * p.iz, q = -((double)gx * p.xs + (double)gy * p.ys) * p.iz;
+            sum[6 % NS] += gxz;
+            sum[7 % NS] += gyz;
+            sum[8 % NS] += q;
+            sum[3 % NS] += gxz * y;
+            sum[4 % NS] += gyz * y;
+            sum[5 % NS] += q * y;
+        }
+        p = pn; s = sn; a = an;
+    }
+    sc.flush(gp);
+    if constexpr (NT != 2) {
+        constexpr int D = NT == 9 ? 3 : 2;
 #pragma unroll
-        for (int k = 0; k < NT; k++) v[k] = acc[k];
-        block_add<NT>(v, gtheta + NT * n);
-    } else if (MODE == kFusedL2) {
-        block_add<NT + 1>(acc, gtheta + (NT + 1) * n);
+        for (int k = 0; k < D; k++) sum[k] = sum[2 * D + k] * x;
+        block_add<NS>(sum, (double *)gpar + NS * n);
     }
 }
 
-// Remap: sample at (x + field[y][x].x, y + field[y][x].y); the adjoint writes gfield per pixel.
-template <int MODE>
-__global__ void __launch_bounds__(256)
-k_remap_f32(int W, int H, Img32 src, Img32 out, Img32 aux, const float2 *field, long long fieldBatch, int fieldStride,
-            float border, Img32 gsrc, float2 *gfield)
+// Rows per warp: `most` where the strips still give every SM 32 warps (its latency hiding),
+// halved until they do.
+int warp_rows(int n, int W, int H, int most)
 {
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5), n = blockIdx.z;
-    if (x >= W || y >= H) return;
-    const size_t fi = fieldBatch * n + (size_t)y * fieldStride + x;
-    const float2 d = field[fi];
-    const Taps t = taps(src.p + src.batch * n, src.stride, src.W, src.H, (double)x + d.x, (double)y + d.y, border);
-    if (MODE == kForward) {
-        out.p[out.batch * n + (size_t)y * out.stride + x] = interp(t);
-    } else {
-        const float g = aux.p[aux.batch * n + (size_t)y * aux.stride + x];
-        scatter(gsrc.p + gsrc.batch * n, gsrc.stride, t, g);
-        gfield[fi] = make_float2(g * dout_dxs(t), g * dout_dys(t));
-    }
+    const long long want = 32ll * agocuda_sm_count();
+    int r = most;
+    while (r > 1 && (long long)n * div_up(W, 32) * div_up(H, r) < want) r >>= 1;
+    return r;
 }
+
+dim3 warp_grid(int n, int W, int H, int rows) { return dim3(div_up(W, 32), div_up(H, 8 * rows), n); }
 
 Img32 img32(const float *p, long long batch, int stride, int W, int H) { return Img32{(float *)p, batch, stride, W, H}; }
 
@@ -194,10 +332,10 @@ extern "C" int agocuda_WarpAffine_F32_Bilinear_Constant_batch(void *stream, int 
 {
     if (!pDst || !pSrc || !theta || !batch_ok(n, W, H, srcW, srcH) || dstStride < W || srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const dim3 grd(div_up(W, 32), div_up(H, 8), n);
-    k_warp_f32<kForward, 6><<<grd, 256, 0, as_stream(stream)>>>(
-        W, H, img32(pSrc, srcBatch, srcStride, srcW, srcH), img32(pDst, dstBatch, dstStride, W, H), Img32{}, theta, border,
-        Img32{}, nullptr);
+    const int rows = warp_rows(n, W, H, 4);
+    k_warp_f32<kForward, 6><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
+        W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), img32(pDst, dstBatch, dstStride, W, H), Img32{}, theta, 0, 0,
+        border, Img32{}, nullptr);
     agocuda_count_launch(1);
     return agocuda_launch_status();
 }
@@ -211,10 +349,10 @@ extern "C" int agocuda_WarpAffine_F32_Bilinear_Constant_adjoint_batch(void *stre
     if (!pGradOut || !pSrc || !theta || !pGradSrc || !pGradTheta || !batch_ok(n, W, H, srcW, srcH) || goStride < W ||
         srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const dim3 grd(div_up(W, 32), div_up(H, 8), n);
-    k_warp_f32<kAdjoint, 6><<<grd, 256, 0, as_stream(stream)>>>(
-        W, H, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pGradOut, goBatch, goStride, W, H), theta, border,
-        img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradTheta);
+    const int rows = warp_rows(n, W, H, 16);
+    k_warp_f32<kAdjoint, 6><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
+        W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pGradOut, goBatch, goStride, W, H), theta, 0, 0,
+        border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradTheta);
     agocuda_count_launch(1);
     return agocuda_launch_status();
 }
@@ -227,10 +365,10 @@ extern "C" int agocuda_WarpAffine_F32_L2_step_batch(void *stream, int n, int W, 
     if (!pTarget || !pSrc || !theta || !pGradSrc || !pGradThetaLoss || !batch_ok(n, W, H, srcW, srcH) || tStride < W ||
         srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const dim3 grd(div_up(W, 32), div_up(H, 8), n);
-    k_warp_f32<kFusedL2, 6><<<grd, 256, 0, as_stream(stream)>>>(
-        W, H, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pTarget, tBatch, tStride, W, H), theta, border,
-        img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradThetaLoss);
+    const int rows = warp_rows(n, W, H, 16);
+    k_warp_f32<kFusedL2, 6><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
+        W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pTarget, tBatch, tStride, W, H), theta, 0, 0,
+        border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradThetaLoss);
     agocuda_count_launch(1);
     return agocuda_launch_status();
 }
@@ -243,10 +381,10 @@ extern "C" int agocuda_Remap_F32_Bilinear_Constant_batch(void *stream, int n, in
     if (!pDst || !pSrc || !pField || !batch_ok(n, W, H, srcW, srcH) || dstStride < W || srcStride < srcW ||
         fieldStride < W || ((uintptr_t)pField & 7))
         return AGOCUDA_INVALID_PARAMS;
-    const dim3 grd(div_up(W, 32), div_up(H, 8), n);
-    k_remap_f32<kForward><<<grd, 256, 0, as_stream(stream)>>>(
-        W, H, img32(pSrc, srcBatch, srcStride, srcW, srcH), img32(pDst, dstBatch, dstStride, W, H), Img32{},
-        (const float2 *)pField, fieldBatch, fieldStride, border, Img32{}, nullptr);
+    const int rows = warp_rows(n, W, H, 4);
+    k_warp_f32<kForward, 2><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
+        W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), img32(pDst, dstBatch, dstStride, W, H), Img32{}, pField,
+        fieldBatch, fieldStride, border, Img32{}, nullptr);
     agocuda_count_launch(1);
     return agocuda_launch_status();
 }
@@ -260,11 +398,10 @@ extern "C" int agocuda_Remap_F32_Bilinear_Constant_adjoint_batch(void *stream, i
     if (!pGradOut || !pSrc || !pField || !pGradSrc || !pGradField || !batch_ok(n, W, H, srcW, srcH) || goStride < W ||
         srcStride < srcW || fieldStride < W || ((uintptr_t)pField & 7) || ((uintptr_t)pGradField & 7))
         return AGOCUDA_INVALID_PARAMS;
-    const dim3 grd(div_up(W, 32), div_up(H, 8), n);
-    k_remap_f32<kAdjoint><<<grd, 256, 0, as_stream(stream)>>>(
-        W, H, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pGradOut, goBatch, goStride, W, H),
-        (const float2 *)pField, fieldBatch, fieldStride, border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH),
-        (float2 *)pGradField);
+    const int rows = warp_rows(n, W, H, 16);
+    k_warp_f32<kAdjoint, 2><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
+        W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pGradOut, goBatch, goStride, W, H),
+        pField, fieldBatch, fieldStride, border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradField);
     agocuda_count_launch(1);
     return agocuda_launch_status();
 }
@@ -276,10 +413,10 @@ extern "C" int agocuda_WarpPerspective_F32_Bilinear_Constant_batch(void *stream,
 {
     if (!pDst || !pSrc || !theta || !batch_ok(n, W, H, srcW, srcH) || dstStride < W || srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const dim3 grd(div_up(W, 32), div_up(H, 8), n);
-    k_warp_f32<kForward, 9><<<grd, 256, 0, as_stream(stream)>>>(
-        W, H, img32(pSrc, srcBatch, srcStride, srcW, srcH), img32(pDst, dstBatch, dstStride, W, H), Img32{}, theta, border,
-        Img32{}, nullptr);
+    const int rows = warp_rows(n, W, H, 4);
+    k_warp_f32<kForward, 9><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
+        W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), img32(pDst, dstBatch, dstStride, W, H), Img32{}, theta, 0, 0,
+        border, Img32{}, nullptr);
     agocuda_count_launch(1);
     return agocuda_launch_status();
 }
@@ -294,10 +431,10 @@ extern "C" int agocuda_WarpPerspective_F32_Bilinear_Constant_adjoint_batch(void 
     if (!pGradOut || !pSrc || !theta || !pGradSrc || !pGradTheta || !batch_ok(n, W, H, srcW, srcH) || goStride < W ||
         srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const dim3 grd(div_up(W, 32), div_up(H, 8), n);
-    k_warp_f32<kAdjoint, 9><<<grd, 256, 0, as_stream(stream)>>>(
-        W, H, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pGradOut, goBatch, goStride, W, H), theta, border,
-        img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradTheta);
+    const int rows = warp_rows(n, W, H, 16);
+    k_warp_f32<kAdjoint, 9><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
+        W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pGradOut, goBatch, goStride, W, H), theta, 0, 0,
+        border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradTheta);
     agocuda_count_launch(1);
     return agocuda_launch_status();
 }
@@ -310,10 +447,10 @@ extern "C" int agocuda_WarpPerspective_F32_L2_step_batch(void *stream, int n, in
     if (!pTarget || !pSrc || !theta || !pGradSrc || !pGradThetaLoss || !batch_ok(n, W, H, srcW, srcH) || tStride < W ||
         srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const dim3 grd(div_up(W, 32), div_up(H, 8), n);
-    k_warp_f32<kFusedL2, 9><<<grd, 256, 0, as_stream(stream)>>>(
-        W, H, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pTarget, tBatch, tStride, W, H), theta, border,
-        img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradThetaLoss);
+    const int rows = warp_rows(n, W, H, 16);
+    k_warp_f32<kFusedL2, 9><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
+        W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pTarget, tBatch, tStride, W, H), theta, 0, 0,
+        border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradThetaLoss);
     agocuda_count_launch(1);
     return agocuda_launch_status();
 }

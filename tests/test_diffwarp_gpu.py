@@ -172,3 +172,36 @@ def test_perspective_degenerate_rows(cuda):
     o = out.detach().cpu().numpy()[0]
     assert np.isfinite(o).all() and np.all(o[:, 32] == 0.5)
     assert torch.isfinite(tht.grad).all() and torch.isfinite(src.grad).all()
+
+
+# sizes around the 32-column, 1..16-row strips of a warp; maps whose neighbouring samples share
+# taps (unit scale), skip columns (2.5), sit on one cell (0.2), run backwards or leave the source
+@pytest.mark.parametrize("kind", ["shift", "wide", "tight", "mirror", "off"])
+@pytest.mark.parametrize("H,W", [(1, 1), (1, 40), (2, 33), (17, 31), (67, 130)])
+def test_adjoint_at_strip_edges(cuda, H, W, kind):
+    import torch
+
+    from mivisionx_b200 import diffwarp
+    rng = np.random.default_rng(H * 1000 + W)
+    n = 3
+    img = rng.random((n, H, W)).astype(np.float32)
+    tgt = rng.random((n, H, W)).astype(np.float32)
+    base = {"shift": [1, 0, 0, 1, 0.3, -0.4], "wide": [2.5, 0.1, -0.1, 2.5, -3.2, 1.1], "tight": [0.2, 0, 0, 0.2, 1.1, 0.6],
+            "mirror": [-1, 0, 0, -1, W - 1.25, H - 1.75], "off": [1, 0, 0, 1, W - 2.5, -H + 1.5]}[kind]
+    theta = np.array([base, base, [1.01, 0.02, -0.02, 0.99, 0.1, 0.2]], np.float32)
+    d = [torch.from_numpy(a).cuda() for a in (img, theta, tgt)]
+    loss, gsrc, gth = diffwarp.warp_affine_l2_step(*d)
+    field = torch.from_numpy(rng.uniform(-3, 3, (n, H, W, 2)).astype(np.float32)).cuda().requires_grad_(True)
+    src = d[0].clone().requires_grad_(True)
+    (diffwarp.remap(src, field) * d[2]).sum().backward()
+    for i in range(n):
+        _, l, gs, gt = fp64(img, theta, tgt, i)
+        assert abs(float(loss[i]) - l) <= 1e-5 * max(l, 1e-6)
+        # float residuals and derivatives (1e-6 of a term), each term at most the size of the sum's scale
+        scale = 4 * H * W * max(H, W)
+        assert np.abs(gth[i].cpu().numpy() - gt).max() <= 1e-6 * scale
+        assert np.abs(gsrc[i].cpu().numpy() - gs).max() <= 1e-5 * max(np.abs(gs).max(), 1.0)
+        f = field[i].detach().cpu().numpy().astype(np.float64)
+        gs, gf = D.remap_adjoint(img[i].astype(np.float64), f, tgt[i].astype(np.float64))
+        assert np.abs(src.grad[i].cpu().numpy() - gs).max() <= 1e-5 * max(np.abs(gs).max(), 1.0)
+        assert np.abs(field.grad[i].cpu().numpy() - gf).max() <= 1e-5 * max(np.abs(gf).max(), 1.0)
