@@ -236,3 +236,29 @@ def test_engine_motion_graph(cuda, flags):
                 np.testing.assert_array_equal(got[4:h - 4, 4:w - 4], want[4:h - 4, 4:w - 4])
     finally:
         api.vxReleaseContext(C.byref(C.c_void_p(ctx)))
+
+
+# runs of 0 / 255 values, which the fused kernel keeps on bit planes: begun by a threshold of the
+# input, of an element-wise result or of each stencil's, with both threshold kinds at the ends of
+# their range, thresholds and Not inside the run, and byte ops after it
+BIT_RUNS = {
+    "from_input": [("thr", 100), ("dilate",), ("median",), ("erode",)],
+    "from_elementwise": [("absdiff", 0), ("range", 10, 90), ("median",), ("not",), ("dilate",)],
+    "from_gauss": [("gauss",), ("range", 60, 180), ("erode",), ("thr", 3), ("dilate",), ("and", 1)],
+    "from_box": [("box",), ("thr", 0), ("not",), ("median",), ("box",)],
+    "from_median": [("median",), ("thr", 254), ("dilate",), ("gauss",), ("thr", 20), ("median",)],
+    "from_dilate": [("dilate",), ("range", 0, 255), ("median",), ("xor", 1), ("thr", 200), ("erode",)],
+    "never": [("erode",), ("thr", 255), ("dilate",), ("range", 0, 0), ("median",)],
+    "thresholds_inside": [("thr", 90), ("median",), ("thr", 255), ("not",), ("erode",), ("range", 0, 254), ("add", 0, SAT)],
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["tma", "cp_async"])
+@pytest.mark.parametrize("name", sorted(BIT_RUNS))
+def test_engine_bit_runs(cuda, name, form):
+    sizes = [(640, 360), (37, 21), (128, 64), (129, 67), (271, 130), (16, 9)]
+    frames = _frames(sizes, seed=11 * len(name))
+    res, plan = run_chains(V.OpenVX(), BIT_RUNS[name], frames, flags=FORMS[form])
+    _check(res, BIT_RUNS[name], frames)
+    assert [s for s, _ in plan] == [f"fused_PixelChain x{len(sizes)}"], plan
