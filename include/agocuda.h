@@ -417,6 +417,15 @@ int agocuda_fused_CannyEdgeDetector_3x3_L1(void *stream, uint32_t width, uint32_
                                            uint16_t hystLower, uint16_t hystUpper,
                                            void *scratch, size_t scratchBytes, uint32_t *pStatus);
 
+/* The other gradients (3x3 with l2Norm, 5x5 and 7x7 with either norm): the gradient plane goes
+ * through scratch, then as above.  hystLower / hystUpper as the suppression kernel takes them
+ * (7x7: already divided by 4).  Scratch: the _NxN_scratch_size bytes. */
+size_t agocuda_fused_CannyEdgeDetector_NxN_scratch_size(uint32_t width, uint32_t height);
+int agocuda_fused_CannyEdgeDetector_NxN(void *stream, uint32_t width, uint32_t height, uint8_t *pDst, uint32_t dstStride,
+                                        const uint8_t *pSrc, uint32_t srcStride, uint32_t gradientSize, int32_t l2Norm,
+                                        uint16_t hystLower, uint16_t hystUpper, void *scratch, size_t scratchBytes,
+                                        uint32_t *pStatus);
+
 /* RGB -> NV12 + IYUV + half-size bilinear ScaleImage + half-size area ScaleImage of Y, in
  * one pass over the RGB frame (W even, >= 16; H even).  Outputs bit-identical to the four
  * unfused AGO nodes (the scaled images read the Y plane both colour outputs share). */
@@ -440,6 +449,13 @@ int agocuda_fused_HarrisCorners_3x3(void *stream, uint32_t width, uint32_t heigh
                                     float sensitivity, float strengthThreshold, float normFactor, float minDistance,
                                     void *pCorners, uint32_t cornerCapacity, uint32_t *pCornerCount,
                                     uint32_t *pNumCorners, void *scratch, size_t scratchBytes, uint32_t *pStatus);
+
+/* The same for every gradient and block size of {3, 5, 7}; scratch as above. */
+int agocuda_fused_HarrisCorners_NxN(void *stream, uint32_t width, uint32_t height, const uint8_t *pSrc, uint32_t srcStride,
+                                    uint32_t gradientSize, uint32_t blockSize, float sensitivity, float strengthThreshold,
+                                    float normFactor, float minDistance, void *pCorners, uint32_t cornerCapacity,
+                                    uint32_t *pCornerCount, uint32_t *pNumCorners, void *scratch, size_t scratchBytes,
+                                    uint32_t *pStatus);
 
 /* ---------------------------------------------------------------- differentiable F32 warps */
 /* F32 bilinear WarpAffine / Remap with a constant border and their adjoints, for batches of

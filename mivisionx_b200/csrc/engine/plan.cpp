@@ -925,34 +925,54 @@ static bool match_gauss_sobelmag_thresh(Graph *g, LNode &a, Chain &c)
     return true;
 }
 
-// CannySobel -> CannySuppThreshold -> CannyEdgeTrace (one vxCannyEdgeDetectorNode)
+// CannySobel -> CannySuppThreshold -> CannyEdgeTrace (one vxCannyEdgeDetectorNode), any
+// gradient size and norm
 static bool match_canny(Graph *g, LNode &a, Chain &c)
 {
-    if (a.k != LK::CANNY_SOBEL_U16_U8_3x3_L1NORM || !private_virtual(g, a.p[0])) return false;
+    int64_t gs = 0, l2 = 0;
+    switch (a.k) {
+    case LK::CANNY_SOBEL_U16_U8_3x3_L1NORM: gs = 3; break;
+    case LK::CANNY_SOBEL_U16_U8_3x3_L2NORM: gs = 3; l2 = 1; break;
+    case LK::CANNY_SOBEL_U16_U8_5x5_L1NORM: gs = 5; break;
+    case LK::CANNY_SOBEL_U16_U8_5x5_L2NORM: gs = 5; l2 = 1; break;
+    case LK::CANNY_SOBEL_U16_U8_7x7_L1NORM: gs = 7; break;
+    case LK::CANNY_SOBEL_U16_U8_7x7_L2NORM: gs = 7; l2 = 1; break;
+    default: return false;
+    }
+    if (!private_virtual(g, a.p[0])) return false;
     LNode *b = const_cast<LNode *>(reader_of(g, a.p[0]));
-    if (!b || b->k != LK::CANNY_SUPP_THRESHOLD_U8XY_U16_3x3 || !b->p[1]->is_virtual) return false;
+    if (!b || !b->p[1]->is_virtual) return false;
+    if (b->k != LK::CANNY_SUPP_THRESHOLD_U8XY_U16_3x3 && b->k != LK::CANNY_SUPP_THRESHOLD_U8XY_U16_7x7) return false;
     LNode *t = const_cast<LNode *>(reader_of(g, b->p[1]));
     if (!t || t->k != LK::CANNY_EDGE_TRACE_U8_U8XY || t->p[0] != b->p[0]) return false;
     Threshold *th = static_cast<Threshold *>(b->p[3]);
     c.kind = "fused_CannyEdgeDetector";
     c.nodes = {&a, b, t};
-    c.key = {(int64_t)(uint16_t)th->lower.U32, (int64_t)(uint16_t)th->upper.U32};
+    const int32_t q4 = b->k == LK::CANNY_SUPP_THRESHOLD_U8XY_U16_7x7 ? 4 : 1;   // as in the per-node step
+    c.key = {(int64_t)(uint16_t)((int32_t)th->lower.U32 / q4), (int64_t)(uint16_t)((int32_t)th->upper.U32 / q4), gs, l2};
     c.src = a.p[1]; c.dst = b->p[0];
     c.elide = {a.p[0], b->p[1]};
     return true;
 }
 
-// HarrisSobel -> HarrisScore -> NonMaxSupp -> HarrisMergeSortAndPick (one vxHarrisCornersNode)
+// HarrisSobel -> HarrisScore -> NonMaxSupp -> HarrisMergeSortAndPick (one vxHarrisCornersNode),
+// any gradient and block size
 static bool match_harris(Graph *g, LNode &a, Chain &c)
 {
-    if (a.k != LK::HARRIS_SOBEL_HG3_U8_3x3 || !private_virtual(g, a.p[0])) return false;
+    const int64_t gs = a.k == LK::HARRIS_SOBEL_HG3_U8_3x3 ? 3 : a.k == LK::HARRIS_SOBEL_HG3_U8_5x5 ? 5
+                     : a.k == LK::HARRIS_SOBEL_HG3_U8_7x7 ? 7 : 0;
+    if (!gs || !private_virtual(g, a.p[0])) return false;
     LNode *b = const_cast<LNode *>(reader_of(g, a.p[0]));
-    if (!b || b->k != LK::HARRIS_SCORE_HVC_HG3_3x3 || !private_virtual(g, b->p[0])) return false;
+    if (!b || !private_virtual(g, b->p[0])) return false;
+    const int64_t bs = b->k == LK::HARRIS_SCORE_HVC_HG3_3x3 ? 3 : b->k == LK::HARRIS_SCORE_HVC_HG3_5x5 ? 5
+                     : b->k == LK::HARRIS_SCORE_HVC_HG3_7x7 ? 7 : 0;
+    if (!bs) return false;
     LNode *n = const_cast<LNode *>(reader_of(g, b->p[0]));
     if (!n || n->k != LK::NON_MAX_SUPP_XY_ANY_3x3 || !private_virtual(g, n->p[0])) return false;
     LNode *pk = const_cast<LNode *>(reader_of(g, n->p[0]));
     if (!pk || pk->k != LK::HARRIS_MERGE_SORT_AND_PICK_XY_XYS) return false;
     c.kind = "fused_HarrisCorners";
+    c.key = {gs, bs};
     c.nodes = {&a, b, n, pk};
     c.src = a.p[1]; c.dst = pk->p[0];
     c.elide = {a.p[0], b->p[0], n->p[0]};
@@ -1036,18 +1056,24 @@ static vx_status build_fused_batch(Graph *g, std::vector<Chain> &chains, Step &s
             if (c.kind == "fused_CannyEdgeDetector") {
                 Image *d = IMG(c.dst);
                 uint8_t *dst = d->planes[0].dev; const uint32_t ds = d->planes[0].dev_stride;
-                const size_t sb = agocuda_fused_CannyEdgeDetector_scratch_size(w, h);
+                const uint32_t gs = (uint32_t)c.key[2];
+                const int32_t l2 = (int32_t)c.key[3];
+                const bool l1x3 = gs == 3 && !l2;
+                const size_t sb = l1x3 ? agocuda_fused_CannyEdgeDetector_scratch_size(w, h)
+                                       : agocuda_fused_CannyEdgeDetector_NxN_scratch_size(w, h);
                 void *scr = scratch(g, sb);
                 if (!scr) return VX_ERROR_NO_MEMORY;
                 const uint16_t lo = (uint16_t)c.key[0], hi = (uint16_t)c.key[1];
                 fns.push_back([=](cudaStream_t q) {
-                    return agocuda_fused_CannyEdgeDetector_3x3_L1(S(q), w, h, dst, ds, src, ss, lo, hi, scr, sb, status);
+                    if (l1x3) return agocuda_fused_CannyEdgeDetector_3x3_L1(S(q), w, h, dst, ds, src, ss, lo, hi, scr, sb, status);
+                    return agocuda_fused_CannyEdgeDetector_NxN(S(q), w, h, dst, ds, src, ss, gs, l2, lo, hi, scr, sb, status);
                 });
                 st.parts.push_back(Part{fns.back(), c.nodes});
-                st.num_kernels += 4;
+                st.num_kernels += l1x3 ? 4 : 5;
             } else {
                 LNode *sc = c.nodes[1], *pk = c.nodes[3];
-                const float k = sc_f32(sc->p[2]), tc = sc_f32(sc->p[3]), norm = harris_norm(sc_i32(sc->p[4]));
+                const float k = sc_f32(sc->p[2]), tc = sc_f32(sc->p[3]), norm = harris_norm(sc_i32(sc->p[4]), (int32_t)c.key[1]);
+                const uint32_t gs = (uint32_t)c.key[0], bs = (uint32_t)c.key[1];
                 const float mind = sc_f32(pk->p[3]);
                 Array *corners = static_cast<Array *>(pk->p[0]);
                 Scalar *num = pk->p[1] ? static_cast<Scalar *>(pk->p[1]) : nullptr;
@@ -1058,7 +1084,7 @@ static vx_status build_fused_batch(Graph *g, std::vector<Chain> &chains, Step &s
                 void *scr = scratch(g, sb);
                 if (!scr) return VX_ERROR_NO_MEMORY;
                 fns.push_back([=](cudaStream_t q) {
-                    return agocuda_fused_HarrisCorners_3x3(S(q), w, h, src, ss, k, tc, norm, mind, out, ocap, oc, nc, scr, sb, status);
+                    return agocuda_fused_HarrisCorners_NxN(S(q), w, h, src, ss, gs, bs, k, tc, norm, mind, out, ocap, oc, nc, scr, sb, status);
                 });
                 st.parts.push_back(Part{fns.back(), c.nodes});
                 st.num_kernels += 3;

@@ -128,8 +128,8 @@ __global__ void k_canny_sobel(int W, int H, uint16_t *dst, int dstStride, const 
 // (r0 at +16 bytes, r1 right after, ALIGN16(W) entries each), and scalar columns from A - 1
 // on; the two formulas differ per variant (16-bit squares for 3x3 L2, a quarter-scale
 // saturating body for 7x7, Gy signs, a sign slip in the 5x5 L2 scalar top row), and the
-// SIMD part reads r0 / r1 up to R columns outside [0, A).  Each thread evaluates the
-// formula of its column, with those scratch reads resolved to the values they find there.
+// SIMD part reads r0 / r1 up to R columns outside [0, A).  Every column gets the formula of
+// its part, with those scratch reads resolved to the values they find there.
 // ---------------------------------------------------------------------------------
 template <int G> struct CannyWin;
 template <> struct CannyWin<3> { __device__ static int v(int k) { return k == 0 ? 2 : 1; }
@@ -147,10 +147,9 @@ __device__ __forceinline__ int16_t cabs16(int16_t v) { return (int16_t)(v < 0 ? 
 // pitch L = ALIGN16(W), zero padding) finds it; 0 outside the buffer
 __device__ __forceinline__ int ago_flat_px(const uint8_t *src, int stride, int W, int H, int L, int x, int y)
 {
-    const long f = (long)y * L + x;
-    if (f < 0 || f >= (long)H * L) return 0;
-    const int yy = (int)(f / L), xx = (int)(f - (long)yy * L);
-    return xx < W ? src[(size_t)yy * stride + xx] : 0;
+    if (x < 0) { x += L; y--; }              // windows reach at most 3 columns past a row of at least 16
+    else if (x >= L) { x -= L; y++; }
+    return y >= 0 && y < H && x < W ? src[(size_t)y * stride + x] : 0;
 }
 
 template <int G>
@@ -188,45 +187,45 @@ __device__ __forceinline__ uint16_t canny_l2_pack(int16_t gx, int16_t gy, bool b
     return (uint16_t)((uint16_t)(m << 2) | canny_dir(gx, gy));
 }
 
+// SIMD-body gradient from the vertical sums around a column: v0(k) / v1(k) are the reference's
+// r0 / r1 at column x + k (7x7: already quartered)
+template <int G, bool L2, class V0, class V1>
+__device__ __forceinline__ uint16_t canny_body(V0 v0, V1 v1)
+{
+    int16_t t0, t1;
+    if (G == 3) {
+        t0 = cw16(v0(1) - v0(-1));
+        t1 = cw16(0 - cw16(cw16(v1(-1) + v1(1)) + cw16(v1(0) << 1)));
+    } else if (G == 5) {
+        t0 = cs16(cw16(cw16(v0(1) - v0(-1)) << 1) + cw16(v0(2) - v0(-2)));
+        int16_t u = cw16(cw16(cw16(v1(-1) + v1(1)) << 2) + cw16(v1(-2) + v1(2)));
+        u = L2 ? cs16(u + cw16(v1(0) * 6)) : cw16(u + cw16(v1(0) * 6));
+        t1 = cw16(0 - u);
+    } else {
+        const int16_t a = cw16(cs16(v0(2) - v0(-2)) << 2);
+        const int16_t b = cw16(cs16(v0(1) - v0(-1)) * 5);
+        t0 = cs16(cs16(a + cs16(v0(3) - v0(-3))) + b);
+        int16_t u = cs16(cw16(cw16(v1(-2) + v1(2)) * 6) + cw16(v1(0) * 20));
+        const int16_t v = cw16(cw16(v1(-1) + v1(1)) * 15);
+        u = cs16(u + cs16(v1(-3) + v1(3)));
+        u = cs16(u + v);
+        t1 = cs16(0 - u);
+    }
+    if (L2) return canny_l2_pack(t0, t1, G == 3);
+    int16_t m = cw16(cabs16(t0) + cabs16(t1));
+    if (G == 7 && m > 0x3FFF) m = 0x3FFF;
+    return (uint16_t)((uint16_t)(m << 2) | canny_dir(t0, t1));
+}
+
+// the columns near the row's ends: the body's reads of its scratch, or the scalar formula
 template <int G, bool L2>
-__global__ void k_canny_sobel_nxn(int W, int H, uint16_t *dst, int dstStride, const uint8_t *src, int srcStride)
+__device__ __noinline__ uint16_t canny_edge_column(int W, int H, const uint8_t *src, int srcStride, int x, int y)
 {
     constexpr int R = G / 2;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y;
-    if (x >= W) return;
-    uint16_t *d = (uint16_t *)((uint8_t *)dst + (size_t)y * dstStride);
-    if (y < R || y >= H - R) { d[x] = 0; return; }
     const int L = (W + 15) & ~15, A = W - (W & 15);
     if (x < A - 1) {
         const CannyRowSums<G> sc{src, srcStride, y, A, L};
-        int16_t t0, t1;
-        if (G == 3) {
-            t0 = cw16(sc.r0(x + 1) - sc.r0(x - 1));
-            t1 = cw16(0 - cw16(cw16(sc.r1(x - 1) + sc.r1(x + 1)) + cw16(sc.r1(x) << 1)));
-        } else if (G == 5) {
-            t0 = cs16(cw16(cw16(sc.r0(x + 1) - sc.r0(x - 1)) << 1) + cw16(sc.r0(x + 2) - sc.r0(x - 2)));
-            int16_t u = cw16(cw16(cw16(sc.r1(x - 1) + sc.r1(x + 1)) << 2) + cw16(sc.r1(x - 2) + sc.r1(x + 2)));
-            u = L2 ? cs16(u + cw16(sc.r1(x) * 6)) : cw16(u + cw16(sc.r1(x) * 6));
-            t1 = cw16(0 - u);
-        } else {
-            const int16_t a = cw16(cs16(sc.r0(x + 2) - sc.r0(x - 2)) << 2);
-            const int16_t b = cw16(cs16(sc.r0(x + 1) - sc.r0(x - 1)) * 5);
-            t0 = cs16(cs16(a + cs16(sc.r0(x + 3) - sc.r0(x - 3))) + b);
-            int16_t u = cs16(cw16(cw16(sc.r1(x - 2) + sc.r1(x + 2)) * 6) + cw16(sc.r1(x) * 20));
-            const int16_t v = cw16(cw16(sc.r1(x - 1) + sc.r1(x + 1)) * 15);
-            u = cs16(u + cs16(sc.r1(x - 3) + sc.r1(x + 3)));
-            u = cs16(u + v);
-            t1 = cs16(0 - u);
-        }
-        if (L2) {
-            d[x] = canny_l2_pack(t0, t1, G == 3);
-        } else {
-            int16_t m = cw16(cabs16(t0) + cabs16(t1));
-            if (G == 7 && m > 0x3FFF) m = 0x3FFF;
-            d[x] = (uint16_t)((uint16_t)(m << 2) | canny_dir(t0, t1));
-        }
-        return;
+        return canny_body<G, L2>([&](int k) { return sc.r0(x + k); }, [&](int k) { return sc.r1(x + k); });
     }
     int gxs = 0, gys = 0;
 #pragma unroll
@@ -249,7 +248,105 @@ __global__ void k_canny_sobel_nxn(int W, int H, uint16_t *dst, int dstStride, co
         t = cw16(abs(gx) + abs(gy));
     }
     t = cw16(t << 2);
-    d[x] = (uint16_t)cw16(t | canny_dir(gx, gy));
+    return (uint16_t)cw16(t | canny_dir(gx, gy));
+}
+
+// Vertical window sums of G rows over a 4-column word per item, in 16-bit lanes: `smooth` at
+// weight CannyWin::v, `diff` at CannyWin::d biased by kVBias (both below 2^15, so the lanes
+// stay apart).  in: words of tile rows, `words` per row; out rows r need in rows r .. r+G-1.
+constexpr int kVBias = 4096;
+template <int G>
+__device__ __forceinline__ void vertical_sums(const uint32_t *in, int words, int rows, uint16_t *smooth, uint16_t *diff)
+{
+    for (int i = threadIdx.x; i < rows * words; i += blockDim.x) {
+        const int r = i / words, q = i - r * words;
+        uint32_t sE = 0, sO = 0, dE = kVBias * 0x10001u, dO = kVBias * 0x10001u;
+#pragma unroll
+        for (int k = 0; k < G; k++) {
+            const uint32_t w = in[(r + k) * words + q];
+            const uint32_t e = w & 0x00ff00ffu, o = (w >> 8) & 0x00ff00ffu;
+            const int v = CannyWin<G>::v(k - G / 2), d = CannyWin<G>::d(k - G / 2);
+            sE += (uint32_t)v * e;
+            sO += (uint32_t)v * o;
+            dE += (uint32_t)d * e;
+            dO += (uint32_t)d * o;
+        }
+        *(uint2 *)(smooth + 4 * (r * words + q)) = make_uint2(__byte_perm(sE, sO, 0x5410), __byte_perm(sE, sO, 0x7632));
+        *(uint2 *)(diff + 4 * (r * words + q)) = make_uint2(__byte_perm(dE, dO, 0x5410), __byte_perm(dE, dO, 0x7632));
+    }
+}
+
+// 12 vertical sums (columns c-4 .. c+7) as ints
+__device__ __forceinline__ void unpack12(const uint16_t *v, int bias, int out[12])
+{
+    const uint2 *p = (const uint2 *)v;
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const uint2 w = p[j];
+        out[4 * j] = (int)(w.x & 0xffff) - bias;
+        out[4 * j + 1] = (int)(w.x >> 16) - bias;
+        out[4 * j + 2] = (int)(w.y & 0xffff) - bias;
+        out[4 * j + 3] = (int)(w.y >> 16) - bias;
+    }
+}
+
+// A tile of source words in shared memory: columns xq .. xq + 4 words - 1, rows yq ..; what
+// lies outside the image is 0
+__device__ __forceinline__ void load_words(uint32_t *tile, int words, int rows, const uint8_t *src, int stride, int W, int H,
+                                           int xq, int yq)
+{
+    const bool al = (((uintptr_t)src | (uintptr_t)stride) & 3) == 0;
+    for (int i = threadIdx.x; i < words * rows; i += blockDim.x) {
+        const int r = i / words, q = i - r * words, y = yq + r, x = xq + 4 * q;
+        uint32_t w = 0;
+        if ((unsigned)y < (unsigned)H) {
+            const uint8_t *p = src + (size_t)y * stride + x;
+            if (al && x >= 0 && x + 4 <= W) w = __ldg((const uint32_t *)p);
+            else
+                for (int k = 0; k < 4; k++)
+                    if (x + k >= 0 && x + k < W) w |= (uint32_t)p[k] << (8 * k);
+        }
+        tile[i] = w;
+    }
+}
+
+// Gradient plane, a 64x16 tile per block: the source words, then per column the vertical sums
+// (two adds per tap for two columns in 16-bit lanes), then four pixels per thread from 12 sums
+// each.  One thread per pixel summed every column of its window again, G^2 byte loads twice (44 us
+// per 1917x1077 frame at 5x5 L2).
+constexpr int kCgW = 64, kCgH = 16, kCgWords = (kCgW + 8) / 4;
+template <int G, bool L2>
+__global__ void __launch_bounds__(256) k_canny_sobel_nxn(int W, int H, uint16_t *dst, int dstStride, const uint8_t *src, int srcStride)
+{
+    constexpr int R = G / 2;
+    __shared__ uint32_t sIn[(kCgH + 2 * R) * kCgWords];
+    __shared__ __align__(16) uint16_t sS[kCgH * kCgWords * 4], sD[kCgH * kCgWords * 4];
+    const int x0 = blockIdx.x * kCgW, y0 = blockIdx.y * kCgH;
+    load_words(sIn, kCgWords, kCgH + 2 * R, src, srcStride, W, H, x0 - 4, y0 - R);
+    __syncthreads();
+    vertical_sums<G>(sIn, kCgWords, kCgH, sS, sD);
+    __syncthreads();
+    const int r = threadIdx.x >> 4, c = 4 * (threadIdx.x & 15), x = x0 + c, y = y0 + r;
+    if (x >= W || y >= H) return;
+    const int A = W - (W & 15);
+    uint32_t g[4] = {0, 0, 0, 0};
+    if (y >= R && y < H - R) {
+        int v0[12], v1[12];
+        unpack12(sS + r * kCgWords * 4 + c, 0, v0);
+        unpack12(sD + r * kCgWords * 4 + c, kVBias, v1);
+#pragma unroll
+        for (int j = 0; j < 12; j++) { v0[j] >>= G == 7 ? 2 : 0; v1[j] >>= G == 7 ? 2 : 0; }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (x + j >= R && x + j + R < A)
+                g[j] = canny_body<G, L2>([&](int k) { return v0[4 + j + k]; }, [&](int k) { return v1[4 + j + k]; });
+            else if (x + j < W)
+                g[j] = canny_edge_column<G, L2>(W, H, src, srcStride, x + j, y);
+    }
+    uint16_t *d = (uint16_t *)((uint8_t *)dst + (size_t)y * dstStride) + x;
+    if (x + 4 <= W && ((uintptr_t)d & 7) == 0) *(uint2 *)d = make_uint2(g[0] | (g[1] << 16), g[2] | (g[3] << 16));
+    else
+        for (int j = 0; j < 4 && x + j < W; j++) d[j] = (uint16_t)g[j];
 }
 
 __global__ void k_canny_supp(int W, int H, uint8_t *dst, int dstStride, const uint16_t *g, int gStride,
@@ -478,14 +575,19 @@ __device__ __forceinline__ int sG_mag3(uint32_t g) { return (int)(g | 3u); }   /
 constexpr int kInPitchTma = 24, kInOffTma = 3;
 constexpr int kCannyWaitLimit = 1 << 20;                 // bounded mbarrier waits
 
-template <bool TMA>
+// Where the front's gradient comes from: the 3x3 L1 formula on source words, on a TMA box, or a
+// plane of packed gradients (the other window sizes and norms; src then points to that plane)
+enum CannySrc { kCannyWords = 0, kCannyTma = 1, kCannyPlane = 2 };
+
+template <int SRC>
 __global__ void __launch_bounds__(256, 6)
 k_canny_ccl_front(int W, int H, const uint8_t *__restrict__ src, int srcStride, int lower, int upper,
                   uint8_t *__restrict__ dst, int dstStride, CannyTiles T, uint32_t *__restrict__ err,
                   const __grid_constant__ CUtensorMap map)
 {
+    constexpr bool TMA = SRC == kCannyTma;
     constexpr int kPitch = TMA ? kInPitchTma : kInWords, kOff = TMA ? kInOffTma : 0;
-    __shared__ __align__(128) uint32_t sIn[kIH][kPitch];
+    __shared__ __align__(128) uint32_t sIn[SRC == kCannyPlane ? 1 : kIH][kPitch];
     __shared__ __align__(16) uint16_t sG[kGH][kGC];
     __shared__ __align__(16) int sLab[kTS];
     __shared__ unsigned long long sNZ[kTH], sST[kTH];   // per tile row: non-zero / strong pixels
@@ -508,7 +610,7 @@ k_canny_ccl_front(int W, int H, const uint8_t *__restrict__ src, int srcStride, 
                 "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                 ::"r"(smem_addr_u32(&sIn[0][0])), "l"((uint64_t)&map), "r"(x0 - 16), "r"(y0 - 2), "r"(b) : "memory");
         }
-    } else {
+    } else if constexpr (SRC == kCannyWords) {
         const bool al = (((uintptr_t)src | (uintptr_t)srcStride) & 3) == 0;
         static_assert(kIH * kInWords <= 3 * 256, "three words per thread");
 #pragma unroll
@@ -530,7 +632,7 @@ k_canny_ccl_front(int W, int H, const uint8_t *__restrict__ src, int srcStride, 
     if (tid < kTS / 32) { sStrongRoot[tid] = 0; sOpen[tid] = 0; }
     if (tid < kOpenMax / 32) sOpenStrong[tid] = 0;
     if (tid == 0) sRunN = 0;
-    const bool needV = x0 == 0 && (W & 15) == 0 && W >= 16;
+    const bool needV = SRC != kCannyPlane && x0 == 0 && (W & 15) == 0 && W >= 16;
     if (needV && tid < kGH) {
         const int y = y0 - 1 + tid;
         sV[tid] = (y >= 1 && y < H - 1)
@@ -572,7 +674,14 @@ k_canny_ccl_front(int W, int H, const uint8_t *__restrict__ src, int srcStride, 
         const int gr = i / kInWords, q = i - gr * kInWords;
         const int y = y0 - 1 + gr, xq = x0 - 4 + 4 * q;
         uint32_t out0 = 0, out1 = 0;
-        if (y >= 1 && y < H - 1) {
+        if constexpr (SRC == kCannyPlane) {
+            if ((unsigned)y < (unsigned)H && xq >= 0 && xq < W) {   // rows hold whole 8-byte groups
+                const uint2 v = __ldg((const uint2 *)((const uint16_t *)(src + (size_t)y * srcStride) + xq));
+                const int n = W - xq;
+                out0 = n >= 2 ? v.x : v.x & 0xffffu;
+                out1 = n >= 4 ? v.y : n == 3 ? v.y & 0xffffu : 0u;
+            }
+        } else if (y >= 1 && y < H - 1) {
             Lanes4 t, m, b;
             {
                 const uint32_t *r0 = sIn[gr] + kOff, *r1 = sIn[gr + 1] + kOff, *r2 = sIn[gr + 2] + kOff;
@@ -1614,6 +1723,109 @@ __global__ void __launch_bounds__(256) k_harris_score_nxn(int W, int H, float *d
     *(float *)((uint8_t *)dst + (size_t)y * dstStride + 4 * (size_t)x) = v;
 }
 
+// Harris front end for the other gradient and block sizes, a 64x16 tile per block in one pass:
+// source words, vertical gradient sums (as in the Canny gradients; the integer sums are exact in
+// any order), products, scores and suppression, all in shared memory.  The window sums of the
+// products are floats beyond 2^24, so they keep the reference's (row, column) order; a thread
+// makes four scores from shared loads of 16 bytes.  The separate kernels moved 12 bytes of
+// products and 4 of scores per pixel through global memory and read every product B^2 times.
+// Canny 5x5 L2 + Harris 5x5 / 5x5 of four 1917x1077 frames: 1328 us one launch per node, 308 us
+// with this front and the tiled Canny gradient feeding the connected-components front.
+constexpr int kHnW = 64, kHnH = 16;
+constexpr int kHnWords = 21, kHnPW = 76, kHnSW = 72;   // words of columns x0-8.., products of x0-4.., scores of x0-4..
+
+template <int G, int B>
+__global__ void __launch_bounds__(256) k_harris_front_nxn(int W, int H, const uint8_t *__restrict__ src, int srcStride, float k,
+                                                         float Tc, float norm, uint64_t *list, uint32_t *count, uint32_t capacity)
+{
+    constexpr int RG = G / 2, RB = B / 2, SHIFT = B == 7 ? 1 : 0;   // B = 7: column x holds the score of column x + 1
+    constexpr int kSR = kHnH + 2, kPR = kSR + 2 * RB, kIR = kPR + 2 * RG;   // score, product, source rows
+    __shared__ uint32_t sIn[kIR * kHnWords];
+    __shared__ __align__(16) uint16_t sV[2][kPR * kHnWords * 4];
+    __shared__ __align__(16) float sP[3][kPR][kHnPW];
+    __shared__ __align__(16) float sS[kSR][kHnSW];
+    const int x0 = blockIdx.x * kHnW, y0 = blockIdx.y * kHnH, tid = threadIdx.x;
+    const int yP = y0 - 1 - RB, yI = yP - RG;              // image rows of product row 0, source row 0
+    load_words(sIn, kHnWords, kIR, src, srcStride, W, H, x0 - 8, yI);
+    // columns outside the image read AGO's bytes (the neighbouring rows'): at most RG on each side
+    if (x0 == 0 || x0 - 8 + 4 * kHnWords > W) {
+        __syncthreads();
+        uint8_t *b8 = (uint8_t *)sIn;
+        for (int i = tid; i < kIR * 2 * RG; i += blockDim.x) {
+            const int r = i / (2 * RG), q = i - r * 2 * RG, x = q < RG ? q - RG : W + q - RG, c = x - (x0 - 8);
+            if (c >= 0 && c < 4 * kHnWords && yI + r >= 0 && yI + r < H)
+                b8[r * 4 * kHnWords + c] = (uint8_t)ago_byte(src, (size_t)srcStride, W, H, yI + r, x);
+        }
+    }
+    __syncthreads();
+    vertical_sums<G>(sIn, kHnWords, kPR, sV[0], sV[1]);
+    __syncthreads();
+    for (int i = tid; i < kPR * (kHnPW / 4); i += blockDim.x) {
+        const int r = i / (kHnPW / 4), q = i - r * (kHnPW / 4), y = yP + r;
+        float p[3][4] = {};
+        if (y >= RG && y < H - RG) {
+            int vs[12], vd[12];                            // columns of the word before, this and the next
+            unpack12(sV[0] + (r * kHnWords + q) * 4, 0, vs);
+            unpack12(sV[1] + (r * kHnWords + q) * 4, kVBias, vd);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                int gx = 0, gy = 0;
+#pragma unroll
+                for (int u = -RG; u <= RG; u++) {
+                    gx += CannyWin<G>::d(u) * vs[4 + j + u];
+                    gy += CannyWin<G>::v(u) * vd[4 + j + u];
+                }
+                const float fx = (float)gx, fy = (float)gy;
+                p[0][j] = __fmul_rn(fx, fx);
+                p[1][j] = __fmul_rn(fx, fy);
+                p[2][j] = __fmul_rn(fy, fy);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) *(float4 *)&sP[c][r][4 * q] = make_float4(p[c][0], p[c][1], p[c][2], p[c][3]);
+    }
+    __syncthreads();
+    for (int i = tid; i < kSR * (kHnSW / 4); i += blockDim.x) {
+        const int r = i / (kHnSW / 4), q = i - r * (kHnSW / 4), y = y0 - 1 + r, x = x0 - 4 + 4 * q;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        // the outer groups hold one column each that is read (x0 - 1 and x0 + 64): their other
+        // windows leave the product tile and are not needed
+        if (y >= RB && y < H - RB && x + 3 + SHIFT >= RB && x + SHIFT < W - RB) {
+            float sum[3][4] = {};
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int j = 0; j < B; j++) {
+                    float t[12];                           // columns x-4 .. x+7
+                    const float *row = sP[c][r + j] + 4 * q;
+#pragma unroll
+                    for (int e = 0; e < 3; e++) {
+                        const bool in = (e > 0 || q > 0) && (e < 2 || q + 1 < kHnPW / 4);
+                        const float4 f = in ? *(const float4 *)(row + 4 * (e - 1)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        t[4 * e] = f.x; t[4 * e + 1] = f.y; t[4 * e + 2] = f.z; t[4 * e + 3] = f.w;
+                    }
+#pragma unroll
+                    for (int p = 0; p < 4; p++)
+#pragma unroll
+                        for (int u = -RB; u <= RB; u++) sum[c][p] = __fadd_rn(sum[c][p], t[4 + p + SHIFT + u]);
+                }
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                const int c = x + p + SHIFT;
+                if (c >= RB && c < W - RB) v[p] = harris_score(sum[0][p], sum[1][p], sum[2][p], k, Tc, norm);
+            }
+        }
+        *(float4 *)&sS[r][4 * q] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+    __syncthreads();
+    for (int i = tid; i < kHnH * kHnW; i += blockDim.x) {  // warps stay whole: xys_append votes
+        const int r = i / kHnW, c = i - r * kHnW, x = x0 + c, y = y0 + r;
+        auto S = [&](int dx, int dy) { return sS[r + 1 + dy][c + 4 + dx]; };
+        const bool keep = x >= 1 && x < W - 1 && y >= 1 && y < H - 1 && harris_nms(S);
+        xys_append(list, count, capacity, xys_pack(x, y, S(0, 0)), keep);
+    }
+}
+
 bool aligned(const void *p, unsigned a) { return ((uintptr_t)p & (a - 1)) == 0; }
 
 }  // namespace
@@ -1640,9 +1852,8 @@ extern "C" int agocuda_CannySobel_U16_U8_3x3_L1NORM(void *stream, uint32_t W, ui
         if (!pDst || !pSrc || W < G || H < G || dstStride < 2 * W || srcStride < W || !aligned(pDst, 2) ||   \
             (dstStride & 1))                                                                                    \
             return AGOCUDA_INVALID_PARAMS;                                                                      \
-        k_canny_sobel_nxn<G, L2><<<row_grid(W, H, 128), 128, 0, as_stream(stream)>>>((int)W, (int)H, pDst,    \
-                                                                                     (int)dstStride, pSrc,     \
-                                                                                     (int)srcStride);          \
+        k_canny_sobel_nxn<G, L2><<<dim3(div_up(W, kCgW), div_up(H, kCgH)), 256, 0, as_stream(stream)>>>(        \
+            (int)W, (int)H, pDst, (int)dstStride, pSrc, (int)srcStride);                                       \
         agocuda_count_launch(1);                                                                                \
         return agocuda_launch_status();                                                                         \
     }
@@ -1797,6 +2008,17 @@ static size_t canny_tiles_layout(uint32_t W, uint32_t H, void *base, CannyTiles 
     return o;
 }
 
+// what follows the front: unions across tile borders, flatten, patch
+static void canny_ccl_tail(cudaStream_t s, int W, int H, uint8_t *dst, int dstStride, const CannyTiles &T, uint32_t *status)
+{
+    const int tiles = T.tilesX * T.tilesY, nodes = tiles * kOpenMax;
+    constexpr int kPer = kTH + kTW + kTH;
+    k_canny_ccl_border<<<dim3(div_up(kPer, 128), tiles), 128, 0, s>>>(W, H, T, status);
+    k_canny_ccl_flatten<<<div_up(nodes, 256), 256, 0, s>>>(T, nodes);
+    k_canny_ccl_patch<<<div_up(tiles, 8), 256, 0, s>>>(tiles, T, dst, dstStride);
+    agocuda_count_launch(3);
+}
+
 extern "C" int agocuda_fused_CannyEdgeDetector_3x3_L1(void *stream, uint32_t W, uint32_t H, uint8_t *pDst, uint32_t dstStride,
                                                       const uint8_t *pSrc, uint32_t srcStride, uint16_t hystLower,
                                                       uint16_t hystUpper, void *scratch, size_t scratchBytes, uint32_t *pStatus)
@@ -1807,22 +2029,54 @@ extern "C" int agocuda_fused_CannyEdgeDetector_3x3_L1(void *stream, uint32_t W, 
     CannyTiles T{};
     if (scratchBytes < canny_tiles_layout(W, H, scratch, &T)) return AGOCUDA_INVALID_PARAMS;
     cudaStream_t s = as_stream(stream);
-    const int tiles = T.tilesX * T.tilesY, nodes = tiles * kOpenMax;
     // the input tiles come by TMA where the plane allows a tensor map (16-byte aligned rows);
     // the map is a kernel parameter, so a captured launch keeps it
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
     if (agocuda_u8_tensor_map(&map, pSrc, W, H, srcStride, kInPitchTma * 4, kIH))
-        k_canny_ccl_front<true><<<dim3(T.tilesX, T.tilesY), 256, 0, s>>>(
+        k_canny_ccl_front<kCannyTma><<<dim3(T.tilesX, T.tilesY), 256, 0, s>>>(
             (int)W, (int)H, pSrc, (int)srcStride, hystLower, hystUpper, pDst, (int)dstStride, T, pStatus, map);
     else
-        k_canny_ccl_front<false><<<dim3(T.tilesX, T.tilesY), 256, 0, s>>>(
+        k_canny_ccl_front<kCannyWords><<<dim3(T.tilesX, T.tilesY), 256, 0, s>>>(
             (int)W, (int)H, pSrc, (int)srcStride, hystLower, hystUpper, pDst, (int)dstStride, T, pStatus, map);
-    constexpr int kPer = kTH + kTW + kTH;
-    k_canny_ccl_border<<<dim3(div_up(kPer, 128), tiles), 128, 0, s>>>((int)W, (int)H, T, pStatus);
-    k_canny_ccl_flatten<<<div_up(nodes, 256), 256, 0, s>>>(T, nodes);
-    k_canny_ccl_patch<<<div_up(tiles, 8), 256, 0, s>>>(tiles, T, pDst, (int)dstStride);
-    agocuda_count_launch(4);
+    agocuda_count_launch(1);
+    canny_ccl_tail(s, (int)W, (int)H, pDst, (int)dstStride, T, pStatus);
+    return agocuda_launch_status();
+}
+
+// scratch of the general form: the tiles' state, then the gradient plane (rows of whole 64 bytes)
+static uint32_t canny_plane_stride(uint32_t W) { return (2 * W + 63) & ~63u; }
+
+extern "C" size_t agocuda_fused_CannyEdgeDetector_NxN_scratch_size(uint32_t W, uint32_t H)
+{
+    return canny_tiles_layout(W, H, nullptr, nullptr) + (size_t)canny_plane_stride(W) * H;
+}
+
+extern "C" int agocuda_fused_CannyEdgeDetector_NxN(void *stream, uint32_t W, uint32_t H, uint8_t *pDst, uint32_t dstStride,
+                                                   const uint8_t *pSrc, uint32_t srcStride, uint32_t gradientSize, int32_t l2Norm,
+                                                   uint16_t hystLower, uint16_t hystUpper, void *scratch, size_t scratchBytes,
+                                                   uint32_t *pStatus)
+{
+    if (!pDst || !pSrc || !scratch || !pStatus || dstStride < W || srcStride < W || W > 65535 || H > 65535 ||
+        !aligned(scratch, 256) || scratchBytes < agocuda_fused_CannyEdgeDetector_NxN_scratch_size(W, H))
+        return AGOCUDA_INVALID_PARAMS;
+    CannyTiles T{};
+    uint16_t *plane = (uint16_t *)((uint8_t *)scratch + canny_tiles_layout(W, H, scratch, &T));
+    const uint32_t pitch = canny_plane_stride(W);
+    int rc = AGOCUDA_INVALID_PARAMS;
+    if (gradientSize == 3 && l2Norm) rc = agocuda_CannySobel_U16_U8_3x3_L2NORM(stream, W, H, plane, pitch, pSrc, srcStride);
+    else if (gradientSize == 5)
+        rc = (l2Norm ? agocuda_CannySobel_U16_U8_5x5_L2NORM : agocuda_CannySobel_U16_U8_5x5_L1NORM)(stream, W, H, plane, pitch, pSrc, srcStride);
+    else if (gradientSize == 7)
+        rc = (l2Norm ? agocuda_CannySobel_U16_U8_7x7_L2NORM : agocuda_CannySobel_U16_U8_7x7_L1NORM)(stream, W, H, plane, pitch, pSrc, srcStride);
+    if (rc) return rc;
+    cudaStream_t s = as_stream(stream);
+    CUtensorMap map;
+    memset(&map, 0, sizeof(map));
+    k_canny_ccl_front<kCannyPlane><<<dim3(T.tilesX, T.tilesY), 256, 0, s>>>(
+        (int)W, (int)H, (const uint8_t *)plane, (int)pitch, hystLower, hystUpper, pDst, (int)dstStride, T, pStatus, map);
+    agocuda_count_launch(1);
+    canny_ccl_tail(s, (int)W, (int)H, pDst, (int)dstStride, T, pStatus);
     return agocuda_launch_status();
 }
 
@@ -1981,4 +2235,39 @@ extern "C" int agocuda_HarrisScore_HVC_HG3_NxN(void *stream, uint32_t W, uint32_
                                                                   sensitivity, strengthThreshold, normFactor);
     agocuda_count_launch(1);
     return agocuda_launch_status();
+}
+
+extern "C" int agocuda_fused_HarrisCorners_NxN(void *stream, uint32_t W, uint32_t H, const uint8_t *pSrc, uint32_t srcStride,
+                                               uint32_t gradientSize, uint32_t blockSize, float sensitivity,
+                                               float strengthThreshold, float normFactor, float minDistance, void *pCorners,
+                                               uint32_t cornerCapacity, uint32_t *pCornerCount, uint32_t *pNumCorners,
+                                               void *scratch, size_t scratchBytes, uint32_t *pStatus)
+{
+    const uint32_t G = gradientSize, B = blockSize, cap = harris_list_capacity(W, H), least = G > B ? G : B;
+    if (!pSrc || !pCorners || !pCornerCount || !scratch || !pStatus || W < least || H < least || srcStride < W ||
+        (G != 3 && G != 5 && G != 7) || (B != 3 && B != 5 && B != 7) ||
+        scratchBytes < agocuda_fused_HarrisCorners_scratch_size(W, H, minDistance) || !aligned(scratch, 256))
+        return AGOCUDA_INVALID_PARAMS;
+    if (G == 3 && B == 3)
+        return agocuda_fused_HarrisCorners_3x3(stream, W, H, pSrc, srcStride, sensitivity, strengthThreshold, normFactor, minDistance,
+                                               pCorners, cornerCapacity, pCornerCount, pNumCorners, scratch, scratchBytes, pStatus);
+    uint32_t *cnt = (uint32_t *)scratch;
+    uint64_t *list = (uint64_t *)((uint8_t *)scratch + 256);
+    void *pickScratch = (uint8_t *)scratch + 256 + pick_align((size_t)cap * 8);
+    cudaStream_t s = as_stream(stream);
+    cudaMemsetAsync(cnt, 0, 4, s);
+    const dim3 grd(div_up(W, kHnW), div_up(H, kHnH));
+#define HARRIS_CASE(g, b)                                                                                                     \
+    if (G == g && B == b)                                                                                                     \
+        k_harris_front_nxn<g, b><<<grd, 256, 0, s>>>((int)W, (int)H, pSrc, (int)srcStride, sensitivity, strengthThreshold,   \
+                                                     normFactor, list, cnt, cap);
+    HARRIS_CASE(3, 5) HARRIS_CASE(3, 7) HARRIS_CASE(5, 3) HARRIS_CASE(5, 5) HARRIS_CASE(5, 7) HARRIS_CASE(7, 3) HARRIS_CASE(7, 5)
+    HARRIS_CASE(7, 7)
+#undef HARRIS_CASE
+    agocuda_count_launch(1);
+    const int rc = agocuda_launch_status();
+    if (rc) return rc;
+    return agocuda_HarrisMergeSortAndPick_XY_XYS(stream, W, H, list, cnt, cap, minDistance, pCorners, cornerCapacity,
+                                                 pCornerCount, pNumCorners, pickScratch,
+                                                 agocuda_HarrisMergeSortAndPick_scratch_size(W, H, cap, minDistance), pStatus);
 }

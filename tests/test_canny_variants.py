@@ -178,3 +178,17 @@ def test_engine_canny_variants_share_a_context(cuda):
             api.ok(api.vxProcessGraph(g), "process after other graphs were released")
     finally:
         assert api.vxReleaseContext(C.byref(C.c_void_p(ctx))) == 0
+
+
+# the fused form at the edges of its tiles (64 columns; 16 gradient and 32 hysteresis rows)
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(63, 33), (65, 31), (129, 49), (192, 47)])
+@pytest.mark.parametrize("gs,norm", VARIANTS)
+def test_fused_canny_at_tile_edges(cuda, gs, norm, W, H):
+    img = np.random.default_rng(W * gs + H).integers(0, 256, (H, W), dtype=np.int32).astype(np.uint8)
+    lo, hi = THRESH[gs]
+    got, _ = run_canny(V.OpenVX(), img, gs, norm, lo, hi)
+    want = oracle_canny(img, gs, norm == "L2", lo, hi)
+    b = gs // 2 + 1
+    np.testing.assert_array_equal(got[b:H - b, b:W - b], want[b:H - b, b:W - b])
+    assert 0.05 < (want[b:H - b, b:W - b] == 255).mean() < 0.95

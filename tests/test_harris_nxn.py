@@ -142,3 +142,15 @@ def test_engine_harris_variants(cuda, gs, bs, W, H):
     """The engine's graph (gradient, score, suppression, device pick) equals the oracle chain:
     the same corners in the same order and the same count."""
     _check(V.OpenVX(), gs, bs, W, H)
+
+
+# the fused front at the edges of its 64x16 tiles, and dense corners (noise)
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(127, 49), (129, 33), (192, 64), (66, 47)])
+@pytest.mark.parametrize("gs,bs", PAIRS)
+def test_fused_harris_at_tile_edges(cuda, gs, bs, W, H):
+    img = np.random.default_rng(W * gs + bs).integers(0, 256, (H, W), dtype=np.int32).astype(np.uint8)
+    got, num = run_harris(V.OpenVX(), img, gs, bs, TC[gs])
+    want, want_num = OC.harris(img, tc=TC[gs], capacity=32768, gs=gs, bs=bs)
+    assert num == want_num and want_num > 20
+    np.testing.assert_array_equal(got, want)
