@@ -616,6 +616,11 @@ size_t agocuda_OpticalFlowPyrLK_carry_size(uint32_t levels, uint32_t height1);
  * frame's `carry` buffer provides exactly those (without one they read as 0). */
 int agocuda_OpticalFlowPyrLK_batch(void *stream, agocuda_lk_frame *frames, uint32_t numFrames, uint32_t maxPoints,
                                    uint32_t *pStatus);
+/* The same for frames that all satisfy agocuda_OpticalFlowPyrLK_window9 (host descriptor: a
+ * 9x9 window, planes and pitches multiples of 4): tracked by the kernel for that window. */
+int agocuda_OpticalFlowPyrLK_window9(const agocuda_lk_frame *frameHost);
+int agocuda_OpticalFlowPyrLK_batch_window9(void *stream, agocuda_lk_frame *frames, uint32_t numFrames, uint32_t maxPoints,
+                                           uint32_t *pStatus);
 
 /* Single node with the reference's argument meaning.  oldPyramid/newPyramid are HOST arrays
  * of `levels` descriptors (device images); counts are device words.  scratch (device,

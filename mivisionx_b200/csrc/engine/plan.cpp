@@ -171,7 +171,12 @@ static vx_status lk_batch_step(Graph *g, const std::vector<LNode *> &nodes, Step
         const uint32_t pts = *std::max_element(cap.begin() + k0, cap.begin() + k1);
         agocuda_lk_frame *d0 = (agocuda_lk_frame *)dev + k0;
         const uint32_t n = (uint32_t)(k1 - k0);
-        fns.push_back([=](cudaStream_t q) { return agocuda_OpticalFlowPyrLK_batch(S(q), d0, n, pts, status); });
+        const bool win9 = std::all_of(fr.begin() + k0, fr.begin() + k1,
+                                      [](const agocuda_lk_frame &f) { return agocuda_OpticalFlowPyrLK_window9(&f) != 0; });
+        fns.push_back([=](cudaStream_t q) {
+            return win9 ? agocuda_OpticalFlowPyrLK_batch_window9(S(q), d0, n, pts, status)
+                        : agocuda_OpticalFlowPyrLK_batch(S(q), d0, n, pts, status);
+        });
         st.parts.push_back(Part{fns.back(), std::vector<LNode *>(nodes.begin() + k0, nodes.begin() + k1)});
     }
     st.num_kernels = 3 * (int)fns.size();

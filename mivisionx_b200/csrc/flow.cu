@@ -681,6 +681,369 @@ __device__ void lk_track_point(const agocuda_lk_frame &F, uint32_t pt, LkWarpSme
     (void)pStatus;
 }
 
+// ---------------------------------------------------------------------------------
+// The 9x9 window: five lanes per point, six points per warp.
+//
+// The reference sums a window row by row into four float lanes (columns k and k + 4 in lane
+// k) and one scalar (column 8), so lane k of a point owns columns k and k + 4 and lane 4 owns
+// column 8: every float chain is one lane's own, the products never leave its registers, and
+// nothing is staged in shared memory.  A lane keeps its two columns of the template, of its
+// gradients and of the J window (one word of four bytes per row: both columns and their right
+// neighbours, so a bilinear sample is two dp2a) in registers over the iterations; an iteration
+// is about 200 instructions for six points, where one warp per point spent about 300 on
+// staging 81 products and adding them by ten of its lanes.  Column 8's sum is exact in any
+// order (integers), so it is an int32 sum; where a product could pass 2^24, which the
+// reference rounds to float, the lane adds in double instead.  64 uneven pairs of 2000 points:
+// tracking 2.51 -> 1.40 ms; one 720p pair of 1000 points: 87 -> 67 us (latency: one warp per
+// scheduler at most).
+//
+// Points whose window meets what the reference takes from scratch memory (first row or
+// column, the columns from W & ~7 on) take those derivatives one by one (lk9_special).
+// ---------------------------------------------------------------------------------
+constexpr int kL9 = 5, kL9Points = 6, kL9Warps = 4;
+
+// the 8 bytes at byte offset `off` (>= -1) of a row of 32-bit aligned words; byte -1 reads 0
+__device__ __forceinline__ uint2 lk9_bytes(const uint8_t *row, int off)
+{
+    const int a = off & ~3, last = (off + 7) & ~3;          // only words holding one of the 8 bytes
+    const uint32_t w0 = a >= 0 ? __ldg((const uint32_t *)(row + a)) : 0u, w1 = __ldg((const uint32_t *)(row + a + 4)),
+                   w2 = __ldg((const uint32_t *)(row + last));
+    const int sh = 8 * (off & 3);
+    return make_uint2(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh));
+}
+
+// the 6 bytes at offset `off` >= 0: (b0, b1, b4, b5)
+__device__ __forceinline__ uint32_t lk9_pairs(const uint8_t *row, int off)
+{
+    const int a = off & ~3, last = (off + 5) & ~3;
+    const uint32_t w0 = __ldg((const uint32_t *)(row + a)), w1 = __ldg((const uint32_t *)(row + a + 4)),
+                   w2 = __ldg((const uint32_t *)(row + last));
+    const int sh = 8 * (off & 3);
+    return __byte_perm(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), 0x5410);
+}
+
+// one Scharr derivative the reference's way (lk_track_point's rules) at column gc, row gr from
+// the 8-byte rows r0, r1, r2 whose byte j is column gc - 1 + (j - at); packed gx | gy << 16
+__device__ __noinline__ uint32_t lk9_special(const agocuda_lk_frame &F, int level, int W8, int gc, int gr, uint2 r0, uint2 r1,
+                                            uint2 r2, int at)
+{
+    if (gr <= 0) return 0;
+    if (gc >= W8) {
+        const int j = gc - W8;
+        if (level > 0 && F.carry && j < AGOCUDA_LK_CARRY_COLUMNS && gr < (int)F.carryRows)
+            return (uint32_t)F.carry[((level - 1) * AGOCUDA_LK_CARRY_COLUMNS + j) * (int)F.carryRows + gr];
+        return 0;
+    }
+    auto px = [&](const uint2 &r, int j) { return (int)((j < 4 ? r.x >> (8 * j) : r.y >> (8 * (j - 4))) & 0xff); };
+    const int tL = (int)(F.scharrWords[level][0] & 0xFFFF);
+    const int t0R = (int)(F.scharrWords[level][1] & 0xFFFF), t1R = (int)(F.scharrWords[level][1] >> 16);
+    const int v1c = px(r2, at + 1) - px(r0, at + 1);
+    const int v0l = gc == 0 ? 0 : 3 * (px(r0, at) + px(r2, at)) + 10 * px(r1, at);
+    const int v1l = gc == 0 ? tL : px(r2, at) - px(r0, at);
+    const int v0r = gc + 1 == W8 ? t0R : 3 * (px(r0, at + 2) + px(r2, at + 2)) + 10 * px(r1, at + 2);
+    const int v1r = gc + 1 == W8 ? t1R : px(r2, at + 2) - px(r0, at + 2);
+    return (uint32_t)(uint16_t)(v0r - v0l) | ((uint32_t)(uint16_t)(3 * (v1l + v1r) + 10 * v1c) << 16);
+}
+
+// dp2a: c + lo16(a) * byte(b, 0 / 2) + hi16(a) * byte(b, 1 / 3)
+__device__ __forceinline__ int dp2a_lo(int a, uint32_t b, int c) { int d; asm("dp2a.lo.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
+__device__ __forceinline__ int dp2a_hi(int a, uint32_t b, int c) { int d; asm("dp2a.hi.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
+
+__global__ void __launch_bounds__(kL9Warps * 32, 4) k_lk_track9(agocuda_lk_frame *frames)
+{
+    constexpr int win = 9;
+    constexpr unsigned kAll = 0xffffffffu;
+    const agocuda_lk_frame &F = frames[blockIdx.y];
+    const int lane = threadIdx.x & 31, grp = min(lane / kL9, kL9Points - 1), k = lane - grp * kL9, base = grp * kL9;
+    const uint32_t first = (blockIdx.x * kL9Warps + (threadIdx.x >> 5)) * kL9Points, pt = first + grp;
+    if (first >= F.count) return;                          // warp-uniform
+    const bool mine = pt < F.count && lane < kL9 * kL9Points;   // lanes 30, 31 idle along
+    const int kk = min(k, 4);                              // this lane's columns kk and kk + 4 (lane 4: only 8)
+    const vx_keypoint_like *oldKP = (const vx_keypoint_like *)F.oldPoints;
+    vx_keypoint_like *outKP = (vx_keypoint_like *)F.newPoints;
+    vx_keypoint_like o{};
+    if (mine) o = oldKP[pt];
+    const bool tracked = mine && o.tracking_status != 0;
+    if (mine && !tracked && k == 0) {                      // untracked input: copied (opticalflow.cpp:199)
+        vx_keypoint_like &d = outKP[pt];
+        d.x = o.x; d.y = o.y; d.strength = o.strength; d.tracking_status = o.tracking_status;
+        d.scale = o.scale; d.error = o.error;
+    }
+    int32_t ox = 0, oy = 0, ost = 0;
+    float ostr = 0.f, oerr = 0.f, carryX = 0.f, carryY = 0.f;
+    unsigned wr = 0;
+    const float fHalf = 4.f;
+    const int top = (int)F.levels - 1;
+    const bool epsOnly = F.termination == kTermEpsilon, epsTest = epsOnly || F.termination == kTermBoth;
+    const float epsilon = F.epsilon;
+    const unsigned most = epsOnly ? max(F.numIterations, (unsigned)AGOCUDA_LK_EPSILON_ONLY_MAX_ITERATIONS) : F.numIterations;
+
+    for (int level = top; level >= 0; level--) {
+        const agocuda_pyramid_level LI = F.oldPyr[level], LJ = F.newPyr[level];
+        const float ptScale = ldexpf(1.0f, -level);
+        float px = __fmul_rn((float)o.x, ptScale), py = __fmul_rn((float)o.y, ptScale);
+        float nx, ny;
+        if (level == top) {
+            if (F.useInitialEstimate) {
+                vx_keypoint_like e{};
+                if (tracked) e = ((const vx_keypoint_like *)F.estPoints)[pt];
+                nx = __fmul_rn((float)e.x, ptScale); ny = __fmul_rn((float)e.y, ptScale);
+                ostr = e.strength; ost = e.tracking_status; oerr = e.error;
+                wr |= kWrStrength | kWrStatus | kWrError;
+            } else {
+                nx = px; ny = py;
+                ost = o.tracking_status; ostr = o.strength;
+                wr |= kWrStatus | kWrStrength;
+            }
+            carryX = nx; carryY = ny;
+        } else {
+            carryX = __fmul_rn(carryX, 2.0f); carryY = __fmul_rn(carryY, 2.0f);
+            nx = carryX; ny = carryY;
+        }
+        bool on = tracked && ost != 0;                     // the point takes part in this level
+        px = __fsub_rn(px, fHalf); py = __fsub_rn(py, fHalf);
+        nx = __fsub_rn(nx, fHalf); ny = __fsub_rn(ny, fHalf);
+        int ipx = (int)floorf(px), ipy = (int)floorf(py);
+        const int limX = (int)(LI.width - 2u - (uint32_t)win), limY = (int)(LI.height - 2u - (uint32_t)win);
+        auto lost = [&]() {
+            if (!level) { ox = (int)nx; oy = (int)ny; ost = 0; oerr = 0.f; wr |= kWrX | kWrY | kWrStatus | kWrError; }
+            on = false;
+        };
+        if (on && (ipx < 0 || ipx >= limX || ipy < 0 || ipy >= limY)) lost();
+        if (!__any_sync(kAll, on)) continue;
+        float a = __fsub_rn(px, (float)ipx), b = __fsub_rn(py, (float)ipy);
+        int w[4];
+        lk_weights(a, b, w);
+        const bool whole = on && a == 0.0f && b == 0.0f;
+
+        // ---- template: I as the bits of 2^23 + I, gradients as floats (lane 4: its first column
+        // holds its gradients as ints, for the int sums of column 8)
+        uint32_t Ib[2][win];
+        float gX[2][win], gY[2][win];
+        bool big = false;                                  // lane 4: |gradient| * |difference| could reach 2^24
+        if (on) {
+            const int W8 = (int)(LI.width & ~7u), col = ipx + kk - 1;      // column of byte 0
+            const bool special = ipy == 0 || ipx == 0 || ipx + win + 1 >= W8;
+            const int w01 = (w[0] & 0xffff) | (w[1] << 16), w23 = (w[2] & 0xffff) | (w[3] << 16);
+            const uint8_t *row = LI.image + (ptrdiff_t)(ipy - 1) * LI.stride;
+            uint2 r0 = ipy > 0 ? lk9_bytes(row, col) : make_uint2(0u, 0u), r1 = lk9_bytes(row + LI.stride, col), r2;
+            uint32_t gxa0 = 0, gxb0 = 0, gya0 = 0, gyb0 = 0;   // derivative pairs of the row above: columns c, c+1 and c+4, c+5
+            uint32_t pair0 = 0;
+#pragma unroll
+            for (int y = 0; y <= win; y++) {
+                r2 = lk9_bytes(row + (ptrdiff_t)(y + 2) * LI.stride, col);
+                // vertical sums of the 8 columns in 16-bit lanes; t1 biased by 256
+                uint32_t t0[4], t1[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const uint32_t sel = j & 1 ? 0x4342u : 0x4140u;
+                    const uint32_t p0 = __byte_perm(j < 2 ? r0.x : r0.y, 0, sel), p1 = __byte_perm(j < 2 ? r1.x : r1.y, 0, sel),
+                                   p2 = __byte_perm(j < 2 ? r2.x : r2.y, 0, sel);
+                    t0[j] = 3u * (p0 + p2) + 10u * p1;
+                    t1[j] = p2 + 0x01000100u - p0;
+                }
+                // gx biased by 8192, gy by 16 * 256 + 4096 = 8192
+                const uint32_t gxa = t0[1] + 0x20002000u - t0[0], gxb = t0[3] + 0x20002000u - t0[2];
+                const uint32_t gya = 3u * (t1[0] + t1[1]) + 10u * __funnelshift_r(t1[0], t1[1], 16) + 0x10001000u;
+                const uint32_t gyb = 3u * (t1[2] + t1[3]) + 10u * __funnelshift_r(t1[2], t1[3], 16) + 0x10001000u;
+                uint32_t xa = gxa, xb = gxb, ya = gya, yb = gyb;
+                if (special) {
+                    uint32_t v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const int off = (j & 1) + 4 * (j >> 1);
+                        v[j] = lk9_special(F, level, W8, ipx + kk + off, ipy + y, r0, r1, r2, off);
+                    }
+                    auto lanes = [](uint32_t p, uint32_t q, int sh) {
+                        return (uint32_t)((int)(int16_t)(p >> sh) + 8192) | ((uint32_t)((int)(int16_t)(q >> sh) + 8192) << 16);
+                    };
+                    xa = lanes(v[0], v[1], 0); xb = lanes(v[2], v[3], 0);
+                    ya = lanes(v[0], v[1], 16); yb = lanes(v[2], v[3], 16);
+                }
+                const uint32_t pair = __byte_perm(r1.x, r1.y, 0x6521);     // bytes c, c+1, c+4, c+5
+                if (y > 0) {
+                    const int i = y - 1;
+                    // bilinear blends keep the bias: the weights add up to 2^14
+                    auto mix = [&](uint32_t up, uint32_t dn) {
+                        return (int)(((up & 0xffff) * (uint32_t)w[0] + (up >> 16) * (uint32_t)w[1] + (dn & 0xffff) * (uint32_t)w[2] +
+                                      (dn >> 16) * (uint32_t)w[3] + (1u << (kWBits - 1))) >> kWBits) - 8192;
+                    };
+                    const int xA = mix(gxa0, xa), xB = mix(gxb0, xb), yA = mix(gya0, ya), yB = mix(gyb0, yb);
+                    const int iA = dp2a_lo(w01, pair0, dp2a_lo(w23, pair, 256)), iB = dp2a_hi(w01, pair0, dp2a_hi(w23, pair, 256));
+                    Ib[0][i] = 0x4B000000u + (uint32_t)(iA >> 9);
+                    Ib[1][i] = 0x4B000000u + (uint32_t)(iB >> 9);
+                    gX[1][i] = (float)xB;
+                    gY[1][i] = (float)yB;
+                    if (k == 4) {
+                        gX[0][i] = __int_as_float(xB);
+                        gY[0][i] = __int_as_float(yB);
+                        big |= max(abs(xB), abs(yB)) > 2056;      // 2056 * 8160 < 2^24 < 2057 * 8160
+                    } else {
+                        gX[0][i] = (float)xA;
+                        gY[0][i] = (float)yA;
+                    }
+                }
+                gxa0 = xa; gxb0 = xb; gya0 = ya; gyb0 = yb;
+                pair0 = pair;
+                r0 = r1;
+                r1 = r2;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < win; i++) { Ib[0][i] = Ib[1][i] = 0; gX[0][i] = gX[1][i] = gY[0][i] = gY[1][i] = 0.f; }
+        }
+
+        // ---- covariance: the interpolated path's four float lanes and scalar column
+        float A11, A12, A22;
+        {
+            float s11 = 0.f, s12 = 0.f, s22 = 0.f;
+#pragma unroll
+            for (int i = 0; i < win; i++) {
+                if (k != 4) {
+                    s11 = __fadd_rn(s11, __fmul_rn(gX[0][i], gX[0][i]));
+                    s12 = __fadd_rn(s12, __fmul_rn(gX[0][i], gY[0][i]));
+                    s22 = __fadd_rn(s22, __fmul_rn(gY[0][i], gY[0][i]));
+                }
+                s11 = __fadd_rn(s11, __fmul_rn(gX[1][i], gX[1][i]));
+                s12 = __fadd_rn(s12, __fmul_rn(gX[1][i], gY[1][i]));
+                s22 = __fadd_rn(s22, __fmul_rn(gY[1][i], gY[1][i]));
+            }
+            auto total = [&](float v) {
+                const float v0 = __shfl_sync(kAll, v, base), v1 = __shfl_sync(kAll, v, base + 1), v2 = __shfl_sync(kAll, v, base + 2),
+                            v3 = __shfl_sync(kAll, v, base + 3), v4 = __shfl_sync(kAll, v, base + 4);
+                return __fadd_rn(v4, __fadd_rn(__fadd_rn(__fadd_rn(v0, v1), v2), v3));
+            };
+            A11 = total(s11); A12 = total(s12); A22 = total(s22);
+        }
+        if (__any_sync(kAll, whole)) {
+            // integer path: int sums of columns 0..3, of 4..7 and column 8, added in that order
+            float c11 = 0.f, c12 = 0.f, c22 = 0.f;
+            auto sum4 = [&](int v) {
+                return __shfl_sync(kAll, v, base) + __shfl_sync(kAll, v, base + 1) + __shfl_sync(kAll, v, base + 2) + __shfl_sync(kAll, v, base + 3);
+            };
+#pragma unroll
+            for (int i = 0; i < win; i++) {
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int x = k == 4 ? 0 : (int)gX[h][i], y = k == 4 ? 0 : (int)gY[h][i];
+                    c11 = __fadd_rn(c11, (float)sum4(x * x));
+                    c12 = __fadd_rn(c12, (float)sum4(x * y));
+                    c22 = __fadd_rn(c22, (float)sum4(y * y));
+                }
+                const int x = __shfl_sync(kAll, __float_as_int(gX[0][i]), base + 4), y = __shfl_sync(kAll, __float_as_int(gY[0][i]), base + 4);
+                c11 = __fadd_rn(c11, (float)(x * x));
+                c12 = __fadd_rn(c12, (float)(x * y));
+                c22 = __fadd_rn(c22, (float)(y * y));
+            }
+            if (whole) { A11 = c11; A12 = c12; A22 = c22; }
+        }
+        A11 = __fmul_rn(A11, kFltScale);
+        A12 = __fmul_rn(A12, kFltScale);
+        A22 = __fmul_rn(A22, kFltScale);
+        float D = __fsub_rn(__fmul_rn(A11, A22), __fmul_rn(A12, A12));
+        const float t = __fadd_rn(__fmul_rn(__fsub_rn(A11, A22), __fsub_rn(A11, A22)), __fmul_rn(__fmul_rn(4.f, A12), A12));
+        const float minEig = __fdiv_rn(__fsub_rn(__fadd_rn(A22, A11), __fsqrt_rn(t)), (float)(2 * win * win));
+        if (on && (minEig < 1.0e-04F || D < 1.0e-07F)) lost();
+        D = __fdiv_rn(1.f, D);
+
+        // ---- Gauss-Newton iterations, until every point of the warp is done
+        float prevDx = 0.f, prevDy = 0.f, ddx = 0.f, ddy = 0.f;
+        int jx = INT32_MIN, jy = INT32_MIN;               // integer position of the J window held
+        uint32_t J[win + 1];
+#pragma unroll
+        for (int i = 0; i <= win; i++) J[i] = 0;
+        const int jlimX = (int)(LJ.width - (uint32_t)win), jlimY = (int)(LJ.height - (uint32_t)win);
+        bool run = on;
+        for (unsigned j = 0; j < most; j++) {              // every running point is in its own iteration j
+            const int inx = (int)floorf(nx), iny = (int)floorf(ny);
+            if (run && (inx < 0 || inx >= jlimX || iny < 0 || iny >= jlimY)) {
+                if (!level) { ost = 0; oerr = 0.f; wr |= kWrStatus | kWrError; }
+                run = false;
+            }
+            if (!__any_sync(kAll, run)) break;
+            a = __fsub_rn(nx, (float)inx);
+            b = __fsub_rn(ny, (float)iny);
+            lk_weights(a, b, w);
+            if (run && (inx != jx || iny != jy)) {         // the J window only moves with the integer position
+                const uint8_t *row = LJ.image + (size_t)iny * LJ.stride;
+#pragma unroll
+                for (int i = 0; i <= win; i++) J[i] = lk9_pairs(row + (size_t)i * LJ.stride, inx + kk);
+                jx = inx;
+                jy = iny;
+            }
+            const int w01 = (w[0] & 0xffff) | (w[1] << 16), w23 = (w[2] & 0xffff) | (w[3] << 16);
+            float bx = 0.f, by = 0.f;
+            uint32_t sx = 0, sy = 0;
+#pragma unroll
+            for (int i = 0; i < win; i++) {
+                // (v >> 9) with 0x4B000000 above it: the float 2^23 + (v >> 9); v is not negative
+                const uint32_t vA = __funnelshift_r((uint32_t)dp2a_lo(w01, J[i], dp2a_lo(w23, J[i + 1], 256)), 0x96u, 9);
+                const uint32_t vB = __funnelshift_r((uint32_t)dp2a_hi(w01, J[i], dp2a_hi(w23, J[i + 1], 256)), 0x96u, 9);
+                const float dA = __fsub_rn(__uint_as_float(vA), __uint_as_float(Ib[0][i]));
+                const float dB = __fsub_rn(__uint_as_float(vB), __uint_as_float(Ib[1][i]));
+                const uint32_t iB = vB - Ib[1][i];
+                bx = __fadd_rn(__fadd_rn(bx, __fmul_rn(gX[0][i], dA)), __fmul_rn(gX[1][i], dB));
+                by = __fadd_rn(__fadd_rn(by, __fmul_rn(gY[0][i], dA)), __fmul_rn(gY[1][i], dB));
+                sx += __float_as_uint(gX[0][i]) * iB;      // lane 4's
+                sy += __float_as_uint(gY[0][i]) * iB;
+            }
+            double ex = (double)(int)sx, ey = (double)(int)sy;
+            if (k == 4 && big) {
+                ex = ey = 0.0;
+#pragma unroll
+                for (int i = 0; i < win; i++) {
+                    const uint32_t vB = __funnelshift_r((uint32_t)dp2a_hi(w01, J[i], dp2a_hi(w23, J[i + 1], 256)), 0x96u, 9);
+                    const float dB = __fsub_rn(__uint_as_float(vB), __uint_as_float(Ib[1][i]));
+                    ex = __dadd_rn(ex, (double)__fmul_rn(gX[1][i], dB));
+                    ey = __dadd_rn(ey, (double)__fmul_rn(gY[1][i], dB));
+                }
+            }
+            // (column 0 + 2) + (column 1 + 3) in float, then column 8 in double
+            auto lanes4 = [&](float v) {
+                const float v0 = __shfl_sync(kAll, v, base), v1 = __shfl_sync(kAll, v, base + 1), v2 = __shfl_sync(kAll, v, base + 2),
+                            v3 = __shfl_sync(kAll, v, base + 3);
+                return __fadd_rn(__fadd_rn(v0, v2), __fadd_rn(v1, v3));
+            };
+            const float fx = lanes4(bx), fy = lanes4(by);
+            const double ib1 = __dadd_rn(__shfl_sync(kAll, ex, base + 4), (double)fx), ib2 = __dadd_rn(__shfl_sync(kAll, ey, base + 4), (double)fy);
+            const float b1 = __double2float_rn(__dmul_rn(ib1, (double)kFltScale));
+            const float b2 = __double2float_rn(__dmul_rn(ib2, (double)kFltScale));
+            const float dx = __fmul_rn(__fsub_rn(__fmul_rn(A12, b2), __fmul_rn(A22, b1)), D);
+            const float dy = __fmul_rn(__fsub_rn(__fmul_rn(A12, b1), __fmul_rn(A11, b2)), D);
+            if (run) {
+                nx = __fadd_rn(nx, dx);
+                ny = __fadd_rn(ny, dy);
+                if (__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= epsilon && epsTest) run = false;
+                else if (j > 0 && (double)fabsf(__fadd_rn(dx, prevDx)) < 0.01 && (double)fabsf(__fadd_rn(dy, prevDy)) < 0.01) {
+                    ddx = __fmul_rn(dx, 0.5f);
+                    ddy = __fmul_rn(dy, 0.5f);
+                    run = false;
+                }
+                prevDx = dx;
+                prevDy = dy;
+            }
+        }
+        if (on) {
+            if (!level) {
+                ox = (int)__fadd_rn(__fsub_rn(__fadd_rn(nx, fHalf), ddx), 0.5f);
+                oy = (int)__fadd_rn(__fsub_rn(__fadd_rn(ny, fHalf), ddy), 0.5f);
+                wr |= kWrX | kWrY;
+            } else {
+                carryX = __fsub_rn(__fadd_rn(nx, fHalf), ddx);
+                carryY = __fsub_rn(__fadd_rn(ny, fHalf), ddy);
+            }
+        }
+    }
+    if (tracked && k == 0) {
+        vx_keypoint_like &d = outKP[pt];
+        if (wr & kWrX) d.x = ox;
+        if (wr & kWrY) d.y = oy;
+        if (wr & kWrStrength) d.strength = ostr;
+        if (wr & kWrStatus) d.tracking_status = ost;
+        if (wr & kWrError) d.error = oerr;
+    }
+}
+
 // 8 resident blocks (64 warps per SM, 32 registers): the tracking loop is latency-bound (its
 // sums keep the reference's addition order, so each is one dependent chain), and more warps
 // beat the register spills this costs (measured: 2.79 ms per pyramid + LK step at 4 blocks,
@@ -696,11 +1059,13 @@ __global__ void __launch_bounds__(kLkWarps * 32, 8) k_lk_track(agocuda_lk_frame 
 }
 
 // Replays the reference's Scharr row-buffer writes (ComputeSharr, opticalflow.cpp:65): per
-// level, the buffer words the level reads but does not write are captured first, then the
-// level's last processed row is written into the buffer.  The buffer persists per node, so
-// the top level sees what the previous execution's level 0 left.  Also checks the point
-// counts (ago_kernel_api.cpp:20603).
-__global__ void __launch_bounds__(256) k_lk_prep(agocuda_lk_frame *frames, uint32_t *pStatus)
+// level, from the top down, the buffer words the level reads but does not write are captured,
+// then the level's last processed row is written into the buffer.  The buffer persists per
+// node, so the top level sees what the previous execution's level 0 left.  Which write a word
+// holds at any time follows from the widths alone, so the levels need no order here: `seen`
+// gives the word's value before level l, and every word the levels write gets its last one.
+// Also checks the point counts (ago_kernel_api.cpp:20603).
+__global__ void __launch_bounds__(1024) k_lk_prep(agocuda_lk_frame *frames, uint32_t *pStatus)
 {
     agocuda_lk_frame &F = frames[blockIdx.x];
     if (threadIdx.x == 0) {
@@ -711,22 +1076,32 @@ __global__ void __launch_bounds__(256) k_lk_prep(agocuda_lk_frame *frames, uint3
         else *F.pNewCount = n;
     }
     uint16_t *T = F.scharrRows;
-    for (int level = (int)F.levels - 1; level >= 0; level--) {
-        const agocuda_pyramid_level L = F.oldPyr[level];
-        const uint32_t W8 = L.width & ~7u, A = (L.width + 2 + 7) & ~7u;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            F.scharrWords[level][0] = T[A - 1];
-            F.scharrWords[level][1] = (uint32_t)T[W8] | ((uint32_t)T[A + W8] << 16);
+    const int levels = (int)F.levels;
+    bool written = false;
+    auto seen = [&](uint32_t i, int before) -> uint16_t {
+        written = true;
+        for (int m = before + 1; m < levels; m++) {
+            const uint32_t w = F.oldPyr[m].width, h = F.oldPyr[m].height, W8 = w & ~7u, A = (w + 2 + 7) & ~7u;
+            if (h < 3 || !(i < W8 || (i >= A && i < A + W8))) continue;
+            const uint8_t *r0 = F.oldPyr[m].image + (size_t)(h - 3) * F.oldPyr[m].stride, *r1 = r0 + F.oldPyr[m].stride, *r2 = r1 + F.oldPyr[m].stride;
+            if (i < W8) return (uint16_t)(3 * (r0[i] + r2[i]) + 10 * r1[i]);
+            return (uint16_t)((int)r2[i - A] - (int)r0[i - A]);
         }
-        __syncthreads();
-        if (L.height >= 3) {
-            const uint8_t *r0 = L.image + (size_t)(L.height - 3) * L.stride, *r1 = r0 + L.stride, *r2 = r1 + L.stride;
-            for (uint32_t c = threadIdx.x; c < W8; c += blockDim.x) {
-                T[c] = (uint16_t)(3 * (r0[c] + r2[c]) + 10 * r1[c]);
-                T[A + c] = (uint16_t)((int)r2[c] - (int)r0[c]);
-            }
-        }
+        written = false;
+        return T[i];
+    };
+    if (threadIdx.x < 3 * levels) {
+        const int level = threadIdx.x / 3, q = threadIdx.x - 3 * level;
+        const uint32_t w = F.oldPyr[level].width, W8 = w & ~7u, A = (w + 2 + 7) & ~7u;
+        const uint16_t v = seen(q == 0 ? A - 1 : q == 1 ? W8 : A + W8, level);
+        if (q == 0) F.scharrWords[level][0] = v;
+        else ((uint16_t *)&F.scharrWords[level][1])[q - 1] = v;
+    }
+    __syncthreads();
+    const uint32_t w0 = F.oldPyr[0].width, end = ((w0 + 2 + 7) & ~7u) + (w0 & ~7u);
+    for (uint32_t i = threadIdx.x; i < end; i += blockDim.x) {
+        const uint16_t v = seen(i, -1);
+        if (written) T[i] = v;
     }
 }
 
@@ -877,20 +1252,44 @@ extern "C" size_t agocuda_OpticalFlowPyrLK_scharr_rows_size(uint32_t width0)
     return ((size_t)2 * width0 + 32) * sizeof(uint16_t);
 }
 
-extern "C" int agocuda_OpticalFlowPyrLK_batch(void *stream, agocuda_lk_frame *frames, uint32_t numFrames,
-                                              uint32_t maxPoints, uint32_t *pStatus)
+static int lk_batch(void *stream, agocuda_lk_frame *frames, uint32_t numFrames, uint32_t maxPoints, bool win9, uint32_t *pStatus)
 {
     if (!frames || !numFrames || !pStatus) return AGOCUDA_INVALID_PARAMS;
     cudaStream_t s = as_stream(stream);
-    k_lk_prep<<<numFrames, 256, 0, s>>>(frames, pStatus);
+    k_lk_prep<<<numFrames, 1024, 0, s>>>(frames, pStatus);
     agocuda_count_launch(1);
     if (maxPoints) {
-        k_lk_track<<<dim3((maxPoints + kLkWarps - 1) / kLkWarps, numFrames), kLkWarps * 32, 0, s>>>(frames, pStatus);
+        if (win9)
+            k_lk_track9<<<dim3(div_up(maxPoints, kL9Warps * kL9Points), numFrames), kL9Warps * 32, 0, s>>>(frames);
+        else
+            k_lk_track<<<dim3((maxPoints + kLkWarps - 1) / kLkWarps, numFrames), kLkWarps * 32, 0, s>>>(frames, pStatus);
         agocuda_count_launch(1);
     }
     k_lk_carry<<<numFrames, 256, 0, s>>>(frames);
     agocuda_count_launch(1);
     return agocuda_launch_status();
+}
+
+extern "C" int agocuda_OpticalFlowPyrLK_batch(void *stream, agocuda_lk_frame *frames, uint32_t numFrames,
+                                              uint32_t maxPoints, uint32_t *pStatus)
+{
+    return lk_batch(stream, frames, numFrames, maxPoints, false, pStatus);
+}
+
+// five lanes per point (k_lk_track9) for a 9x9 window over planes of aligned 32-bit words
+extern "C" int agocuda_OpticalFlowPyrLK_window9(const agocuda_lk_frame *frame)
+{
+    if (!frame || frame->windowDimension != 9) return 0;
+    for (uint32_t l = 0; l < frame->levels && l < AGOCUDA_LK_MAX_LEVELS; l++)
+        if ((((uintptr_t)frame->oldPyr[l].image | frame->oldPyr[l].stride | (uintptr_t)frame->newPyr[l].image | frame->newPyr[l].stride) & 3))
+            return 0;
+    return 1;
+}
+
+extern "C" int agocuda_OpticalFlowPyrLK_batch_window9(void *stream, agocuda_lk_frame *frames, uint32_t numFrames,
+                                                      uint32_t maxPoints, uint32_t *pStatus)
+{
+    return lk_batch(stream, frames, numFrames, maxPoints, true, pStatus);
 }
 
 extern "C" size_t agocuda_OpticalFlowPyrLK_carry_size(uint32_t levels, uint32_t height1)
@@ -959,5 +1358,5 @@ extern "C" int agocuda_OpticalFlowPyrLK_XY_XY(void *stream, void *newKeyPoint, u
     agocuda_count_launch(1);
     const int rc = agocuda_launch_status();
     if (rc) return rc;
-    return agocuda_OpticalFlowPyrLK_batch(stream, dev, 1, newCapacity, pStatus);
+    return lk_batch(stream, dev, 1, newCapacity, agocuda_OpticalFlowPyrLK_window9(&F) != 0, pStatus);
 }
