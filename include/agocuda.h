@@ -616,11 +616,15 @@ size_t agocuda_OpticalFlowPyrLK_carry_size(uint32_t levels, uint32_t height1);
  * frame's `carry` buffer provides exactly those (without one they read as 0). */
 int agocuda_OpticalFlowPyrLK_batch(void *stream, agocuda_lk_frame *frames, uint32_t numFrames, uint32_t maxPoints,
                                    uint32_t *pStatus);
-/* The same for frames that all satisfy agocuda_OpticalFlowPyrLK_window9 (host descriptor: a
- * 9x9 window, planes and pitches multiples of 4): tracked by the kernel for that window. */
-int agocuda_OpticalFlowPyrLK_window9(const agocuda_lk_frame *frameHost);
-int agocuda_OpticalFlowPyrLK_batch_window9(void *stream, agocuda_lk_frame *frames, uint32_t numFrames, uint32_t maxPoints,
-                                           uint32_t *pStatus);
+/* What holds for a frame (host descriptor), and the same batch for frames for which all of
+ * `hints` hold: WINDOW9 (a 9x9 window; planes and pitches multiples of 4) selects the tracking
+ * kernel for that window, NO_CARRY (no level above 0 with width % 8 >= 3) leaves out the pass
+ * that keeps derivative columns for the next call. */
+#define AGOCUDA_LK_HINT_WINDOW9 1u
+#define AGOCUDA_LK_HINT_NO_CARRY 2u
+uint32_t agocuda_OpticalFlowPyrLK_hints(const agocuda_lk_frame *frameHost);
+int agocuda_OpticalFlowPyrLK_batch_hints(void *stream, agocuda_lk_frame *frames, uint32_t numFrames, uint32_t maxPoints,
+                                         uint32_t hints, uint32_t *pStatus);
 
 /* Single node with the reference's argument meaning.  oldPyramid/newPyramid are HOST arrays
  * of `levels` descriptors (device images); counts are device words.  scratch (device,
@@ -660,6 +664,9 @@ typedef struct agocuda_array_xfer {
     uint32_t itemSize, capacity;
 } agocuda_array_xfer;
 int agocuda_array_upload_batch(void *stream, const agocuda_array_xfer *xfers, uint32_t count);
+/* agocuda_array_download (below) for `count` arrays in one launch; `xfers` is a DEVICE array, its host
+ * members written. */
+int agocuda_array_download_batch(void *stream, const agocuda_array_xfer *xfers, uint32_t count);
 /* hostItems[0 .. n) = devItems[0 .. n), *countSlot = n, n = min(*devCount, capacity). */
 int agocuda_array_download(void *stream, void *hostItemsMapped, uint32_t *countSlotMapped, const void *devItems,
                            const uint32_t *devCount, uint32_t itemSize, uint32_t capacity);

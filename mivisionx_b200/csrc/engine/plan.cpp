@@ -166,20 +166,18 @@ static vx_status lk_batch_step(Graph *g, const std::vector<LNode *> &nodes, Step
         return VX_FAILURE;
     uint32_t *status = g->status_dev;
     std::vector<std::function<int(cudaStream_t)>> fns;
+    st.num_kernels = 0;
     for (size_t k0 = 0; k0 < fr.size(); k0 += kGroupFrames) {
         const size_t k1 = std::min(fr.size(), k0 + kGroupFrames);
         const uint32_t pts = *std::max_element(cap.begin() + k0, cap.begin() + k1);
         agocuda_lk_frame *d0 = (agocuda_lk_frame *)dev + k0;
         const uint32_t n = (uint32_t)(k1 - k0);
-        const bool win9 = std::all_of(fr.begin() + k0, fr.begin() + k1,
-                                      [](const agocuda_lk_frame &f) { return agocuda_OpticalFlowPyrLK_window9(&f) != 0; });
-        fns.push_back([=](cudaStream_t q) {
-            return win9 ? agocuda_OpticalFlowPyrLK_batch_window9(S(q), d0, n, pts, status)
-                        : agocuda_OpticalFlowPyrLK_batch(S(q), d0, n, pts, status);
-        });
+        uint32_t hints = ~0u;
+        for (size_t i = k0; i < k1; i++) hints &= agocuda_OpticalFlowPyrLK_hints(&fr[i]);
+        fns.push_back([=](cudaStream_t q) { return agocuda_OpticalFlowPyrLK_batch_hints(S(q), d0, n, pts, hints, status); });
+        st.num_kernels += hints & AGOCUDA_LK_HINT_NO_CARRY ? 2 : 3;
         st.parts.push_back(Part{fns.back(), std::vector<LNode *>(nodes.begin() + k0, nodes.begin() + k1)});
     }
-    st.num_kernels = 3 * (int)fns.size();
     st.launch = [fns](cudaStream_t q) {
         for (auto &f : fns) { int rc = f(q); if (rc) return rc; }
         return 0;

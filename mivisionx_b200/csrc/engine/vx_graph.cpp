@@ -316,27 +316,48 @@ static vx_status capture(Graph *g)
                 parts.push_back(std::move(cp));
                 g->streamed_out.push_back(img);
             }
-    if (!serial)
+    // output arrays: one launch for all that the same part writes (a batch of frames)
+    size_t downloads = 0;
+    if (!serial) {
+        std::map<int, std::vector<Array *>> by_part;
         for (Ref *r : g->outputs)
             if (r->type == VX_TYPE_ARRAY && slot_free() && stageable(static_cast<Array *>(r))) {
-                Array *a = static_cast<Array *>(r);
-                uint32_t *slot = g->io_slots_dev + g->staged_in.size() + g->staged_out.size();
-                CapPart cp;
-                cp.rd = {a};
-                cp.lane = kArrayLane;
-                cp.launch = [a, slot](cudaStream_t q) {
-                    return agocuda_array_download(q, a->host_mapped, slot, a->dev, a->dev_count, (uint32_t)a->item_size,
-                                                  (uint32_t)a->capacity);
-                };
-                parts.push_back(std::move(cp));
-                g->staged_out.push_back(a);
+                int last = -1;
+                for (int j = 0; j < (int)parts.size(); j++)
+                    if (std::find(parts[j].wr.begin(), parts[j].wr.end(), r) != parts[j].wr.end()) last = j;
+                by_part[last].push_back(static_cast<Array *>(r));
+                g->staged_out.push_back(static_cast<Array *>(r));
             }
+        std::vector<agocuda_array_xfer> xf;
+        for (auto &kv : by_part)
+            for (Array *a : kv.second) {
+                const size_t i = std::find(g->staged_out.begin(), g->staged_out.end(), a) - g->staged_out.begin();
+                xf.push_back(agocuda_array_xfer{a->dev, a->dev_count, a->host_mapped, g->io_slots_dev + g->staged_in.size() + i,
+                                                (uint32_t)a->item_size, (uint32_t)a->capacity});
+            }
+        agocuda_array_xfer *table = nullptr;
+        if (!xf.empty()) {
+            if (cudaMalloc((void **)&table, xf.size() * sizeof(agocuda_array_xfer)) != cudaSuccess) return VX_ERROR_NO_MEMORY;
+            g->dev_scratch.push_back(table);
+            if (cudaMemcpy(table, xf.data(), xf.size() * sizeof(agocuda_array_xfer), cudaMemcpyHostToDevice) != cudaSuccess)
+                return VX_FAILURE;
+        }
+        for (auto &kv : by_part) {
+            const uint32_t n = (uint32_t)kv.second.size();
+            CapPart cp;
+            for (Array *a : kv.second) cp.rd.push_back(a);
+            cp.lane = kArrayLane;
+            cp.launch = [table, n](cudaStream_t q) { return agocuda_array_download_batch(q, table, n); };
+            parts.push_back(std::move(cp));
+            table += n;
+            downloads++;
+        }
+    }
 
     // the array transfers are kernels of the CUDA graph too: list them with the plan
     if (!g->staged_in.empty()) g->plan_text += "array_upload_batch\t1\n";
     if (!g->staged_out.empty())
-        g->plan_text += "array_download x" + std::to_string(g->staged_out.size()) + "\t" +
-                        std::to_string(g->staged_out.size()) + "\n";
+        g->plan_text += "array_download x" + std::to_string(g->staged_out.size()) + "\t" + std::to_string(downloads) + "\n";
 
     // ---- dependencies: read-after-write, write-after-write, write-after-read
     std::map<Ref *, int> last_writer;

@@ -228,9 +228,11 @@ __global__ void __launch_bounds__(kHalfThreads) k_gauss_half_one(const agocuda_h
 // TMA-staged form: a block of 112 threads produces 112 output columns x 32 output rows of one
 // level.  One tensor copy brings the source box -- columns 2*ox0-16 .. 2*ox0+239, rows
 // 2*oy0+ro-2 .. +67 -- into shared memory (completion on an mbarrier, bounded wait; the box
-// start column is a multiple of 16 bytes); box columns outside the row are then rewritten with
-// the bytes AGO's buffer layout holds there (ago_byte), so every output equals the register
-// form's.  A thread computes 8 output columns x 4 output rows from shared-memory words.
+// start column is a multiple of 16 bytes); the four columns outside the row that outputs read
+// are then rewritten with the bytes AGO's buffer layout holds there, so every output equals the
+// register form's.  Most launches are one partial wave, so a tile's own latency counts: one warp
+// finds the job in one load and starts the copy, and only those four columns are looked at (16 and
+// more, by 64-bit divisions, before: 12 us for the smallest level).  A thread computes 8 output columns x 4 output rows from shared-memory words.
 // ---------------------------------------------------------------------------------
 constexpr int kHtCols = 112, kHtRows = 32, kHtThreads = 112;
 constexpr int kHtGroups = kHtCols / 8;                  // 14 column groups of 8 outputs
@@ -293,30 +295,39 @@ __global__ void __launch_bounds__(kHtThreads) k_gauss_half_tma(const agocuda_hal
 {
     __shared__ __align__(128) uint8_t tile[kHtBoxH][kHtBoxW];
     __shared__ __align__(8) uint64_t bar;
-    uint32_t lo = 0, hi = numJobs - 1;
+    __shared__ uint32_t sJob;
     const uint32_t t = blockIdx.x;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].tileBegin <= t) lo = mid; else hi = mid - 1;
+    const int tid = threadIdx.x;
+    const uint32_t b = smem_addr_u32(&bar);
+    // warp 0: the job owning this tile (jobs are sorted by tileBegin; 32 of them per step, one
+    // load deep), then the copy of its source box
+    if (tid < 32) {
+        uint32_t lo = 0;
+        for (uint32_t j0 = 0; j0 < numJobs; j0 += 32) {
+            const uint32_t j = j0 + tid;
+            const unsigned m = __ballot_sync(0xffffffffu, j < numJobs && jobs[j].tileBegin <= t);
+            if (m) lo = j0 + 31 - __clz(m);
+            if (m != 0xffffffffu) break;
+        }
+        if (tid == 0) {
+            const agocuda_half_job &J = jobs[lo];
+            const uint32_t local = t - J.tileBegin, tilesX = (J.dstW + kHtCols - 1) / kHtCols;
+            const int x = 2 * (int)(local % tilesX) * kHtCols - 16, y = 2 * (int)(local / tilesX) * kHtRows + ((J.srcH & 1) ? 0 : 1) - 2;
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(kHtBoxW * kHtBoxH) : "memory");
+            asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                         ::"r"(smem_addr_u32(&tile[0][0])), "l"((uint64_t)(maps + lo)), "r"(x), "r"(y), "r"(b) : "memory");
+            sJob = lo;
+        }
     }
-    const agocuda_half_job J = jobs[lo];
+    __syncthreads();
+    const agocuda_half_job J = jobs[sJob];
     const uint32_t local = t - J.tileBegin;
     const uint32_t tilesX = (J.dstW + kHtCols - 1) / kHtCols;
     const int ox0 = (int)(local % tilesX) * kHtCols, oy0 = (int)(local / tilesX) * kHtRows;
     const int ro = (J.srcH & 1) ? 0 : 1;
     const int sx0 = 2 * ox0 - 16, sy0 = 2 * oy0 + ro - 2;
-    const int tid = threadIdx.x;
-    const uint32_t b = smem_addr_u32(&bar);
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (tid == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(kHtBoxW * kHtBoxH) : "memory");
-        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                     ::"r"(smem_addr_u32(&tile[0][0])), "l"((uint64_t)(maps + lo)), "r"(sx0), "r"(sy0), "r"(b) : "memory");
-    }
     bool done = false;
     for (int i = 0; i < kHtWaitLimit && !done; i++) done = mbarrier_try_wait_parity(b, 0);
     if (!done) {
@@ -324,18 +335,16 @@ __global__ void __launch_bounds__(kHtThreads) k_gauss_half_tma(const agocuda_hal
         for (int i = 0; i < kHtWaitLimit && !done; i++) done = mbarrier_try_wait_parity(b, 0);
         return;
     }
-    // box columns the tile reads that lie outside the row take AGO's bytes: 16 on the left at
-    // most, on the right from the row end to the last column read
-    const int W = (int)J.srcW, H = (int)J.srcH;
-    const int cEnd = min(kHtBoxW, 2 * (min(ox0 + kHtCols, (int)J.dstW) - ox0) + 36);
-    const int lEnd = max(0, min(-sx0, cEnd)), rBeg = max(W - sx0, 0);
-    const int nL = lEnd, nR = max(0, cEnd - rBeg), per = nL + nR;
-    if (per > 0) {
-        const int rows = min(kHtBoxH, 2 * (min(oy0 + kHtRows, (int)J.dstH) - oy0) + 4);
-        for (int i = tid; i < rows * per; i += kHtThreads) {
-            const int r = i / per, k = i - r * per;
-            const int c = k < nL ? k : rBeg + (k - nL);
-            tile[r][c] = (uint8_t)ago_byte(J.src, (size_t)J.srcStride, W, H, sy0 + r, sx0 + c);
+    // The outputs read columns -2, -1, W and W + 1 outside the row.  TMA filled them with zeros,
+    // as AGO's layout does except where the row's pitch ends within two bytes of its pixels
+    // (W % 16 is 0 or 15): there they are the neighbouring rows' last and first pixels.
+    const int W = (int)J.srcW, H = (int)J.srcH, S = (W + 15) & ~15;
+    if (S - W <= 1 && (sx0 < 0 || sx0 + kHtBoxW > W)) {
+        for (int i = tid; i < 4 * kHtBoxH; i += kHtThreads) {
+            const int r = i >> 2, k = i & 3, c = k < 2 ? k - 2 : W + k - 2;
+            const int rr = sy0 + r + (k < 2 ? -1 : 1), cc = c + (k < 2 ? S : -S);
+            if (c >= sx0 && c < sx0 + kHtBoxW)
+                tile[r][c - sx0] = rr >= 0 && rr < H && cc >= 0 && cc < W ? J.src[(size_t)rr * J.srcStride + cc] : 0;
         }
         __syncthreads();
     }
@@ -918,8 +927,10 @@ __global__ void __launch_bounds__(kL9Warps * 32, 4) k_lk_track9(agocuda_lk_frame
         if (__any_sync(kAll, whole)) {
             // integer path: int sums of columns 0..3, of 4..7 and column 8, added in that order
             float c11 = 0.f, c12 = 0.f, c22 = 0.f;
+            const int across1 = base + (kk ^ 1), across2 = base + (kk ^ 2);   // of lanes 0..3; lane 4's sum is not used
             auto sum4 = [&](int v) {
-                return __shfl_sync(kAll, v, base) + __shfl_sync(kAll, v, base + 1) + __shfl_sync(kAll, v, base + 2) + __shfl_sync(kAll, v, base + 3);
+                const int s = v + __shfl_sync(kAll, v, across1);
+                return s + __shfl_sync(kAll, s, across2);
             };
 #pragma unroll
             for (int i = 0; i < win; i++) {
@@ -935,6 +946,9 @@ __global__ void __launch_bounds__(kL9Warps * 32, 4) k_lk_track9(agocuda_lk_frame
                 c12 = __fadd_rn(c12, (float)(x * y));
                 c22 = __fadd_rn(c22, (float)(y * y));
             }
+            c11 = __shfl_sync(kAll, c11, base);            // lane 4 has no sums of its own
+            c12 = __shfl_sync(kAll, c12, base);
+            c22 = __shfl_sync(kAll, c22, base);
             if (whole) { A11 = c11; A12 = c12; A22 = c22; }
         }
         A11 = __fmul_rn(A11, kFltScale);
@@ -1252,44 +1266,48 @@ extern "C" size_t agocuda_OpticalFlowPyrLK_scharr_rows_size(uint32_t width0)
     return ((size_t)2 * width0 + 32) * sizeof(uint16_t);
 }
 
-static int lk_batch(void *stream, agocuda_lk_frame *frames, uint32_t numFrames, uint32_t maxPoints, bool win9, uint32_t *pStatus)
+static int lk_batch(void *stream, agocuda_lk_frame *frames, uint32_t numFrames, uint32_t maxPoints, uint32_t hints, uint32_t *pStatus)
 {
     if (!frames || !numFrames || !pStatus) return AGOCUDA_INVALID_PARAMS;
     cudaStream_t s = as_stream(stream);
     k_lk_prep<<<numFrames, 1024, 0, s>>>(frames, pStatus);
     agocuda_count_launch(1);
     if (maxPoints) {
-        if (win9)
+        if (hints & AGOCUDA_LK_HINT_WINDOW9)
             k_lk_track9<<<dim3(div_up(maxPoints, kL9Warps * kL9Points), numFrames), kL9Warps * 32, 0, s>>>(frames);
         else
             k_lk_track<<<dim3((maxPoints + kLkWarps - 1) / kLkWarps, numFrames), kLkWarps * 32, 0, s>>>(frames, pStatus);
         agocuda_count_launch(1);
     }
-    k_lk_carry<<<numFrames, 256, 0, s>>>(frames);
-    agocuda_count_launch(1);
+    if (!(hints & AGOCUDA_LK_HINT_NO_CARRY)) {
+        k_lk_carry<<<numFrames, 256, 0, s>>>(frames);
+        agocuda_count_launch(1);
+    }
     return agocuda_launch_status();
 }
 
 extern "C" int agocuda_OpticalFlowPyrLK_batch(void *stream, agocuda_lk_frame *frames, uint32_t numFrames,
                                               uint32_t maxPoints, uint32_t *pStatus)
 {
-    return lk_batch(stream, frames, numFrames, maxPoints, false, pStatus);
+    return lk_batch(stream, frames, numFrames, maxPoints, 0, pStatus);
 }
 
-// five lanes per point (k_lk_track9) for a 9x9 window over planes of aligned 32-bit words
-extern "C" int agocuda_OpticalFlowPyrLK_window9(const agocuda_lk_frame *frame)
+extern "C" uint32_t agocuda_OpticalFlowPyrLK_hints(const agocuda_lk_frame *frame)
 {
-    if (!frame || frame->windowDimension != 9) return 0;
-    for (uint32_t l = 0; l < frame->levels && l < AGOCUDA_LK_MAX_LEVELS; l++)
-        if ((((uintptr_t)frame->oldPyr[l].image | frame->oldPyr[l].stride | (uintptr_t)frame->newPyr[l].image | frame->newPyr[l].stride) & 3))
-            return 0;
-    return 1;
+    if (!frame || frame->levels > AGOCUDA_LK_MAX_LEVELS) return 0;
+    uint32_t h = AGOCUDA_LK_HINT_NO_CARRY | (frame->windowDimension == 9 ? AGOCUDA_LK_HINT_WINDOW9 : 0);
+    for (uint32_t l = 0; l < frame->levels; l++) {
+        if (((uintptr_t)frame->oldPyr[l].image | frame->oldPyr[l].stride | (uintptr_t)frame->newPyr[l].image | frame->newPyr[l].stride) & 3)
+            h &= ~AGOCUDA_LK_HINT_WINDOW9;
+        if (l > 0 && (frame->oldPyr[l].width & 7) > 2) h &= ~AGOCUDA_LK_HINT_NO_CARRY;
+    }
+    return h;
 }
 
-extern "C" int agocuda_OpticalFlowPyrLK_batch_window9(void *stream, agocuda_lk_frame *frames, uint32_t numFrames,
-                                                      uint32_t maxPoints, uint32_t *pStatus)
+extern "C" int agocuda_OpticalFlowPyrLK_batch_hints(void *stream, agocuda_lk_frame *frames, uint32_t numFrames,
+                                                    uint32_t maxPoints, uint32_t hints, uint32_t *pStatus)
 {
-    return lk_batch(stream, frames, numFrames, maxPoints, true, pStatus);
+    return lk_batch(stream, frames, numFrames, maxPoints, hints, pStatus);
 }
 
 extern "C" size_t agocuda_OpticalFlowPyrLK_carry_size(uint32_t levels, uint32_t height1)
@@ -1358,5 +1376,5 @@ extern "C" int agocuda_OpticalFlowPyrLK_XY_XY(void *stream, void *newKeyPoint, u
     agocuda_count_launch(1);
     const int rc = agocuda_launch_status();
     if (rc) return rc;
-    return lk_batch(stream, dev, 1, newCapacity, agocuda_OpticalFlowPyrLK_window9(&F) != 0, pStatus);
+    return lk_batch(stream, dev, 1, newCapacity, agocuda_OpticalFlowPyrLK_hints(&F), pStatus);
 }

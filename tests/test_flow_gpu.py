@@ -272,3 +272,38 @@ def test_lk_rejects_mismatched_counts(lib):
             stream_ptr(), d_out.data_ptr(), n, cnt.data_ptr() + 8, scale, levels, level_descs(old_lv),
             level_descs(new_lv), cnt.data_ptr(), d_old.data_ptr(), cnt.data_ptr() + 4, d_est.data_ptr(), PF.TERM_BOTH,
             0.01, 20, 0, win, sbase, scratch.numel() - 256, status.data_ptr()) == -10
+
+
+# full-contrast blocks (0 / 255), moved: gradients and differences at their extremes, where a
+# product passes 2^24 and the reference's float conversion rounds it; one point, and counts that
+# leave lanes and warps part-filled
+@pytest.mark.parametrize("W,H,cell,n", [(64, 40, 2, 1), (107, 61, 3, 25), (333, 97, 4, 601), (640, 480, 6, 500)])
+def test_lk_window9_full_contrast(lib, W, H, cell, n):
+    import torch
+
+    from devbuf import stream_ptr
+    levels, term, eps, iters, win = 3, PF.TERM_ITER, 0.01, 12, 9
+    rng = np.random.default_rng(W)
+    big = np.kron(rng.integers(0, 2, (H // cell + 4, W // cell + 4)), np.ones((cell, cell), np.int64)) * 255
+    f1, f2 = big[:H, :W].astype(np.uint8), big[2:H + 2, 1:W + 1].astype(np.uint8)
+    kp = PF.points(W + H, W, H, n)
+    size = lib.agocuda_OpticalFlowPyrLK_scratch_size_carry(W, H, levels)
+    scratch = torch.zeros(size + 256, dtype=torch.uint8, device="cuda")
+    sbase = scratch.data_ptr() + (-scratch.data_ptr() % 256)
+    oscratch = PF.lk_scratch(W, H, n)
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    for call in range(2):
+        a, b = (f1, f2) if call == 0 else (f2, 255 - f1)
+        old_lv, new_lv = gpu_pyramid(lib, a, levels), gpu_pyramid(lib, b, levels)
+        d_old, d_est = dev_bytes(kp), dev_bytes(kp)
+        out = np.zeros(n, KP)
+        out.view(np.uint8)[:] = 0xA5
+        d_out = dev_bytes(out)
+        cnt = torch.tensor([n, n, 0, 0], dtype=torch.int32, device="cuda")
+        assert lib.agocuda_OpticalFlowPyrLK_XY_XY(
+            stream_ptr(), d_out.data_ptr(), n, cnt.data_ptr() + 8, 0.5, levels, level_descs(old_lv), level_descs(new_lv),
+            cnt.data_ptr(), d_old.data_ptr(), cnt.data_ptr() + 4, d_est.data_ptr(), term, eps, iters, 0, win,
+            sbase, scratch.numel() - 256, status.data_ptr()) == 0
+        got = d_out.cpu().numpy().view(KP)
+        want = oracle_lk(a, b, levels, kp, kp, term, eps, iters, 0, win, oscratch)
+        np.testing.assert_array_equal(got, want)
