@@ -450,12 +450,13 @@ int agocuda_fused_HarrisCorners_3x3(void *stream, uint32_t width, uint32_t heigh
                                     void *pCorners, uint32_t cornerCapacity, uint32_t *pCornerCount,
                                     uint32_t *pNumCorners, void *scratch, size_t scratchBytes, uint32_t *pStatus);
 
-/* The same for every gradient and block size of {3, 5, 7}; scratch as above. */
+/* The same for every gradient and block size of {3, 5, 7}; scratch as above.  framesInFlight: how
+ * many such calls the caller runs side by side (it picks the strip height of the 3x3 form). */
 int agocuda_fused_HarrisCorners_NxN(void *stream, uint32_t width, uint32_t height, const uint8_t *pSrc, uint32_t srcStride,
                                     uint32_t gradientSize, uint32_t blockSize, float sensitivity, float strengthThreshold,
                                     float normFactor, float minDistance, void *pCorners, uint32_t cornerCapacity,
                                     uint32_t *pCornerCount, uint32_t *pNumCorners, void *scratch, size_t scratchBytes,
-                                    uint32_t *pStatus);
+                                    uint32_t framesInFlight, uint32_t *pStatus);
 
 /* ---------------------------------------------------------------- differentiable F32 warps */
 /* F32 bilinear WarpAffine / Remap with a constant border and their adjoints, for batches of

@@ -1047,6 +1047,7 @@ static vx_status build_fused_batch(Graph *g, std::vector<Chain> &chains, Step &s
     }
     if (chains[0].kind == "fused_CannyEdgeDetector" || chains[0].kind == "fused_HarrisCorners") {
         // one step holding every frame's launches (one CUDA graph segment)
+        const uint32_t frames = (uint32_t)chains.size();
         std::vector<std::function<int(cudaStream_t)>> fns;
         st.name = chains[0].kind + " x" + std::to_string(chains.size());
         st.num_kernels = 0;
@@ -1087,7 +1088,7 @@ static vx_status build_fused_batch(Graph *g, std::vector<Chain> &chains, Step &s
                 void *scr = scratch(g, sb);
                 if (!scr) return VX_ERROR_NO_MEMORY;
                 fns.push_back([=](cudaStream_t q) {
-                    return agocuda_fused_HarrisCorners_NxN(S(q), w, h, src, ss, gs, bs, k, tc, norm, mind, out, ocap, oc, nc, scr, sb, status);
+                    return agocuda_fused_HarrisCorners_NxN(S(q), w, h, src, ss, gs, bs, k, tc, norm, mind, out, ocap, oc, nc, scr, sb, frames, status);
                 });
                 st.parts.push_back(Part{fns.back(), c.nodes});
                 st.num_kernels += 3;

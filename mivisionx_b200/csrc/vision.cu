@@ -1100,8 +1100,9 @@ __global__ void k_harris_nms(int W, int H, const float *sc, int scStride, uint64
 }
 
 // Harris front end as column strips: a warp owns 120 output columns (lanes 1..30, four
-// columns each; lanes 0 and 31 carry the halo) and walks down 32 output rows with rolling
-// registers.  Per input row a lane loads one word; the Sobel sums run in 16-bit lanes
+// columns each; lanes 0 and 31 carry the halo) and walks down `rows` output rows with rolling
+// registers (64 where the frames in flight fill the device with such strips, fewer where they
+// do not: harris_rows).  Per input row a lane loads one word; the Sobel sums run in 16-bit lanes
 // (four columns in four registers), the products and window sums in float -- integers
 // below 2^24, i.e. exactly the float sums the reference forms in any order.  The score
 // keeps the reference's float operation order, and its division is skipped only where the
@@ -1120,7 +1121,7 @@ __device__ __forceinline__ uint32_t harris_word(const uint8_t *src, int stride, 
 __device__ __forceinline__ float lane_lo(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7610)) - 8389632.0f; }
 __device__ __forceinline__ float lane_hi(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7632)) - 8389632.0f; }
 
-// TMA form: each warp copies its source rows ys-3 .. ys+kHRows+2, columns from (xs-4) rounded
+// TMA form: each warp copies its source rows ys-3 .. ys+rows+2, columns from (xs-4) rounded
 // down to 16 bytes, 144 bytes wide, into shared memory with one tensor copy on its own
 // mbarrier (the warps of a block are independent)
 constexpr int kHBoxW = 144, kHBoxH = kHRows + 6;
@@ -1128,14 +1129,14 @@ constexpr int kHBoxSlot = (kHBoxH * kHBoxW + 127) & ~127;   // a TMA destination
 
 template <bool TMA>
 __global__ void __launch_bounds__(128)
-k_harris_rows(int W, int H, const uint8_t *__restrict__ src, int srcStride, float k, float Tc, float norm,
+k_harris_rows(int W, int H, int rows, const uint8_t *__restrict__ src, int srcStride, float k, float Tc, float norm,
               uint64_t *list, uint32_t *count, uint32_t capacity, uint32_t *pStatus, const __grid_constant__ CUtensorMap map)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int xs = (blockIdx.x * (blockDim.x >> 5) + wib) * kHCols;
     if (xs >= W) return;                                   // warp-uniform
     const int xl = xs - 4 + 4 * lane;                      // this lane's columns xl .. xl+3
-    const int ys = blockIdx.y * kHRows, yEnd = min(ys + kHRows, H);
+    const int ys = blockIdx.y * rows, yEnd = min(ys + rows, H), boxH = rows + 6;
     const bool fast = ((((uintptr_t)src | (uintptr_t)srcStride) & 3) == 0) && xl >= 0 && xl + 4 <= W;
     __shared__ __align__(128) uint8_t sBox[TMA ? 4 : 1][TMA ? kHBoxSlot : 16];
     static_assert(kHBoxSlot % 128 == 0, "each warp's box starts on a 128-byte boundary");
@@ -1146,7 +1147,7 @@ k_harris_rows(int W, int H, const uint8_t *__restrict__ src, int srcStride, floa
         if (lane == 0) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(kHBoxH * kHBoxW) : "memory");
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(boxH * kHBoxW) : "memory");
             asm volatile(
                 "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                 ::"r"(smem_addr_u32(sBox[wib])), "l"((uint64_t)&map), "r"(bx), "r"(ys - 3), "r"(b) : "memory");
@@ -1164,7 +1165,7 @@ k_harris_rows(int W, int H, const uint8_t *__restrict__ src, int srcStride, floa
         // (W % 16 == 0): column -1 is the previous row's last pixel, column W the next row's first
         if ((W & 15) == 0) {
             uint8_t *row = sBox[wib];
-            for (int i = lane; i < kHBoxH; i += 32) {
+            for (int i = lane; i < boxH; i += 32) {
                 const int y = ys - 3 + i;
                 if (bx < 0) row[i * kHBoxW - 1 - bx] = (y >= 1 && y < H) ? src[(size_t)(y - 1) * srcStride + W - 1] : 0;
                 if (W - bx < kHBoxW) row[i * kHBoxW + W - bx] = (y >= 0 && y + 1 < H) ? src[(size_t)(y + 1) * srcStride] : 0;
@@ -2163,10 +2164,23 @@ extern "C" int agocuda_HarrisMergeSortAndPick_XY_XYS(void *stream, uint32_t W, u
 // one pixel of every 2x2 block survives.
 static uint32_t harris_list_capacity(uint32_t W, uint32_t H) { return ((W + 1) / 2) * ((H + 1) / 2); }
 
-extern "C" int agocuda_fused_HarrisCorners_3x3(void *stream, uint32_t W, uint32_t H, const uint8_t *pSrc, uint32_t srcStride,
+// Rows per strip.  A strip repeats 6 halo rows (three extra steps each end), so 64 rows cost the
+// least work; but each strip is one warp's serial walk (35 us for 64 rows), and one 720p frame
+// has only 132 of them.  The most rows that still give `kHMinWarps` warps over the frames in
+// flight: one 720p frame 8 rows, one 1080p frame 16, 4K frames and batches 64.
+constexpr int kHMinWarps = 888;      // 6 per SM
+static int harris_rows(int strips, int H, uint32_t framesInFlight)
+{
+    int rows = kHRows;
+    while (rows > 8 && (long long)strips * div_up(H, rows) * min(framesInFlight, 8u) < kHMinWarps) rows >>= 1;
+    return rows;
+}
+
+static int harris_3x3(void *stream, uint32_t W, uint32_t H, const uint8_t *pSrc, uint32_t srcStride,
                                                float sensitivity, float strengthThreshold, float normFactor, float minDistance,
                                                void *pCorners, uint32_t cornerCapacity, uint32_t *pCornerCount,
-                                               uint32_t *pNumCorners, void *scratch, size_t scratchBytes, uint32_t *pStatus)
+                                               uint32_t *pNumCorners, void *scratch, size_t scratchBytes,
+                                               uint32_t framesInFlight, uint32_t *pStatus)
 {
     const uint32_t cap = harris_list_capacity(W, H);
     const size_t listBytes = pick_align((size_t)cap * 8);
@@ -2183,12 +2197,13 @@ extern "C" int agocuda_fused_HarrisCorners_3x3(void *stream, uint32_t W, uint32_
     // the map is a kernel parameter, so a captured launch keeps it
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
-    const dim3 grd(div_up(strips, 4), div_up(H, kHRows));
-    if (agocuda_u8_tensor_map(&map, pSrc, W, H, srcStride, kHBoxW, kHBoxH))
-        k_harris_rows<true><<<grd, 128, 0, s>>>((int)W, (int)H, pSrc, (int)srcStride, sensitivity, strengthThreshold,
+    const int rows = harris_rows(strips, (int)H, framesInFlight);
+    const dim3 grd(div_up(strips, 4), div_up(H, rows));
+    if (agocuda_u8_tensor_map(&map, pSrc, W, H, srcStride, kHBoxW, rows + 6))
+        k_harris_rows<true><<<grd, 128, 0, s>>>((int)W, (int)H, rows, pSrc, (int)srcStride, sensitivity, strengthThreshold,
                                                 normFactor, list, cnt, cap, pStatus, map);
     else
-        k_harris_rows<false><<<grd, 128, 0, s>>>((int)W, (int)H, pSrc, (int)srcStride, sensitivity, strengthThreshold,
+        k_harris_rows<false><<<grd, 128, 0, s>>>((int)W, (int)H, rows, pSrc, (int)srcStride, sensitivity, strengthThreshold,
                                                  normFactor, list, cnt, cap, pStatus, map);
     agocuda_count_launch(1);
     int rc = agocuda_launch_status();
@@ -2196,6 +2211,15 @@ extern "C" int agocuda_fused_HarrisCorners_3x3(void *stream, uint32_t W, uint32_
     return agocuda_HarrisMergeSortAndPick_XY_XYS(stream, W, H, list, cnt, cap, minDistance, pCorners, cornerCapacity,
                                                  pCornerCount, pNumCorners, pickScratch,
                                                  agocuda_HarrisMergeSortAndPick_scratch_size(W, H, cap, minDistance), pStatus);
+}
+
+extern "C" int agocuda_fused_HarrisCorners_3x3(void *stream, uint32_t W, uint32_t H, const uint8_t *pSrc, uint32_t srcStride,
+                                               float sensitivity, float strengthThreshold, float normFactor, float minDistance,
+                                               void *pCorners, uint32_t cornerCapacity, uint32_t *pCornerCount,
+                                               uint32_t *pNumCorners, void *scratch, size_t scratchBytes, uint32_t *pStatus)
+{
+    return harris_3x3(stream, W, H, pSrc, srcStride, sensitivity, strengthThreshold, normFactor, minDistance, pCorners,
+                      cornerCapacity, pCornerCount, pNumCorners, scratch, scratchBytes, 1, pStatus);
 }
 
 extern "C" size_t agocuda_fused_HarrisCorners_scratch_size(uint32_t W, uint32_t H, float minDistance)
@@ -2241,7 +2265,7 @@ extern "C" int agocuda_fused_HarrisCorners_NxN(void *stream, uint32_t W, uint32_
                                                uint32_t gradientSize, uint32_t blockSize, float sensitivity,
                                                float strengthThreshold, float normFactor, float minDistance, void *pCorners,
                                                uint32_t cornerCapacity, uint32_t *pCornerCount, uint32_t *pNumCorners,
-                                               void *scratch, size_t scratchBytes, uint32_t *pStatus)
+                                               void *scratch, size_t scratchBytes, uint32_t framesInFlight, uint32_t *pStatus)
 {
     const uint32_t G = gradientSize, B = blockSize, cap = harris_list_capacity(W, H), least = G > B ? G : B;
     if (!pSrc || !pCorners || !pCornerCount || !scratch || !pStatus || W < least || H < least || srcStride < W ||
@@ -2249,8 +2273,8 @@ extern "C" int agocuda_fused_HarrisCorners_NxN(void *stream, uint32_t W, uint32_
         scratchBytes < agocuda_fused_HarrisCorners_scratch_size(W, H, minDistance) || !aligned(scratch, 256))
         return AGOCUDA_INVALID_PARAMS;
     if (G == 3 && B == 3)
-        return agocuda_fused_HarrisCorners_3x3(stream, W, H, pSrc, srcStride, sensitivity, strengthThreshold, normFactor, minDistance,
-                                               pCorners, cornerCapacity, pCornerCount, pNumCorners, scratch, scratchBytes, pStatus);
+        return harris_3x3(stream, W, H, pSrc, srcStride, sensitivity, strengthThreshold, normFactor, minDistance, pCorners,
+                          cornerCapacity, pCornerCount, pNumCorners, scratch, scratchBytes, framesInFlight, pStatus);
     uint32_t *cnt = (uint32_t *)scratch;
     uint64_t *list = (uint64_t *)((uint8_t *)scratch + 256);
     void *pickScratch = (uint8_t *)scratch + 256 + pick_align((size_t)cap * 8);
