@@ -15,9 +15,10 @@
 // appends with atomics; this one keeps the CPU path's order.
 //
 // Four launches: k_fast_map (strengths / flags, one 128x8 tile per CTA staged in shared
-// memory), k_fast_rows (a warp per row: suppression, ballot bitmap and row count),
-// k_fast_scan (one CTA: row offsets and counts) and k_fast_emit (a warp per row writes its
-// keypoints at its offset).
+// memory), k_fast_rows (a warp per row, a lane per 32 pixels: suppression, bitmap and row
+// count), k_fast_scan (one CTA: row offsets and counts) and k_fast_emit (a warp per row writes
+// its keypoints at its offset, a lane per bitmap word).  Corners are rare, so what bounds the map
+// is the circle test itself: it runs on the four pixels of a word at once, one byte each.
 #include "agocuda_internal.cuh"
 
 uint64_t agocuda_count_launch(unsigned n);
@@ -41,6 +42,24 @@ __device__ __forceinline__ bool arc9(uint32_t m)
     return (a & 0xFFFFu) != 0;
 }
 
+// bit 7 of each byte: a > b (the average of a and ~b, rounded down, is at least 128)
+__device__ __forceinline__ uint32_t gt4(uint32_t a, uint32_t b)
+{
+    const uint32_t n = ~b;
+    return (a & n) + (((a ^ n) & 0xfefefefeu) >> 1);
+}
+
+// bit 7 of each byte: bit 7 set in nine consecutive words of the circle f
+__device__ __forceinline__ uint32_t arc9x4(const uint32_t f[16])
+{
+    uint32_t a3[16], any = 0;
+#pragma unroll
+    for (int i = 0; i < 16; i++) a3[i] = f[i] & f[(i + 1) & 15] & f[(i + 2) & 15];
+#pragma unroll
+    for (int i = 0; i < 16; i++) any |= a3[i] & a3[(i + 3) & 15] & a3[(i + 6) & 15];
+    return any;
+}
+
 // max over the 16 circular windows of 9 of the window minimum of d
 __device__ __forceinline__ int best_arc_min(const int d[16])
 {
@@ -59,7 +78,12 @@ __device__ __forceinline__ int best_arc_min(const int d[16])
 
 // map: suppression -> strength (0 = no corner) for rows 3..H-4, columns 3..W-4; otherwise 1 for
 // a corner in rows 3..H-4 (every column).  Every other pixel of the map is written 0.
-template <bool SUP>
+//
+// PACKED (t >= 0): the tests c + t < p and p < c - t of the four pixels of a word in byte lanes,
+// with saturated bounds (a bound of 255 or 0 is never passed, as the unsaturated one); the arcs
+// by ANDs of the 16 circle words.  One pixel at a time took 16 byte loads and 32 compares each:
+// 25 us per 1080p frame.  Negative thresholds take the other form.
+template <bool SUP, bool PACKED>
 __global__ void __launch_bounds__(256) k_fast_map(int W, int H, const uint8_t *src, int srcStride, int t, uint8_t *map,
                                                  int mapStride)
 {
@@ -83,9 +107,36 @@ __global__ void __launch_bounds__(256) k_fast_map(int W, int H, const uint8_t *s
     const int y = y0 + threadIdx.y;
     if (y >= H) return;
     const int lx0 = 4 * threadIdx.x;
-    uint32_t out = 0;
+    uint32_t out = 0, plus4 = 0, minus4 = 0;
+    if constexpr (PACKED) {
+        uint32_t f[16], g[16], c = 0, hi = 0, lo = 0;
+        const uint32_t T = (uint32_t)min(t, 255) * 0x01010101u;
+        auto row = [&](int dy, uint32_t w[3]) {
+            const uint32_t *p = (const uint32_t *)&tile[3 + threadIdx.y + dy][lx0];
+            w[0] = p[0]; w[1] = p[1]; w[2] = p[2];
+        };
+        auto at = [](const uint32_t w[3], int dx) {        // the four pixels dx columns to the right
+            return dx == 0 ? w[1] : dx > 0 ? __funnelshift_r(w[1], w[2], 8 * dx) : __funnelshift_r(w[0], w[1], 32 + 8 * dx);
+        };
+        auto test = [&](int i, uint32_t v) { f[i] = gt4(v, hi); g[i] = gt4(lo, v); };
+        uint32_t w[3];
+        row(0, w);
+        c = w[1];
+        hi = __vaddus4(c, T);
+        lo = __vsubus4(c, T);
+        test(4, at(w, 3)); test(12, at(w, -3));
+        row(-3, w); test(15, at(w, -1)); test(0, at(w, 0)); test(1, at(w, 1));
+        row(3, w); test(9, at(w, -1)); test(8, at(w, 0)); test(7, at(w, 1));
+        row(-2, w); test(14, at(w, -2)); test(2, at(w, 2));
+        row(2, w); test(10, at(w, -2)); test(6, at(w, 2));
+        row(-1, w); test(13, at(w, -3)); test(3, at(w, 3));
+        row(1, w); test(11, at(w, -3)); test(5, at(w, 3));
+        plus4 = arc9x4(f) & 0x80808080u;
+        minus4 = arc9x4(g) & 0x80808080u;
+    }
 #pragma unroll
     for (int q = 0; q < 4; q++) {
+        if (PACKED && !(((plus4 | minus4) >> (8 * q)) & 0x80)) continue;
         const int x = x0 + lx0 + q;
         const bool cand = y >= 3 && y < H - 3 && x < W && (!SUP || (x >= 3 && x < W - 3));
         int v = 0;
@@ -95,14 +146,21 @@ __global__ void __launch_bounds__(256) k_fast_map(int W, int H, const uint8_t *s
             int b[16];
 #pragma unroll
             for (int i = 0; i < 16; i++) b[i] = tile[cy + kCircleDy[i]][cx + kCircleDx[i]];
-            const int hi = (int16_t)(c + t), lo = (int16_t)(c - t);
-            uint32_t plus = 0, minus = 0;
+            bool cp, cm;
+            if constexpr (PACKED) {
+                cp = (plus4 >> (8 * q)) & 0x80;
+                cm = (minus4 >> (8 * q)) & 0x80;
+            } else {
+                const int hi = (int16_t)(c + t), lo = (int16_t)(c - t);
+                uint32_t plus = 0, minus = 0;
 #pragma unroll
-            for (int i = 0; i < 16; i++) {
-                plus |= (uint32_t)(b[i] > hi) << i;
-                minus |= (uint32_t)(b[i] < lo) << i;
+                for (int i = 0; i < 16; i++) {
+                    plus |= (uint32_t)(b[i] > hi) << i;
+                    minus |= (uint32_t)(b[i] < lo) << i;
+                }
+                cp = arc9(plus);
+                cm = arc9(minus);
             }
-            const bool cp = arc9(plus), cm = arc9(minus);
             if (!SUP) {
                 v = cp || cm;
             } else if (cp || cm) {
@@ -129,7 +187,7 @@ __global__ void __launch_bounds__(256) k_fast_map(int W, int H, const uint8_t *s
     else for (int q = 0; q < mapStride - x; q++) d[q] = (uint8_t)(out >> (8 * q));
 }
 
-// one warp per row: the surviving corners of the row as a bitmap and their count
+// one warp per row, 32 pixels per lane: the surviving corners as a bitmap and their count
 template <bool SUP>
 __global__ void __launch_bounds__(256) k_fast_rows(int W, int H, const uint8_t *map, int mapStride, uint32_t *bitmap,
                                                   int words, uint32_t *rowCount)
@@ -137,24 +195,29 @@ __global__ void __launch_bounds__(256) k_fast_rows(int W, int H, const uint8_t *
     const int y = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (y >= H) return;
     uint32_t count = 0;
-    const uint8_t *row = map + (size_t)y * mapStride;
-    for (int w = 0; w < words; w++) {
-        const int x = 32 * w + lane;
-        bool keep = false;
-        if (y >= 3 && y < H - 3 && x < W) {
-            const int v = row[x];
-            if (!SUP) {
-                keep = v != 0;
-            } else if (v && x >= 3 && x < W - 3) {
-                const uint8_t *u = row - mapStride, *d = row + mapStride;
-                keep = v >= u[x - 1] && v >= u[x] && v >= u[x + 1] && v >= row[x - 1] && v > row[x + 1] && v > d[x - 1] &&
-                       v > d[x] && v > d[x + 1];
-            }
+    const uint8_t *row = map + (size_t)y * mapStride, *u = row - mapStride, *d = row + mapStride;
+    const bool in = y >= 3 && y < H - 3;
+    for (int w = lane; w < words; w += 32) {
+        uint32_t bits = 0;
+        const int x0 = 32 * w;
+        if (in) {
+            const uint4 a = *(const uint4 *)(row + x0);    // rows are whole 16-byte groups
+            const uint4 b = x0 + 32 <= mapStride ? *(const uint4 *)(row + x0 + 16) : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t v4[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                for (uint32_t m = v4[k], q = 0; m; m >>= 8, q++) {
+                    const int v = m & 0xff, x = x0 + 4 * k + q;
+                    if (!v || x >= W) continue;
+                    const bool keep = !SUP || (x >= 3 && x < W - 3 && v >= u[x - 1] && v >= u[x] && v >= u[x + 1] && v >= row[x - 1] &&
+                                               v > row[x + 1] && v > d[x - 1] && v > d[x] && v > d[x + 1]);
+                    bits |= (uint32_t)keep << (4 * k + q);
+                }
         }
-        const uint32_t bits = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) bitmap[(size_t)y * words + w] = bits;
+        bitmap[(size_t)y * words + w] = bits;
         count += __popc(bits);
     }
+    count = __reduce_add_sync(0xffffffffu, count);
     if (lane == 0) rowCount[y] = count;
 }
 
@@ -206,25 +269,28 @@ __global__ void __launch_bounds__(256) k_fast_emit(int W, int H, const uint8_t *
     if (y >= H) return;
     uint32_t at = rowStart[y];
     if (at >= capacity) return;
-    const uint32_t below = (1u << lane) - 1u;
-    for (int w = 0; w < words && at < capacity; w++) {
-        const uint32_t bits = bitmap[(size_t)y * words + w];
-        if ((bits >> lane) & 1u) {
-            const uint32_t i = at + __popc(bits & below);
-            if (i < capacity) {
-                const int x = 32 * w + lane;
-                vx_keypoint_like k;
-                k.x = x;
-                k.y = y;
-                k.strength = SUP ? (float)map[(size_t)y * mapStride + x] : threshold;
-                k.scale = 0.f;
-                k.orientation = 0.f;
-                k.tracking_status = 1;
-                k.error = 0.f;
-                corners[i] = k;
-            }
+    for (int w0 = 0; w0 < words && at < capacity; w0 += 32) {
+        uint32_t bits = w0 + lane < words ? bitmap[(size_t)y * words + w0 + lane] : 0;
+        const uint32_t n = __popc(bits);
+        uint32_t upTo = n;                                 // corners of the lanes up to this one
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, upTo, o);
+            if (lane >= o) upTo += v;
         }
-        at += __popc(bits);
+        for (uint32_t i = at + upTo - n; bits && i < capacity; i++, bits &= bits - 1) {
+            const int x = 32 * (w0 + lane) + __ffs(bits) - 1;
+            vx_keypoint_like k;
+            k.x = x;
+            k.y = y;
+            k.strength = SUP ? (float)map[(size_t)y * mapStride + x] : threshold;
+            k.scale = 0.f;
+            k.orientation = 0.f;
+            k.tracking_status = 1;
+            k.error = 0.f;
+            corners[i] = k;
+        }
+        at += __shfl_sync(0xffffffffu, upTo, 31);
     }
 }
 
@@ -276,10 +342,10 @@ extern "C" int agocuda_FastCorners_XY_U8(void *stream, uint32_t W, uint32_t H, c
     const unsigned g2 = div_up(H, 8);
     vx_keypoint_like *kp = (vx_keypoint_like *)pCorners;
     if (nonmaxSuppression) {
-        k_fast_map<true><<<g1, b1, 0, q>>>((int)W, (int)H, pSrc, (int)srcStride, t, s.map, s.mapStride);
+        (t >= 0 ? k_fast_map<true, true> : k_fast_map<true, false>)<<<g1, b1, 0, q>>>((int)W, (int)H, pSrc, (int)srcStride, t, s.map, s.mapStride);
         k_fast_rows<true><<<g2, 256, 0, q>>>((int)W, (int)H, s.map, s.mapStride, s.bitmap, s.words, s.rowCount);
     } else {
-        k_fast_map<false><<<g1, b1, 0, q>>>((int)W, (int)H, pSrc, (int)srcStride, t, s.map, s.mapStride);
+        (t >= 0 ? k_fast_map<false, true> : k_fast_map<false, false>)<<<g1, b1, 0, q>>>((int)W, (int)H, pSrc, (int)srcStride, t, s.map, s.mapStride);
         k_fast_rows<false><<<g2, 256, 0, q>>>((int)W, (int)H, s.map, s.mapStride, s.bitmap, s.words, s.rowCount);
     }
     k_fast_scan<<<1, 1024, 0, q>>>((int)H, s.rowCount, s.rowStart, cornerCapacity, pCornerCount, pNumCorners);

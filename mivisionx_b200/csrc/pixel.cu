@@ -1142,62 +1142,127 @@ extern "C" int agocuda_Lut_S16_S16(void *stream, uint32_t dstWidth, uint32_t dst
 
 // ---------------------------------------------------------------------------------
 // Integral image U8 -> U32 (HafCpu_IntegralImage_U32_U8, ago_haf_cpu_arithmetic.cpp:7057):
-// out(x, y) = sum of in(i, j) for i <= x, j <= y, modulo 2^32.  Three launches: row prefix
-// sums (a block per row), column totals of 32-row segments, then each segment's rows get
-// the totals of the segments above plus their running column sum.
+// out(x, y) = sum of in(i, j) for i <= x, j <= y, modulo 2^32, over tiles of 128 columns and 32
+// rows, a warp each.  Three launches: the tiles' row and column sums; for every row the sum of
+// everything left of each tile in the rows up to it (left), for every column the sum above
+// each tile (above, in place); then a tile's warp walks down its rows with the column sums of
+// four columns per lane, and out = left + the lanes' running prefix.  The output, which is most
+// of the traffic, is written once, 16 bytes per lane (row prefixes in place, read twice and
+// rewritten, took 38 us per 1080p frame).
 // ---------------------------------------------------------------------------------
 namespace {
 
-constexpr int kIiThreads = 256, kIiSeg = 32;
+constexpr int kIiCols = 128, kIiRows = 32, kIiWarps = 4;
 
-__global__ void __launch_bounds__(kIiThreads)
-k_integral_rows(int W, uint32_t *dst, int dstStride, const uint8_t *src, int srcStride)
+// scratch: column sums [tile row][W], row sums and left sums [tile column][H]
+struct IiScratch { uint32_t *cols, *rows, *left; int tx, ty; };
+
+// the four pixels from column x on (zeros from W on)
+__device__ __forceinline__ uint32_t ii_word(const uint8_t *row, int x, int W, bool words)
 {
-    __shared__ uint32_t warpSum[kIiThreads / 32];
-    const int y = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int per = (W + kIiThreads - 1) / kIiThreads, x0 = tid * per, x1 = min(x0 + per, W);
-    const uint8_t *s = src + (size_t)y * srcStride;
-    uint32_t *d = (uint32_t *)((uint8_t *)dst + (size_t)y * dstStride);
-    uint32_t sum = 0;
-    for (int x = x0; x < x1; x++) sum += s[x];
-    // exclusive prefix of the threads' sums
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
+    if (words && x + 4 <= W) return __ldg((const uint32_t *)(row + x));
+    uint32_t w = 0;
+    for (int k = 0; k < 4 && x + k < W; k++) w |= (uint32_t)row[x + k] << (8 * k);
+    return w;
+}
+
+__global__ void __launch_bounds__(kIiWarps * 32)
+k_integral_sums(int W, int H, const uint8_t *src, int srcStride, IiScratch S, bool words)
+{
+    const int t = blockIdx.x * kIiWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= S.tx * S.ty) return;
+    const int tx = t % S.tx, ty = t / S.tx, x = tx * kIiCols + 4 * lane, y0 = ty * kIiRows, n = min(kIiRows, H - y0);
+    const uint8_t *p = src + (size_t)y0 * srcStride;
+    uint32_t e = 0, o = 0, mine = 0;                       // 32 bytes of 255 fit a 16-bit lane
+#pragma unroll 8
+    for (int r = 0; r < kIiRows; r++) {
+        const uint32_t w = r < n ? ii_word(p + (size_t)r * srcStride, x, W, words) : 0u;
+        e += w & 0x00ff00ffu;
+        o += (w >> 8) & 0x00ff00ffu;
+        const uint32_t s = __reduce_add_sync(0xffffffffu, __dp4a(w, 0x01010101u, 0u));
+        if (lane == r) mine = s;
     }
-    if (lane == 31) warpSum[warp] = incl;
-    __syncthreads();
-    uint32_t base = 0;
-    for (int w = 0; w < warp; w++) base += warpSum[w];
-    uint32_t run = base + incl - sum;
-    for (int x = x0; x < x1; x++) { run += s[x]; d[x] = run; }
+    if (lane < n) S.rows[(size_t)tx * H + y0 + lane] = mine;
+    const uint32_t c[4] = {e & 0xffff, o & 0xffff, e >> 16, o >> 16};
+    for (int k = 0; k < 4 && x + k < W; k++) S.cols[(size_t)ty * W + x + k] = c[k];
 }
 
-__global__ void __launch_bounds__(kIiThreads)
-k_integral_seg_totals(int W, int H, const uint32_t *dst, int dstStride, uint32_t *totals)
+// blocks [0, tx): left sums of tile column blockIdx.x, scanned down the rows; the others: the
+// columns' sums above each tile row
+__global__ void __launch_bounds__(1024) k_integral_scan(int W, int H, IiScratch S)
 {
-    const int x = blockIdx.x * kIiThreads + threadIdx.x, seg = blockIdx.y;
-    if (x >= W) return;
-    const int y0 = seg * kIiSeg, y1 = min(y0 + kIiSeg, H);
-    uint32_t t = 0;
-    for (int y = y0; y < y1; y++) t += ((const uint32_t *)((const uint8_t *)dst + (size_t)y * dstStride))[x];
-    totals[(size_t)seg * W + x] = t;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if ((int)blockIdx.x >= S.tx) {
+        const int x = ((int)blockIdx.x - S.tx) * 1024 + tid;
+        if (x >= W) return;
+        uint32_t run = 0;
+#pragma unroll 4
+        for (int t = 0; t < S.ty; t++) {
+            const uint32_t v = S.cols[(size_t)t * W + x];
+            S.cols[(size_t)t * W + x] = run;
+            run += v;
+        }
+        return;
+    }
+    __shared__ uint32_t warpSum[32];
+    uint32_t before = 0;
+    for (int y0 = 0; y0 < H; y0 += 1024) {
+        const int y = y0 + tid;
+        uint32_t v = 0;
+        if (y < H)
+#pragma unroll 4
+            for (int t = 0; t < (int)blockIdx.x; t++) v += S.rows[(size_t)t * H + y];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        if (lane == 31) warpSum[wid] = v;
+        __syncthreads();
+        uint32_t w = warpSum[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += u;
+        }
+        const uint32_t lower = __shfl_sync(0xffffffffu, w, (wid + 31) & 31), all = __shfl_sync(0xffffffffu, w, 31);
+        if (y < H) S.left[(size_t)blockIdx.x * H + y] = before + v + (wid ? lower : 0u);
+        before += all;
+        __syncthreads();
+    }
 }
 
-__global__ void __launch_bounds__(kIiThreads)
-k_integral_columns(int W, int H, uint32_t *dst, int dstStride, const uint32_t *totals)
+__global__ void __launch_bounds__(kIiWarps * 32)
+k_integral_tiles(int W, int H, uint32_t *dst, int dstStride, const uint8_t *src, int srcStride, IiScratch S, bool words)
 {
-    const int x = blockIdx.x * kIiThreads + threadIdx.x, seg = blockIdx.y;
-    if (x >= W) return;
-    uint32_t run = 0;
-    for (int s = 0; s < seg; s++) run += totals[(size_t)s * W + x];
-    const int y0 = seg * kIiSeg, y1 = min(y0 + kIiSeg, H);
-    for (int y = y0; y < y1; y++) {
-        uint32_t *p = (uint32_t *)((uint8_t *)dst + (size_t)y * dstStride) + x;
-        run += *p;
-        *p = run;
+    const int t = blockIdx.x * kIiWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= S.tx * S.ty) return;
+    const int tx = t % S.tx, ty = t / S.tx, x = tx * kIiCols + 4 * lane, y0 = ty * kIiRows, n = min(kIiRows, H - y0);
+    const uint8_t *p = src + (size_t)y0 * srcStride;
+    uint32_t c[4] = {0, 0, 0, 0};
+    for (int k = 0; k < 4 && x + k < W; k++) c[k] = S.cols[(size_t)ty * W + x + k];
+    const uint32_t left = lane < n ? S.left[(size_t)tx * H + y0 + lane] : 0;
+    const bool vec = (((uintptr_t)dst | (uintptr_t)dstStride) & 15) == 0 && x + 4 <= W;
+#pragma unroll 4
+    for (int r = 0; r < n; r++) {
+        const uint32_t w = ii_word(p + (size_t)r * srcStride, x, W, words);
+        c[0] += w & 0xff;
+        c[1] += (w >> 8) & 0xff;
+        c[2] += (w >> 16) & 0xff;
+        c[3] += w >> 24;
+        const uint32_t s1 = c[0] + c[1], s2 = s1 + c[2], s3 = s2 + c[3];
+        uint32_t u = s3;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, u, o);
+            if (lane >= o) u += v;
+        }
+        const uint32_t base = u - s3 + __shfl_sync(0xffffffffu, left, r);
+        uint32_t *d = (uint32_t *)((uint8_t *)dst + (size_t)(y0 + r) * dstStride) + x;
+        const uint32_t v[4] = {base + c[0], base + s1, base + s2, base + s3};
+        if (vec) *(uint4 *)d = make_uint4(v[0], v[1], v[2], v[3]);
+        else
+            for (int k = 0; k < 4 && x + k < W; k++) d[k] = v[k];
     }
 }
 
@@ -1205,7 +1270,7 @@ k_integral_columns(int W, int H, uint32_t *dst, int dstStride, const uint32_t *t
 
 extern "C" size_t agocuda_IntegralImage_scratch_size(uint32_t width, uint32_t height)
 {
-    return (size_t)div_up(height, kIiSeg) * width * sizeof(uint32_t);
+    return ((size_t)div_up(height, kIiRows) * width + (size_t)div_up(width, kIiCols) * height * 2) * sizeof(uint32_t);
 }
 
 extern "C" int agocuda_IntegralImage_U32_U8(void *stream, uint32_t dstWidth, uint32_t dstHeight, uint32_t *pDst,
@@ -1214,14 +1279,20 @@ extern "C" int agocuda_IntegralImage_U32_U8(void *stream, uint32_t dstWidth, uin
 {
     const uint32_t W = dstWidth, H = dstHeight;
     if (!W || !H || !pDst || !pSrc || ((uintptr_t)pDst & 3) || (dstStride & 3) || dstStride < 4 * W || srcStride < W ||
-        !scratch || scratchBytes < agocuda_IntegralImage_scratch_size(W, H) || H > 65535u * kIiSeg)
+        !scratch || scratchBytes < agocuda_IntegralImage_scratch_size(W, H) || H > 65535u * 32)
         return AGOCUDA_INVALID_PARAMS;
     cudaStream_t s = as_stream(stream);
-    uint32_t *tot = (uint32_t *)scratch;
-    k_integral_rows<<<H, kIiThreads, 0, s>>>((int)W, pDst, (int)dstStride, pSrc, (int)srcStride);
-    const dim3 grd(div_up(W, kIiThreads), div_up(H, kIiSeg));
-    k_integral_seg_totals<<<grd, kIiThreads, 0, s>>>((int)W, (int)H, pDst, (int)dstStride, tot);
-    k_integral_columns<<<grd, kIiThreads, 0, s>>>((int)W, (int)H, pDst, (int)dstStride, tot);
+    IiScratch S;
+    S.tx = (int)div_up(W, kIiCols);
+    S.ty = (int)div_up(H, kIiRows);
+    S.cols = (uint32_t *)scratch;
+    S.rows = S.cols + (size_t)S.ty * W;
+    S.left = S.rows + (size_t)S.tx * H;
+    const bool words = (((uintptr_t)pSrc | srcStride) & 3) == 0;
+    const unsigned tiles = div_up((unsigned)(S.tx * S.ty), kIiWarps);
+    k_integral_sums<<<tiles, kIiWarps * 32, 0, s>>>((int)W, (int)H, pSrc, (int)srcStride, S, words);
+    k_integral_scan<<<S.tx + div_up(W, 1024), 1024, 0, s>>>((int)W, (int)H, S);
+    k_integral_tiles<<<tiles, kIiWarps * 32, 0, s>>>((int)W, (int)H, pDst, (int)dstStride, pSrc, (int)srcStride, S, words);
     agocuda_count_launch(3);
     return agocuda_launch_status();
 }

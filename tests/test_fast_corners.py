@@ -155,3 +155,18 @@ def test_fast_kernel_rejects_bad_arguments(cuda, agocuda):
 @pytest.mark.parametrize("kind,thr", [("scene", 20.0), ("noise", 40.5)])
 def test_engine_fast_graph(cuda, kind, thr, suppress, W, H):
     _check(V.OpenVX(), kind, W, H, thr, suppress, capacity=1 << 18)
+
+
+# the byte-lane circle test at the ends of its saturated bounds, on full-contrast pixels, at sizes
+# around the 128x8 tiles and the 1024-pixel steps of a row
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(128, 8), (129, 17), (1040, 23)])
+@pytest.mark.parametrize("suppress", [False, True])
+@pytest.mark.parametrize("thr", [0.0, 1.0, 127.0, 254.0, 255.0, 300.0])
+def test_fast_threshold_ends(cuda, agocuda, thr, suppress, W, H):
+    img = np.random.default_rng(W + H).choice(np.array([0, 1, 127, 128, 254, 255], np.uint8), (H, W), p=[.35, .05, .1, .1, .05, .35])
+    img[2:H - 2, 4:W - 4:9] = 255
+    want, want_n = oracle_fast(img, thr, suppress, 1 << 16)
+    got, _, n = _kernel(agocuda, img, thr, suppress, 1 << 16)
+    assert n == want_n
+    np.testing.assert_array_equal(got, want)

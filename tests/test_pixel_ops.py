@@ -245,3 +245,26 @@ def test_engine_chain_with_virtual_images(cuda):
         np.testing.assert_array_equal(got[1:-1, 1:-1], want[1:-1, 1:-1])
     finally:
         api.vxReleaseContext(C.byref(C.c_void_p(ctx)))
+
+
+# integral images at the edges of the 128x32 tiles, over 1024 rows, and on planes that allow no
+# vector access
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H,align", [(1, 1, 0), (127, 31, 0), (128, 32, 0), (129, 33, 0), (131, 1030, 0), (260, 65, 4)])
+def test_integral_tiles(cuda, W, H, align):
+    import ctypes as CT
+    import torch
+    from devbuf import DevImg, stream_ptr
+    from mivisionx_b200 import native
+    L = native.agocuda()
+    L.agocuda_IntegralImage_scratch_size.argtypes, L.agocuda_IntegralImage_scratch_size.restype = [CT.c_uint32] * 2, CT.c_size_t
+    L.agocuda_IntegralImage_U32_U8.argtypes = [CT.c_void_p, CT.c_uint32, CT.c_uint32, CT.c_void_p, CT.c_uint32, CT.c_void_p,
+                                               CT.c_uint32, CT.c_void_p, CT.c_size_t]
+    img = np.random.default_rng(W + H).integers(0, 256, (H, W), dtype=np.int32).astype(np.uint8)
+    img[0] = 255
+    src = DevImg(H, W, stride=W + 3 if align else None, align_off=align // 4).upload(img)
+    dst = DevImg(H, W, np.uint32, stride=4 * W + 4 if align else None, align_off=align)
+    nb = L.agocuda_IntegralImage_scratch_size(W, H)
+    scratch = torch.full((nb + 256,), 0xA5, dtype=torch.uint8, device="cuda")
+    assert L.agocuda_IntegralImage_U32_U8(stream_ptr(), W, H, dst.ptr, dst.stride, src.ptr, src.stride, scratch.data_ptr(), nb) == 0
+    np.testing.assert_array_equal(dst.download(), P.integral_image(img))
