@@ -10,6 +10,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <set>
 
 #include "vx_internal.h"
@@ -23,6 +24,7 @@ static void plan_state_free(PlanState &ps)
     if (ps.cexec) cudaGraphExecDestroy(ps.cexec);
     if (ps.cgraph) cudaGraphDestroy(ps.cgraph);
     for (void *p : ps.dev_scratch) cudaFree(p);
+    if (ps.dist_host) cudaFreeHost(ps.dist_host);
     ps = PlanState{};
 }
 
@@ -39,6 +41,10 @@ static void plan_state_swap(Graph *g, PlanState &ps)
     std::swap(g->streamed_out, ps.streamed_out);
     std::swap(g->staged_in, ps.staged_in);
     std::swap(g->staged_out, ps.staged_out);
+    std::swap(g->staged_dist, ps.staged_dist);
+    std::swap(g->dist_host, ps.dist_host);
+    std::swap(g->in_route, ps.in_route);
+    std::swap(g->out_streamed, ps.out_streamed);
     std::swap(g->plan_text, ps.plan_text);
 }
 
@@ -60,10 +66,20 @@ void graph_invalidate(Graph *g)
     g->steps.clear();
 }
 
-static uint64_t fnv(uint64_t h, const void *p, size_t n)
+// Hashes 8 bytes per step (the signature is taken on every execution).  Each step is a bijection of
+// the word for a given h and of h for a given word, so changing one parameter always changes the hash.
+static uint64_t mix(uint64_t h, const void *p, size_t n)
 {
     const uint8_t *b = (const uint8_t *)p;
-    for (size_t i = 0; i < n; i++) { h ^= b[i]; h *= 1099511628211ull; }
+    for (; n; ) {
+        uint64_t w = 0;
+        const size_t k = std::min(n, sizeof w);
+        memcpy(&w, b, k);
+        h = (h ^ w) * 0x9E3779B97F4A7C15ull;
+        h ^= h >> 29;
+        b += k;
+        n -= k;
+    }
     return h;
 }
 
@@ -72,29 +88,26 @@ static uint64_t fnv(uint64_t h, const void *p, size_t n)
 static uint64_t param_signature(Graph *g)
 {
     uint64_t h = 1469598103934665603ull;
-    for (LNode &ln : g->lnodes) {
-        for (Ref *r : ln.p) {
-            if (!r) continue;
-            switch (r->type) {
-            case VX_TYPE_SCALAR: h = fnv(h, &static_cast<Scalar *>(r)->version, 8); h = fnv(h, static_cast<Scalar *>(r)->v.raw, 8); break;
-            case VX_TYPE_THRESHOLD: h = fnv(h, &static_cast<Threshold *>(r)->version, 8); break;
-            case VX_TYPE_MATRIX: h = fnv(h, &static_cast<Matrix *>(r)->version, 8); break;
-            case VX_TYPE_LUT: h = fnv(h, &static_cast<Lut *>(r)->version, 8); break;
-            case VX_TYPE_CONVOLUTION: h = fnv(h, &static_cast<Convolution *>(r)->version, 8); break;
-            case VX_TYPE_REMAP: h = fnv(h, &static_cast<Remap *>(r)->version, 8); break;
-            case VX_TYPE_IMAGE: {
-                Image *img = IMG(r);
-                h = fnv(h, &img->valid, sizeof(img->valid));
-                for (int i = 0; i < img->num_planes; i++) h = fnv(h, &img->planes[i].dev, sizeof(void *));
-                break;
-            }
-            // storage that ageing a delay moves between objects
-            case VX_TYPE_ARRAY: h = fnv(h, &static_cast<Array *>(r)->dev, sizeof(void *)); break;
-            case VX_TYPE_PYRAMID:
-                for (Image *lv : static_cast<Pyramid *>(r)->level) h = fnv(h, &lv->planes[0].dev, sizeof(void *));
-                break;
-            default: break;
-            }
+    for (Ref *r : g->signature_refs) {
+        switch (r->type) {
+        case VX_TYPE_SCALAR: h = mix(h, &static_cast<Scalar *>(r)->version, 8); h = mix(h, static_cast<Scalar *>(r)->v.raw, 8); break;
+        case VX_TYPE_THRESHOLD: h = mix(h, &static_cast<Threshold *>(r)->version, 8); break;
+        case VX_TYPE_MATRIX: h = mix(h, &static_cast<Matrix *>(r)->version, 8); break;
+        case VX_TYPE_LUT: h = mix(h, &static_cast<Lut *>(r)->version, 8); break;
+        case VX_TYPE_CONVOLUTION: h = mix(h, &static_cast<Convolution *>(r)->version, 8); break;
+        case VX_TYPE_REMAP: h = mix(h, &static_cast<Remap *>(r)->version, 8); break;
+        case VX_TYPE_IMAGE: {
+            Image *img = IMG(r);
+            h = mix(h, &img->valid, sizeof(img->valid));
+            for (int i = 0; i < img->num_planes; i++) h = mix(h, &img->planes[i].dev, sizeof(void *));
+            break;
+        }
+        // storage that ageing a delay moves between objects
+        case VX_TYPE_ARRAY: h = mix(h, &static_cast<Array *>(r)->dev, sizeof(void *)); break;
+        case VX_TYPE_PYRAMID:
+            for (Image *lv : static_cast<Pyramid *>(r)->level) h = mix(h, &lv->planes[0].dev, sizeof(void *));
+            break;
+        default: break;
         }
     }
     return h;
@@ -206,8 +219,14 @@ static cudaError_t plane_copy(const Plane &p, cudaMemcpyKind kind, cudaStream_t 
 
 constexpr size_t kIoSlots = 1024;   // count slots per graph (arrays staged beyond this use blocking copies)
 
+constexpr int kInSync = -2, kInStreamed = -1;   // Graph::in_route
+
 static void release_capture(Graph *g)
 {
+    if (g->dist_host) { cudaFreeHost(g->dist_host); g->dist_host = nullptr; }
+    g->staged_dist.clear();
+    g->in_route.clear();
+    g->out_streamed.clear();
     if (g->cexec) { cudaGraphExecDestroy(g->cexec); g->cexec = nullptr; }
     if (g->cgraph) { cudaGraphDestroy(g->cgraph); g->cgraph = nullptr; }
     for (cudaEvent_t e : g->cap_events) cudaEventDestroy(e);
@@ -319,22 +338,47 @@ static vx_status capture(Graph *g)
     // output arrays: one launch for all that the same part writes (a batch of frames)
     size_t downloads = 0;
     if (!serial) {
-        std::map<int, std::vector<Array *>> by_part;
+        struct Download { Ref *r; agocuda_array_xfer x; };
+        std::map<int, std::vector<Download>> by_part;
+        std::map<Ref *, int> writer;
+        for (int j = 0; j < (int)parts.size(); j++)
+            for (Ref *r : parts[j].wr) writer[r] = j;
+        auto part_of = [&](Ref *r) { auto it = writer.find(r); return it == writer.end() ? -1 : it->second; };
         for (Ref *r : g->outputs)
             if (r->type == VX_TYPE_ARRAY && slot_free() && stageable(static_cast<Array *>(r))) {
-                int last = -1;
-                for (int j = 0; j < (int)parts.size(); j++)
-                    if (std::find(parts[j].wr.begin(), parts[j].wr.end(), r) != parts[j].wr.end()) last = j;
-                by_part[last].push_back(static_cast<Array *>(r));
-                g->staged_out.push_back(static_cast<Array *>(r));
+                Array *a = static_cast<Array *>(r);
+                uint32_t *slot = g->io_slots_dev + g->staged_in.size() + g->staged_out.size();
+                by_part[part_of(r)].push_back({r, {a->dev, a->dev_count, a->host_mapped, slot, (uint32_t)a->item_size, (uint32_t)a->capacity}});
+                g->staged_out.push_back(a);
             }
+        // distributions: all their bins, through one page-locked block (one word for the counts that
+        // the transfers write back)
+        size_t bins = 0;
+        for (Ref *r : g->outputs)
+            if (r->type == VX_TYPE_DISTRIBUTION && static_cast<Distribution *>(r)->dev) {
+                g->staged_dist.push_back(static_cast<Distribution *>(r));
+                bins += static_cast<Distribution *>(r)->bins;
+            }
+        if (!g->staged_dist.empty()) {
+            uint32_t *mapped = nullptr, *counts = nullptr;
+            std::vector<uint32_t> n;
+            for (Distribution *d : g->staged_dist) n.push_back((uint32_t)d->bins);
+            if (cudaHostAlloc((void **)&g->dist_host, (bins + 1) * 4, cudaHostAllocMapped) != cudaSuccess ||
+                cudaHostGetDevicePointer((void **)&mapped, g->dist_host, 0) != cudaSuccess ||
+                cudaMalloc((void **)&counts, n.size() * 4) != cudaSuccess)
+                return VX_ERROR_NO_MEMORY;
+            g->dev_scratch.push_back(counts);
+            if (cudaMemcpy(counts, n.data(), n.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) return VX_FAILURE;
+            size_t at = 0;
+            for (size_t i = 0; i < n.size(); i++) {
+                Distribution *d = g->staged_dist[i];
+                by_part[part_of(d)].push_back({d, {d->dev, counts + i, mapped + at, mapped + bins, 4, n[i]}});
+                at += n[i];
+            }
+        }
         std::vector<agocuda_array_xfer> xf;
         for (auto &kv : by_part)
-            for (Array *a : kv.second) {
-                const size_t i = std::find(g->staged_out.begin(), g->staged_out.end(), a) - g->staged_out.begin();
-                xf.push_back(agocuda_array_xfer{a->dev, a->dev_count, a->host_mapped, g->io_slots_dev + g->staged_in.size() + i,
-                                                (uint32_t)a->item_size, (uint32_t)a->capacity});
-            }
+            for (Download &d : kv.second) xf.push_back(d.x);
         agocuda_array_xfer *table = nullptr;
         if (!xf.empty()) {
             if (cudaMalloc((void **)&table, xf.size() * sizeof(agocuda_array_xfer)) != cudaSuccess) return VX_ERROR_NO_MEMORY;
@@ -345,7 +389,7 @@ static vx_status capture(Graph *g)
         for (auto &kv : by_part) {
             const uint32_t n = (uint32_t)kv.second.size();
             CapPart cp;
-            for (Array *a : kv.second) cp.rd.push_back(a);
+            for (Download &d : kv.second) cp.rd.push_back(d.r);
             cp.lane = kArrayLane;
             cp.launch = [table, n](cudaStream_t q) { return agocuda_array_download_batch(q, table, n); };
             parts.push_back(std::move(cp));
@@ -356,8 +400,8 @@ static vx_status capture(Graph *g)
 
     // the array transfers are kernels of the CUDA graph too: list them with the plan
     if (!g->staged_in.empty()) g->plan_text += "array_upload_batch\t1\n";
-    if (!g->staged_out.empty())
-        g->plan_text += "array_download x" + std::to_string(g->staged_out.size()) + "\t" + std::to_string(downloads) + "\n";
+    if (!g->staged_out.empty() || !g->staged_dist.empty())
+        g->plan_text += "array_download x" + std::to_string(g->staged_out.size() + g->staged_dist.size()) + "\t" + std::to_string(downloads) + "\n";
 
     // ---- dependencies: read-after-write, write-after-write, write-after-read
     std::map<Ref *, int> last_writer;
@@ -453,11 +497,21 @@ static vx_status capture(Graph *g)
         g->streamed_out.clear();
         g->staged_in.clear();
         g->staged_out.clear();
+        g->staged_dist.clear();
         log_error(g, VX_FAILURE, "ERROR: CUDA graph capture failed (step rc=%d, %s)\n", rc, cudaGetErrorString(e));
         return VX_FAILURE;
     }
     if (cudaGraphInstantiate(&g->cexec, cg, 0) != cudaSuccess) { cudaGraphDestroy(cg); return VX_FAILURE; }
     g->cgraph = cg;
+    for (Ref *r : g->inputs) {
+        auto im = std::find(g->streamed_in.begin(), g->streamed_in.end(), r);
+        auto ar = std::find(g->staged_in.begin(), g->staged_in.end(), r);
+        g->in_route.push_back(im != g->streamed_in.end() ? kInStreamed : ar != g->staged_in.end() ? (int)(ar - g->staged_in.begin()) : kInSync);
+    }
+    for (Ref *r : g->outputs) {
+        Ref *root = r->type == VX_TYPE_IMAGE && IMG(r)->parent ? IMG(r)->parent : r;
+        g->out_streamed.push_back(std::find(g->streamed_out.begin(), g->streamed_out.end(), root) != g->streamed_out.end());
+    }
     return VX_SUCCESS;
 }
 
@@ -577,6 +631,11 @@ vx_status graph_verify(Graph *g)
     if (s) return s;
     s = plan_graph(g);
     if (s) return s;
+    std::set<Ref *> named;
+    g->signature_refs.clear();
+    for (LNode &ln : g->lnodes)
+        for (Ref *r : ln.p)
+            if (r && named.insert(r).second) g->signature_refs.push_back(r);
     g->param_signature = param_signature(g);
     s = capture(g);
     if (s) return s;
@@ -630,10 +689,11 @@ vx_status graph_process(Graph *g, bool wait)
         }
     }
     cudaSetDevice(g->ctx->device);
-    for (Ref *r : g->inputs) {
+    for (size_t i = 0; i < g->inputs.size(); i++) {
+        Ref *r = g->inputs[i];
         vx_status s = VX_SUCCESS;
-        const bool streamed = std::find(g->streamed_in.begin(), g->streamed_in.end(), r) != g->streamed_in.end();
-        if (streamed) {
+        const int route = i < g->in_route.size() ? g->in_route[i] : kInSync;
+        if (route == kInStreamed) {
             // the CUDA graph uploads the application's buffer: make sure that buffer is current
             Image *img = IMG(r);
             if (!img->host_valid && img->dev_valid) s = image_sync_to_host(img);
@@ -643,10 +703,9 @@ vx_status graph_process(Graph *g, bool wait)
         if (r->type == VX_TYPE_IMAGE) s = image_sync_to_device(IMG(r), g->stream);
         else if (r->type == VX_TYPE_ARRAY) {
             Array *a = static_cast<Array *>(r);
-            auto it = std::find(g->staged_in.begin(), g->staged_in.end(), a);
-            if (it != g->staged_in.end()) {
+            if (route >= 0) {
                 // the CUDA graph uploads the host items unless the device copy is current
-                g->io_slots_host[it - g->staged_in.begin()] =
+                g->io_slots_host[route] =
                     a->dev_valid ? AGOCUDA_ARRAY_SKIP : (uint32_t)std::min(a->num_items, a->capacity);
                 continue;
             }
@@ -669,11 +728,12 @@ vx_status graph_process(Graph *g, bool wait)
     for (Array *a : g->staged_in) a->dev_valid = true;
     // outputs are now current on the device only (and in the application's buffer when
     // the CUDA graph downloads them)
-    for (Ref *r : g->outputs) {
+    for (size_t i = 0; i < g->outputs.size(); i++) {
+        Ref *r = g->outputs[i];
         if (r->type == VX_TYPE_IMAGE) {
             Image *root = IMG(r)->parent ? IMG(r)->parent : IMG(r);
             root->dev_valid = true;
-            root->host_valid = std::find(g->streamed_out.begin(), g->streamed_out.end(), root) != g->streamed_out.end();
+            root->host_valid = i < g->out_streamed.size() && g->out_streamed[i];
         } else if (r->type == VX_TYPE_ARRAY) {
             static_cast<Array *>(r)->dev_valid = true; static_cast<Array *>(r)->host_valid = false;
         } else if (r->type == VX_TYPE_SCALAR) {
@@ -730,6 +790,12 @@ vx_status graph_wait(Graph *g)
         Array *a = g->staged_out[i];
         a->num_items = std::min((vx_size)g->io_slots_host[g->staged_in.size() + i], a->capacity);
         a->host_valid = true;
+    }
+    size_t bin = 0;
+    for (Distribution *d : g->staged_dist) {
+        memcpy(d->host.data(), g->dist_host + bin, d->bins * 4);
+        bin += d->bins;
+        d->dev_newer = false;
     }
     // kernels that detect a failure (bounded walks, candidate overflow) set status bits
     if (g->status_host && *(volatile uint32_t *)g->status_host) {

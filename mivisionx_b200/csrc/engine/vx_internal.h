@@ -323,6 +323,10 @@ struct PlanState {
     std::vector<Ref *> inputs, outputs;
     std::vector<Image *> streamed_in, streamed_out;
     std::vector<Array *> staged_in, staged_out;
+    std::vector<Distribution *> staged_dist;
+    uint32_t *dist_host = nullptr;
+    std::vector<int> in_route;
+    std::vector<bool> out_streamed;
     std::string plan_text;
     uint64_t use = 0;                            // last use, for eviction
 };
@@ -351,6 +355,15 @@ struct Graph : Ref {
     // mapped count slot each (io_slots_host[i] <-> staged_in / staged_out in that order)
     std::vector<Array *> staged_in, staged_out;
     uint32_t *io_slots_host = nullptr, *io_slots_dev = nullptr;
+    // distributions copied to page-locked memory inside the CUDA graph (their bins one after another)
+    std::vector<Distribution *> staged_dist;
+    uint32_t *dist_host = nullptr;
+    // how each of `inputs` reaches the device: kInSync, kInStreamed, or its index in staged_in;
+    // which of `outputs` the CUDA graph downloads itself (both empty: no capture)
+    std::vector<int> in_route;
+    std::vector<bool> out_streamed;
+    // the distinct data the lowered nodes name, for param_signature
+    std::vector<Ref *> signature_refs;
     bool scheduled = false;
     vx_status last_status = VX_SUCCESS;
     vx_perf_t perf{};

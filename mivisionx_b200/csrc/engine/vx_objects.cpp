@@ -319,8 +319,10 @@ static vx_status ensure_host(Image *img)
 
 vx_status image_sync_to_device(Image *img, cudaStream_t s)
 {
-    use_device(img);
     Image *root = img->parent ? img->parent : img;
+    // current already, as between executions: nothing to allocate, refresh or copy
+    if (root->dev_valid && root->import_type != VX_MEMORY_TYPE_HOST && !root->uniform && root->allocated()) return VX_SUCCESS;
+    use_device(img);
     vx_status st = image_alloc_device(root);
     if (st) return st;
     if (root->dev_valid && root->import_type != VX_MEMORY_TYPE_HOST) return VX_SUCCESS;
@@ -486,6 +488,7 @@ Graph::~Graph()
     for (cudaStream_t s : lanes) cudaStreamDestroy(s);
     if (stream) cudaStreamDestroy(stream);
     for (void *p : dev_scratch) cudaFree(p);
+    if (dist_host) cudaFreeHost(dist_host);
     if (status_host) cudaFreeHost(status_host);
     if (io_slots_host) cudaFreeHost(io_slots_host);
 }
@@ -1421,7 +1424,11 @@ vx_status vxCopyArrayRange(vx_array array, vx_size range_start, vx_size range_en
     if (!user_ptr || user_mem_type != VX_MEMORY_TYPE_HOST || user_stride < a->item_size) return VX_ERROR_INVALID_PARAMETERS;
     if (array_sync_to_host(a)) return VX_FAILURE;
     if (range_start >= range_end || range_end > a->num_items) return VX_ERROR_INVALID_PARAMETERS;
-    for (vx_size i = range_start; i < range_end; i++) {
+    if (user_stride == a->item_size) {
+        uint8_t *items = &a->host[range_start * a->item_size];
+        const vx_size bytes = (range_end - range_start) * a->item_size;
+        memcpy(usage == VX_READ_ONLY ? user_ptr : items, usage == VX_READ_ONLY ? items : user_ptr, bytes);
+    } else for (vx_size i = range_start; i < range_end; i++) {
         uint8_t *u = (uint8_t *)user_ptr + (i - range_start) * user_stride;
         if (usage == VX_READ_ONLY) memcpy(u, &a->host[i * a->item_size], a->item_size);
         else memcpy(&a->host[i * a->item_size], u, a->item_size);

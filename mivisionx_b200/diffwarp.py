@@ -58,15 +58,26 @@ def _images(t: torch.Tensor, name: str) -> torch.Tensor:
     return t.contiguous()
 
 
+def _like(t: torch.Tensor, src: torch.Tensor) -> torch.Tensor:
+    """t as contiguous float32 on src's device (t itself where it is that already)."""
+    if t.dtype != torch.float32 or t.device != src.device:
+        t = t.to(device=src.device, dtype=torch.float32)
+    return t.contiguous()
+
+
+# the raw handle of the current stream, without a Stream object per call
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _raw_stream(t.get_device()) if _raw_stream else torch.cuda.current_stream(t.device).cuda_stream
 
 
 class WarpAffineF32(torch.autograd.Function):
     @staticmethod
     def forward(ctx, src, theta, border=0.0):
         src = _images(src, "src")
-        theta = theta.to(device=src.device, dtype=torch.float32).contiguous()
+        theta = _like(theta, src)
         N, H, W = src.shape
         if theta.shape != (N, 6):
             raise ValueError("theta must have shape (N, 6)")
@@ -82,7 +93,7 @@ class WarpAffineF32(torch.autograd.Function):
     def backward(ctx, gout):
         src, theta = ctx.saved_tensors
         N, H, W = src.shape
-        gout = gout.to(torch.float32).contiguous()
+        gout = _like(gout, src)
         gsrc = torch.zeros_like(src)
         gth = torch.zeros((N, 6), dtype=torch.float64, device=src.device)
         _check(_L().agocuda_WarpAffine_F32_Bilinear_Constant_adjoint_batch(
@@ -95,7 +106,7 @@ class WarpPerspectiveF32(torch.autograd.Function):
     @staticmethod
     def forward(ctx, src, theta, border=0.0):
         src = _images(src, "src")
-        theta = theta.to(device=src.device, dtype=torch.float32).contiguous()
+        theta = _like(theta, src)
         N, H, W = src.shape
         if theta.shape != (N, 9):
             raise ValueError("theta must have shape (N, 9)")
@@ -111,7 +122,7 @@ class WarpPerspectiveF32(torch.autograd.Function):
     def backward(ctx, gout):
         src, theta = ctx.saved_tensors
         N, H, W = src.shape
-        gout = gout.to(torch.float32).contiguous()
+        gout = _like(gout, src)
         gsrc = torch.zeros_like(src)
         gth = torch.zeros((N, 9), dtype=torch.float64, device=src.device)
         _check(_L().agocuda_WarpPerspective_F32_Bilinear_Constant_adjoint_batch(
@@ -125,7 +136,7 @@ class RemapF32(torch.autograd.Function):
     def forward(ctx, src, field, border=0.0):
         src = _images(src, "src")
         N, H, W = src.shape
-        field = field.to(device=src.device, dtype=torch.float32).contiguous()
+        field = _like(field, src)
         if field.shape != (N, H, W, 2):
             raise ValueError("field must have shape (N, H, W, 2)")
         out = torch.empty_like(src)
@@ -140,7 +151,7 @@ class RemapF32(torch.autograd.Function):
     def backward(ctx, gout):
         src, field = ctx.saved_tensors
         N, H, W = src.shape
-        gout = gout.to(torch.float32).contiguous()
+        gout = _like(gout, src)
         gsrc = torch.zeros_like(src)
         gfield = torch.empty_like(field)
         _check(_L().agocuda_Remap_F32_Bilinear_Constant_adjoint_batch(
@@ -169,7 +180,7 @@ def warp_affine_l2_step(src: torch.Tensor, theta: torch.Tensor, target: torch.Te
     zeroed here)."""
     src, target = _images(src, "src"), _images(target, "target")
     N, H, W = src.shape
-    theta = theta.to(device=src.device, dtype=torch.float32).contiguous()
+    theta = _like(theta, src)
     if gsrc is None:
         gsrc = torch.zeros_like(src)
     else:
@@ -190,7 +201,7 @@ def warp_perspective_l2_step(src: torch.Tensor, theta: torch.Tensor, target: tor
     (N, H, W) float32, gtheta (N, 9) float64)."""
     src, target = _images(src, "src"), _images(target, "target")
     N, H, W = src.shape
-    theta = theta.to(device=src.device, dtype=torch.float32).contiguous()
+    theta = _like(theta, src)
     if theta.shape != (N, 9):
         raise ValueError("theta must have shape (N, 9)")
     if gsrc is None:
