@@ -652,6 +652,10 @@ int agocuda_OpticalFlowPyrLK_XY_XY(void *stream, void *newKeyPoint, uint32_t new
 /* ------------------------------------------------------------------------------------ */
 #define AGOCUDA_ARRAY_SKIP 0xFFFFFFFFu   /* upload count slot: leave the device array as it is */
 
+/* The device's nanosecond clock (%globaltimer) when the stream gets here, into a mapped host word: the
+ * first and last node of a captured graph, whose difference is the execution's device time. */
+int agocuda_time_stamp(void *stream, uint64_t *pMapped);
+
 /* devItems[0 .. n) = hostItems[0 .. n), *devCount = n, n = min(*countSlot, capacity);
  * nothing when *countSlot == AGOCUDA_ARRAY_SKIP. */
 int agocuda_array_upload(void *stream, void *devItems, uint32_t *devCount, const void *hostItemsMapped,

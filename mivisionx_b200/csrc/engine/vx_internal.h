@@ -347,7 +347,8 @@ struct Graph : Ref {
     cudaStream_t stream = nullptr;
     cudaGraph_t cgraph = nullptr;
     cudaGraphExec_t cexec = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;    // device time of executions without a captured graph
+    bool stamped = false;                        // the last execution took its device time inside the graph
     std::vector<cudaStream_t> lanes;             // streams forked from `stream` during capture
     std::vector<cudaEvent_t> cap_events;         // fork/join/dependency events of the capture
     std::vector<Image *> streamed_in, streamed_out;  // host images copied inside the CUDA graph

@@ -82,7 +82,23 @@ k_array_download(uint8_t *host, volatile uint32_t *slot, const uint8_t *dev, con
     if (blockIdx.x == 0 && threadIdx.x == 0) *slot = m;
 }
 
+// the device's nanosecond clock, into a mapped host word
+__global__ void k_time_stamp(unsigned long long *out)
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    *out = t;
+}
+
 }  // namespace
+
+extern "C" int agocuda_time_stamp(void *stream, uint64_t *pMapped)
+{
+    if (!pMapped) return AGOCUDA_INVALID_PARAMS;
+    k_time_stamp<<<1, 1, 0, as_stream(stream)>>>((unsigned long long *)pMapped);
+    agocuda_count_launch(1);
+    return agocuda_launch_status();
+}
 
 extern "C" int agocuda_array_upload(void *stream, void *devItems, uint32_t *devCount, const void *hostItemsMapped,
                                     const uint32_t *countSlotMapped, uint32_t itemSize, uint32_t capacity)
