@@ -649,6 +649,8 @@ vx_status graph_verify(Graph *g)
     g->param_signature = param_signature(g);
     s = capture(g);
     if (s) return s;
+    // tables and fills of the plan went through the legacy stream, which g->stream does not wait for
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) return VX_FAILURE;
     s = user_nodes_init(g);
     if (s) return s;
     g->verified = true;
@@ -686,6 +688,7 @@ vx_status graph_process(Graph *g, bool wait)
             } else {
                 s = plan_graph(g);
                 if (!s) s = capture(g);
+                if (!s && cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) s = VX_FAILURE;   // as in graph_verify
             }
             g->param_signature = sig;
             while (g->plan_cache.size() > kCachedPlans) {

@@ -261,6 +261,7 @@ vx_status image_alloc_device(Image *img)
     use_device(img);
     if (img->parent) return image_alloc_device(img->parent);
     if (!img->num_planes) return VX_ERROR_INVALID_FORMAT;
+    bool fresh = false;
     for (int i = 0; i < img->num_planes; i++) {
         Plane &p = img->planes[i];
         if (p.dev) continue;
@@ -274,6 +275,7 @@ vx_status image_alloc_device(Image *img)
         p.dev = (uint8_t *)d;
         p.dev_owned = true;
         if (!p.host_stride) p.host_stride = p.dev_stride;
+        fresh = true;
     }
     image_refresh_views(img);
     if (img->uniform || (!img->dev_valid && !img->host_valid)) {
@@ -296,7 +298,10 @@ vx_status image_alloc_device(Image *img)
             }
         }
         img->dev_valid = true;
+        fresh = fresh || img->uniform;
     }
+    // the fills above ran on the legacy stream, which graph streams do not wait for
+    if (fresh && cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) return VX_FAILURE;
     return VX_SUCCESS;
 }
 
@@ -406,6 +411,7 @@ vx_status array_alloc_device(Array *a)
     cudaMemset(a->dev, 0, a->item_size * a->capacity + 64);
     if (cudaMalloc((void **)&a->dev_count, 16) != cudaSuccess) return VX_ERROR_NO_MEMORY;
     cudaMemset(a->dev_count, 0, 16);
+    cudaStreamSynchronize(cudaStreamLegacy);       // graph streams do not wait for the fills
     return VX_SUCCESS;
 }
 
@@ -853,6 +859,9 @@ vx_status vxCopyImagePatch(vx_image image, const vx_rectangle_t *image_rect, vx_
         if (cudaMemcpy2D(p.dev + (size_t)y0 * p.dev_stride + (size_t)x0 * p.bpp, p.dev_stride, user_ptr,
                          (size_t)user_addr->stride_y, row_bytes, y1 - y0, kind_in) != cudaSuccess)
             return VX_FAILURE;
+        // a copy from pageable memory may return with its last transfer in flight, one between
+        // device buffers before it starts; graphs run on streams that do not wait for this one
+        if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) return VX_FAILURE;
         if (root->import_type == VX_MEMORY_TYPE_HOST) {
             // keep the application's own buffer authoritative
             for (uint32_t y = y0; y < y1; y++)
