@@ -459,14 +459,17 @@ static vx_status capture(Graph *g)
 
     // ---- record
     cudaSetDevice(g->ctx->device);
-    while ((int)g->lanes.size() < kNumLanes - 1) {
-        cudaStream_t s = nullptr;
-        if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return VX_ERROR_NO_RESOURCES;
-        g->lanes.push_back(s);
+    int top = 0;
+    for (CapPart &cp : parts) top = std::max(top, cp.lane);
+    while ((int)g->lanes.size() < top) g->lanes.push_back(nullptr);
+    std::vector<cudaStream_t> lane(kNumLanes, nullptr);
+    lane[0] = g->stream;   // lane 0 is the graph's own stream; the others exist where a part uses them
+    for (CapPart &cp : parts) {
+        if (!cp.lane) continue;
+        cudaStream_t &s = g->lanes[cp.lane - 1];
+        if (!s && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return VX_ERROR_NO_RESOURCES;
+        lane[cp.lane] = s;
     }
-    std::vector<cudaStream_t> lane(kNumLanes);
-    lane[0] = g->stream;   // lane 0 is the graph's own stream
-    for (int i = 1; i < kNumLanes; i++) lane[i] = g->lanes[i - 1];
     std::vector<bool> used(kNumLanes, false);
     for (CapPart &cp : parts)
         for (int i : cp.deps)

@@ -491,7 +491,7 @@ Graph::~Graph()
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     for (cudaEvent_t e : cap_events) cudaEventDestroy(e);
-    for (cudaStream_t s : lanes) cudaStreamDestroy(s);
+    for (cudaStream_t s : lanes) if (s) cudaStreamDestroy(s);
     if (stream) cudaStreamDestroy(stream);
     for (void *p : dev_scratch) cudaFree(p);
     if (dist_host) cudaFreeHost(dist_host);
