@@ -733,7 +733,7 @@ __device__ __forceinline__ uint32_t lk9_pairs(const uint8_t *row, int off)
 
 // one Scharr derivative the reference's way (lk_track_point's rules) at column gc, row gr from
 // the 8-byte rows r0, r1, r2 whose byte j is column gc - 1 + (j - at); packed gx | gy << 16
-__device__ __noinline__ uint32_t lk9_special(const agocuda_lk_frame &F, int level, int W8, int gc, int gr, uint2 r0, uint2 r1,
+__device__ __forceinline__ uint32_t lk9_special(const agocuda_lk_frame &F, int level, int W8, int gc, int gr, uint2 r0, uint2 r1,
                                             uint2 r2, int at)
 {
     if (gr <= 0) return 0;
@@ -754,6 +754,22 @@ __device__ __noinline__ uint32_t lk9_special(const agocuda_lk_frame &F, int leve
     return (uint32_t)(uint16_t)(v0r - v0l) | ((uint32_t)(uint16_t)(3 * (v1l + v1r) + 10 * v1c) << 16);
 }
 
+// the four of a lane (columns gc, gc + 1, gc + 4, gc + 5) as the biased pairs gx, gx, gy, gy; out of
+// line and rolled: it is rare, and the tracking kernel is bound by its instruction fetches
+__device__ __noinline__ uint4 lk9_special4(const agocuda_lk_frame &F, int level, int W8, int gc, int gr, uint2 r0, uint2 r1, uint2 r2)
+{
+    uint32_t g[4] = {0, 0, 0, 0};
+#pragma unroll 1
+    for (int j = 0; j < 4; j++) {
+        const int off = (j & 1) + 4 * (j >> 1), sh = 16 * (j & 1);
+        const uint32_t v = lk9_special(F, level, W8, gc + off, gr, r0, r1, r2, off);
+        const uint32_t x = (uint32_t)((int)(int16_t)(v & 0xffff) + 8192) << sh, y = (uint32_t)((int)(int16_t)(v >> 16) + 8192) << sh;
+        if (j < 2) { g[0] |= x; g[2] |= y; }
+        else { g[1] |= x; g[3] |= y; }
+    }
+    return make_uint4(g[0], g[1], g[2], g[3]);
+}
+
 // dp2a: c + lo16(a) * byte(b, 0 / 2) + hi16(a) * byte(b, 1 / 3)
 __device__ __forceinline__ int dp2a_lo(int a, uint32_t b, int c) { int d; asm("dp2a.lo.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
 __device__ __forceinline__ int dp2a_hi(int a, uint32_t b, int c) { int d; asm("dp2a.hi.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
@@ -762,6 +778,9 @@ __global__ void __launch_bounds__(kL9Warps * 32, 4) k_lk_track9(agocuda_lk_frame
 {
     constexpr int win = 9;
     constexpr unsigned kAll = 0xffffffffu;
+    // integer gradients (gx | gy << 16) of the lanes' columns, for points at whole positions
+    __shared__ uint32_t sGrad[kL9Warps][2 * win][32];
+    uint32_t (*const grad)[32] = sGrad[threadIdx.x >> 5];
     const agocuda_lk_frame &F = frames[blockIdx.y];
     const int lane = threadIdx.x & 31, grp = min(lane / kL9, kL9Points - 1), k = lane - grp * kL9, base = grp * kL9;
     const uint32_t first = (blockIdx.x * kL9Warps + (threadIdx.x >> 5)) * kL9Points, pt = first + grp;
@@ -857,17 +876,8 @@ __global__ void __launch_bounds__(kL9Warps * 32, 4) k_lk_track9(agocuda_lk_frame
                 const uint32_t gyb = 3u * (t1[2] + t1[3]) + 10u * __funnelshift_r(t1[2], t1[3], 16) + 0x10001000u;
                 uint32_t xa = gxa, xb = gxb, ya = gya, yb = gyb;
                 if (special) {
-                    uint32_t v[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int off = (j & 1) + 4 * (j >> 1);
-                        v[j] = lk9_special(F, level, W8, ipx + kk + off, ipy + y, r0, r1, r2, off);
-                    }
-                    auto lanes = [](uint32_t p, uint32_t q, int sh) {
-                        return (uint32_t)((int)(int16_t)(p >> sh) + 8192) | ((uint32_t)((int)(int16_t)(q >> sh) + 8192) << 16);
-                    };
-                    xa = lanes(v[0], v[1], 0); xb = lanes(v[2], v[3], 0);
-                    ya = lanes(v[0], v[1], 16); yb = lanes(v[2], v[3], 16);
+                    const uint4 v = lk9_special4(F, level, W8, ipx + kk, ipy + y, r0, r1, r2);
+                    xa = v.x; xb = v.y; ya = v.z; yb = v.w;
                 }
                 const uint32_t pair = __byte_perm(r1.x, r1.y, 0x6521);     // bytes c, c+1, c+4, c+5
                 if (y > 0) {
@@ -925,30 +935,30 @@ __global__ void __launch_bounds__(kL9Warps * 32, 4) k_lk_track9(agocuda_lk_frame
             A11 = total(s11); A12 = total(s12); A22 = total(s22);
         }
         if (__any_sync(kAll, whole)) {
-            // integer path: int sums of columns 0..3, of 4..7 and column 8, added in that order
-            float c11 = 0.f, c12 = 0.f, c22 = 0.f;
-            const int across1 = base + (kk ^ 1), across2 = base + (kk ^ 2);   // of lanes 0..3; lane 4's sum is not used
-            auto sum4 = [&](int v) {
-                const int s = v + __shfl_sync(kAll, v, across1);
-                return s + __shfl_sync(kAll, s, across2);
-            };
+            // integer path: int sums of columns 0..3, of 4..7 and column 8, added in that order; lane
+            // q of a point adds entry q
+            __syncwarp();
 #pragma unroll
             for (int i = 0; i < win; i++) {
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int x = k == 4 ? 0 : (int)gX[h][i], y = k == 4 ? 0 : (int)gY[h][i];
-                    c11 = __fadd_rn(c11, (float)sum4(x * x));
-                    c12 = __fadd_rn(c12, (float)sum4(x * y));
-                    c22 = __fadd_rn(c22, (float)sum4(y * y));
-                }
-                const int x = __shfl_sync(kAll, __float_as_int(gX[0][i]), base + 4), y = __shfl_sync(kAll, __float_as_int(gY[0][i]), base + 4);
-                c11 = __fadd_rn(c11, (float)(x * x));
-                c12 = __fadd_rn(c12, (float)(x * y));
-                c22 = __fadd_rn(c22, (float)(y * y));
+                auto pack = [](int x, int y) { return (uint32_t)(uint16_t)x | ((uint32_t)y << 16); };
+                grad[2 * i][lane] = k == 4 ? 0u : pack((int)gX[0][i], (int)gY[0][i]);
+                grad[2 * i + 1][lane] = pack((int)gX[1][i], (int)gY[1][i]);
             }
-            c11 = __shfl_sync(kAll, c11, base);            // lane 4 has no sums of its own
-            c12 = __shfl_sync(kAll, c12, base);
-            c22 = __shfl_sync(kAll, c22, base);
+            __syncwarp();
+            float c = 0.f;
+            auto product = [&](uint32_t v) {
+                const int x = (int16_t)(v & 0xffff), y = (int)v >> 16;
+                return (k == 0 || k == 1 ? x : y) * (k == 0 ? x : y);
+            };
+#pragma unroll 1
+            for (int i = 0; i < 2 * win; i++) {
+                int v = 0;
+#pragma unroll
+                for (int j = 0; j < 4; j++) v += product(grad[i][base + j]);
+                c = __fadd_rn(c, (float)v);
+                if (i & 1) c = __fadd_rn(c, (float)product(grad[i][base + 4]));
+            }
+            const float c11 = __shfl_sync(kAll, c, base), c12 = __shfl_sync(kAll, c, base + 1), c22 = __shfl_sync(kAll, c, base + 2);
             if (whole) { A11 = c11; A12 = c12; A22 = c22; }
         }
         A11 = __fmul_rn(A11, kFltScale);
