@@ -173,7 +173,7 @@ int agocuda_CannyEdgeTrace_U8_U8XY_noalloc(void *stream, uint32_t width, uint32_
  * kept when >= the upper and left neighbours and > the right and lower ones.  Writes
  * vx_keypoint_t records in raster order, *pCornerCount = min(found, capacity), *pNumCorners =
  * found (either may be NULL).  `scratch` (256-byte aligned) holds
- * agocuda_FastCorners_scratch_size(W, H) bytes.  Four kernels.  HafCpu_FastCorners_XY_U8_
+ * agocuda_FastCorners_scratch_size(W, H) bytes.  Three kernels.  HafCpu_FastCorners_XY_U8_
  * {NoSupression,Supression} (ago_haf_cpu_fast_corners.cpp:414, :599); replaces
  * HipExec_FastCorners_XY_U8_{NoSupression,Supression} (hipvx/hip_host_decls.h:858/863), which
  * append in arbitrary order. */

@@ -654,7 +654,7 @@ static vx_status plain_step(Graph *g, LNode &ln, Step &st)
         const size_t sb = agocuda_FastCorners_scratch_size(w, h);
         void *scr = scratch(g, sb);
         if (!scr) return VX_ERROR_NO_MEMORY;
-        st.num_kernels = 4;
+        st.num_kernels = 3;
         st.launch = [=](cudaStream_t q) {
             return agocuda_FastCorners_XY_U8(S(q), w, h, s, ss, thr, sup, out, ocap, oc, nc, scr, sb);
         };

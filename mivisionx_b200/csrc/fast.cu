@@ -14,19 +14,21 @@
 // scalar holds every corner, the array min(count, capacity).  The reference's GPU path
 // appends with atomics; this one keeps the CPU path's order.
 //
-// Four launches: k_fast_map (strengths / flags, one 128x8 tile per CTA staged in shared
-// memory), k_fast_rows (a warp per row, a lane per 32 pixels: suppression, bitmap and row
-// count), k_fast_scan (one CTA: row offsets and counts) and k_fast_emit (a warp per row writes
-// its keypoints at its offset, a lane per bitmap word).  Corners are rare, so what bounds the map
-// is the circle test itself: it runs on the four pixels of a word at once, one byte each.
+// Three launches: k_fast_tile (a 128x13 tile per CTA: circle tests on the four pixels of a word
+// at once, strengths of the few corners from a compacted list, suppression inside the tile with
+// a one-pixel halo; the corners as a bitmap, their strengths, and a count per tile row),
+// k_fast_scan (one CTA: row offsets and counts) and k_fast_emit (a warp per row writes its
+// keypoints at its offset, a lane per bitmap word).  A strength map in memory and a second pass
+// for the suppression took 25 + 25 us per 1080p frame.
 #include "agocuda_internal.cuh"
 
 uint64_t agocuda_count_launch(unsigned n);
 
 namespace {
 
-constexpr int kFtX = 128, kFtY = 8, kFtHalo = 4;
-constexpr int kFtSW = kFtX + 2 * kFtHalo, kFtSH = kFtY + 6;   // 136 x 14 bytes
+constexpr int kFtX = 128, kFtY = 13, kFtHalo = 4;             // 15 tested rows of 34 words: 510 of 512 items
+constexpr int kFtSW = kFtX + 2 * kFtHalo, kFtTH = kFtY + 2, kFtSH = kFtTH + 6;   // 136 bytes, 15 tested rows, 21 source rows
+constexpr int kFtWords = kFtSW / 4;
 
 __device__ __constant__ int8_t kCircleDx[16] = {0, 1, 2, 3, 3, 3, 2, 1, 0, -1, -2, -3, -3, -3, -2, -1};
 __device__ __constant__ int8_t kCircleDy[16] = {-3, -3, -2, -1, 0, 1, 2, 3, 3, 3, 2, 1, 0, -1, -2, -3};
@@ -76,44 +78,22 @@ __device__ __forceinline__ int best_arc_min(const int d[16])
     return best;
 }
 
-// map: suppression -> strength (0 = no corner) for rows 3..H-4, columns 3..W-4; otherwise 1 for
-// a corner in rows 3..H-4 (every column).  Every other pixel of the map is written 0.
+// Corner flags of the four pixels of tile word q (columns x0-4+4q ..) of tested row tr (image row
+// y0-1+tr): bit 7 of each byte of `plus` (brighter arc) and `minus`.
 //
-// PACKED (t >= 0): the tests c + t < p and p < c - t of the four pixels of a word in byte lanes,
-// with saturated bounds (a bound of 255 or 0 is never passed, as the unsaturated one); the arcs
-// by ANDs of the 16 circle words.  One pixel at a time took 16 byte loads and 32 compares each:
-// 25 us per 1080p frame.  Negative thresholds take the other form.
-template <bool SUP, bool PACKED>
-__global__ void __launch_bounds__(256) k_fast_map(int W, int H, const uint8_t *src, int srcStride, int t, uint8_t *map,
-                                                 int mapStride)
+// PACKED (t >= 0): the tests c + t < p and p < c - t in byte lanes, with saturated bounds (a
+// bound of 255 or 0 is never passed, as the unsaturated one); the arcs by ANDs of the 16 circle
+// words.  One pixel at a time takes 16 byte loads and 32 compares each; negative thresholds do.
+template <bool PACKED>
+__device__ __forceinline__ void fast_flags(const uint8_t (*tile)[kFtSW], int tr, int q, int t, uint32_t &plus, uint32_t &minus)
 {
-    __shared__ __align__(16) uint8_t tile[kFtSH][kFtSW];
-    const int x0 = blockIdx.x * kFtX, y0 = blockIdx.y * kFtY;
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    const bool edge = x0 - kFtHalo < 0 || x0 + kFtX + kFtHalo > W || y0 - 3 < 0 || y0 + kFtY + 3 > H;
-    if (!edge) {
-        for (int i = tid; i < kFtSH * (kFtSW / 4); i += 256) {
-            const int r = i / (kFtSW / 4), w = i - r * (kFtSW / 4);
-            *(uint32_t *)&tile[r][4 * w] = ldg_u32(src + (size_t)(y0 - 3 + r) * srcStride + x0 - kFtHalo + 4 * w);
-        }
-    } else {
-        // image-edge tiles: bytes as AGO's layout holds them (across row ends, zero outside)
-        for (int i = tid; i < kFtSH * kFtSW; i += 256) {
-            const int r = i / kFtSW, c = i - r * kFtSW;
-            tile[r][c] = (uint8_t)ago_byte(src, (size_t)srcStride, W, H, y0 - 3 + r, x0 - kFtHalo + c);
-        }
-    }
-    __syncthreads();
-    const int y = y0 + threadIdx.y;
-    if (y >= H) return;
-    const int lx0 = 4 * threadIdx.x;
-    uint32_t out = 0, plus4 = 0, minus4 = 0;
     if constexpr (PACKED) {
         uint32_t f[16], g[16], c = 0, hi = 0, lo = 0;
         const uint32_t T = (uint32_t)min(t, 255) * 0x01010101u;
+        const int ql = max(q - 1, 0), qr = min(q + 1, kFtWords - 1);   // outer words: pixels that are not used
         auto row = [&](int dy, uint32_t w[3]) {
-            const uint32_t *p = (const uint32_t *)&tile[3 + threadIdx.y + dy][lx0];
-            w[0] = p[0]; w[1] = p[1]; w[2] = p[2];
+            const uint32_t *p = (const uint32_t *)tile[3 + tr + dy];
+            w[0] = p[ql]; w[1] = p[q]; w[2] = p[qr];
         };
         auto at = [](const uint32_t w[3], int dx) {        // the four pixels dx columns to the right
             return dx == 0 ? w[1] : dx > 0 ? __funnelshift_r(w[1], w[2], 8 * dx) : __funnelshift_r(w[0], w[1], 32 + 8 * dx);
@@ -131,105 +111,134 @@ __global__ void __launch_bounds__(256) k_fast_map(int W, int H, const uint8_t *s
         row(2, w); test(10, at(w, -2)); test(6, at(w, 2));
         row(-1, w); test(13, at(w, -3)); test(3, at(w, 3));
         row(1, w); test(11, at(w, -3)); test(5, at(w, 3));
-        plus4 = arc9x4(f) & 0x80808080u;
-        minus4 = arc9x4(g) & 0x80808080u;
-    }
+        plus = arc9x4(f) & 0x80808080u;
+        minus = arc9x4(g) & 0x80808080u;
+    } else {
+        plus = minus = 0;
+        for (int j = 0; j < 4; j++) {
+            const int cx = 4 * q + j, cy = 3 + tr;
+            if (cx < kFtHalo - 1 || cx > kFtHalo + kFtX) continue;
+            const int c = tile[cy][cx], hi = (int16_t)(c + t), lo = (int16_t)(c - t);
+            uint32_t p = 0, m = 0;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        if (PACKED && !(((plus4 | minus4) >> (8 * q)) & 0x80)) continue;
-        const int x = x0 + lx0 + q;
-        const bool cand = y >= 3 && y < H - 3 && x < W && (!SUP || (x >= 3 && x < W - 3));
-        int v = 0;
-        if (cand) {
-            const int cx = kFtHalo + lx0 + q, cy = 3 + threadIdx.y;
-            const int c = tile[cy][cx];
-            int b[16];
-#pragma unroll
-            for (int i = 0; i < 16; i++) b[i] = tile[cy + kCircleDy[i]][cx + kCircleDx[i]];
-            bool cp, cm;
-            if constexpr (PACKED) {
-                cp = (plus4 >> (8 * q)) & 0x80;
-                cm = (minus4 >> (8 * q)) & 0x80;
-            } else {
-                const int hi = (int16_t)(c + t), lo = (int16_t)(c - t);
-                uint32_t plus = 0, minus = 0;
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    plus |= (uint32_t)(b[i] > hi) << i;
-                    minus |= (uint32_t)(b[i] < lo) << i;
-                }
-                cp = arc9(plus);
-                cm = arc9(minus);
+            for (int i = 0; i < 16; i++) {
+                const int b = tile[cy + kCircleDy[i]][cx + kCircleDx[i]];
+                p |= (uint32_t)(b > hi) << i;
+                m |= (uint32_t)(b < lo) << i;
             }
-            if (!SUP) {
-                v = cp || cm;
-            } else if (cp || cm) {
-                int d[16];
-                int sp = 0, sn = 0;
-                if (cp) {
-#pragma unroll
-                    for (int i = 0; i < 16; i++) d[i] = b[i] - c;
-                    sp = best_arc_min(d) - 1;
-                }
-                if (cm) {
-#pragma unroll
-                    for (int i = 0; i < 16; i++) d[i] = c - b[i];
-                    sn = best_arc_min(d) - 1;
-                }
-                v = (uint8_t)max(sp, sn);
-            }
+            plus |= arc9(p) ? 0x80u << (8 * j) : 0u;
+            minus |= arc9(m) ? 0x80u << (8 * j) : 0u;
         }
-        out |= (uint32_t)(v & 0xff) << (8 * q);
     }
-    const int x = x0 + lx0;
-    uint8_t *d = map + (size_t)y * mapStride + x;
-    if (x + 4 <= mapStride) *(uint32_t *)d = out;
-    else for (int q = 0; q < mapStride - x; q++) d[q] = (uint8_t)(out >> (8 * q));
 }
 
-// one warp per row, 32 pixels per lane: the surviving corners as a bitmap and their count
-template <bool SUP>
-__global__ void __launch_bounds__(256) k_fast_rows(int W, int H, const uint8_t *map, int mapStride, uint32_t *bitmap,
-                                                  int words, uint32_t *rowCount)
+// Corners: with suppression of rows 3..H-4 and columns 3..W-4, without of rows 3..H-4 and every
+// column.  bitmap: 4 words of a tile row; counts[tile column][row]; map: a corner's strength.
+template <bool SUP, bool PACKED>
+__global__ void __launch_bounds__(256) k_fast_tile(int W, int H, const uint8_t *src, int srcStride, int t, uint8_t *map, int mapStride,
+                                                  uint32_t *bitmap, int words, uint32_t *counts)
 {
-    const int y = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (y >= H) return;
-    uint32_t count = 0;
-    const uint8_t *row = map + (size_t)y * mapStride, *u = row - mapStride, *d = row + mapStride;
-    const bool in = y >= 3 && y < H - 3;
-    for (int w = lane; w < words; w += 32) {
-        uint32_t bits = 0;
-        const int x0 = 32 * w;
-        if (in) {
-            const uint4 a = *(const uint4 *)(row + x0);    // rows are whole 16-byte groups
-            const uint4 b = x0 + 32 <= mapStride ? *(const uint4 *)(row + x0 + 16) : make_uint4(0u, 0u, 0u, 0u);
-            const uint32_t v4[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-                for (uint32_t m = v4[k], q = 0; m; m >>= 8, q++) {
-                    const int v = m & 0xff, x = x0 + 4 * k + q;
-                    if (!v || x >= W) continue;
-                    const bool keep = !SUP || (x >= 3 && x < W - 3 && v >= u[x - 1] && v >= u[x] && v >= u[x + 1] && v >= row[x - 1] &&
-                                               v > row[x + 1] && v > d[x - 1] && v > d[x] && v > d[x + 1]);
-                    bits |= (uint32_t)keep << (4 * k + q);
-                }
+    __shared__ __align__(16) uint8_t tile[kFtSH][kFtSW];
+    __shared__ __align__(16) uint8_t str[kFtTH][kFtSW];
+    __shared__ uint16_t list[kFtTH * kFtSW];               // tr * 136 + column, bit 14: brighter arc, bit 15: darker arc
+    __shared__ uint32_t bits[kFtY][4];
+    __shared__ int n;
+    const int x0 = blockIdx.x * kFtX, y0 = blockIdx.y * kFtY, yT = y0 - 4, tid = threadIdx.x;
+    const bool edge = x0 - kFtHalo < 0 || x0 + kFtX + kFtHalo > W || yT < 0 || yT + kFtSH > H;
+    if (!edge) {
+        for (int i = tid; i < kFtSH * kFtWords; i += 256) {
+            const int r = i / kFtWords, w = i - r * kFtWords;
+            *(uint32_t *)&tile[r][4 * w] = ldg_u32(src + (size_t)(yT + r) * srcStride + x0 - kFtHalo + 4 * w);
         }
-        bitmap[(size_t)y * words + w] = bits;
-        count += __popc(bits);
+    } else {
+        // image-edge tiles: bytes as AGO's layout holds them (across row ends, zero outside)
+        for (int i = tid; i < kFtSH * kFtSW; i += 256) {
+            const int r = i / kFtSW, c = i - r * kFtSW;
+            tile[r][c] = (uint8_t)ago_byte(src, (size_t)srcStride, W, H, yT + r, x0 - kFtHalo + c);
+        }
     }
-    count = __reduce_add_sync(0xffffffffu, count);
-    if (lane == 0) rowCount[y] = count;
+    for (int i = tid; i < kFtTH * kFtWords; i += 256) ((uint32_t *)&str[0][0])[i] = 0;
+    if (tid < kFtY * 4) (&bits[0][0])[tid] = 0;
+    if (tid == 0) n = 0;
+    __syncthreads();
+    for (int i = tid; i < kFtTH * kFtWords; i += 256) {
+        const int tr = i / kFtWords, q = i - tr * kFtWords, y = y0 - 1 + tr;
+        if (y < 3 || y >= H - 3 || (!SUP && (tr == 0 || tr == kFtTH - 1))) continue;
+        uint32_t plus, minus;
+        fast_flags<PACKED>(tile, tr, q, t, plus, minus);
+        for (uint32_t m = plus | minus; m; m &= m - 1) {
+            const int j = (__ffs(m) - 1) >> 3, c = 4 * q + j, x = x0 - kFtHalo + c;
+            const bool wanted = SUP ? c >= kFtHalo - 1 && c <= kFtHalo + kFtX && x >= 3 && x < W - 3
+                                    : c >= kFtHalo && c < kFtHalo + kFtX && x < W;
+            if (!wanted) continue;
+            const uint32_t p = (plus >> (8 * j + 7)) & 1, d = (minus >> (8 * j + 7)) & 1;
+            list[atomicAdd(&n, 1)] = (uint16_t)(tr * kFtSW + c + (p << 14) + (d << 15));
+        }
+    }
+    __syncthreads();
+    const int corners = n;
+    if constexpr (SUP) {
+        for (int i = tid; i < corners; i += 256) {
+            const uint32_t e = list[i];
+            const int at = (int)(e & 0x3fff), tr = at / kFtSW, c = at - tr * kFtSW, v = tile[3 + tr][c];
+            int d[16], sp = 0, sn = 0;
+            if (e & 0x4000) {
+#pragma unroll
+                for (int k = 0; k < 16; k++) d[k] = (int)tile[3 + tr + kCircleDy[k]][c + kCircleDx[k]] - v;
+                sp = best_arc_min(d) - 1;
+            }
+            if (e & 0x8000) {
+#pragma unroll
+                for (int k = 0; k < 16; k++) d[k] = v - (int)tile[3 + tr + kCircleDy[k]][c + kCircleDx[k]];
+                sn = best_arc_min(d) - 1;
+            }
+            str[tr][c] = (uint8_t)max(sp, sn);
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < corners; i += 256) {
+        const int at = (int)(list[i] & 0x3fff), tr = at / kFtSW, c = at - tr * kFtSW;
+        if (tr == 0 || tr == kFtTH - 1 || c < kFtHalo || c >= kFtHalo + kFtX) continue;   // the halo's
+        bool keep = true;
+        if constexpr (SUP) {
+            const uint8_t *s = &str[tr][c], *u = s - kFtSW, *d = s + kFtSW;
+            const int v = s[0];
+            keep = v && v >= u[-1] && v >= u[0] && v >= u[1] && v >= s[-1] && v > s[1] && v > d[-1] && v > d[0] && v > d[1];
+            if (keep) map[(size_t)(y0 - 1 + tr) * mapStride + x0 - kFtHalo + c] = (uint8_t)v;
+        }
+        if (keep) atomicOr(&bits[tr - 1][(c - kFtHalo) >> 5], 1u << ((c - kFtHalo) & 31));
+    }
+    __syncthreads();
+    if (tid < kFtY * 4) {
+        const int r = tid >> 2, w = (x0 >> 5) + (tid & 3), y = y0 + r;
+        uint32_t k = __popc(bits[r][tid & 3]);
+        if (y < H && w < words) bitmap[(size_t)y * words + w] = bits[r][tid & 3];
+        const unsigned quad = 0xfu << (tid & 28);          // the four words of the row
+        k += __shfl_xor_sync(quad, k, 1);
+        k += __shfl_xor_sync(quad, k, 2);
+        if (y < H && (tid & 3) == 0) counts[(size_t)blockIdx.x * H + y] = k;
+    }
 }
 
 // one CTA of 1024 threads: exclusive scan of the row counts; the totals
-__global__ void __launch_bounds__(1024) k_fast_scan(int H, const uint32_t *rowCount, uint32_t *rowStart, uint32_t capacity,
+__global__ void __launch_bounds__(1024) k_fast_scan(int H, int tiles, const uint32_t *counts, uint32_t *rowStart, uint32_t capacity,
                                                    uint32_t *pCornerCount, uint32_t *pNumCorners)
 {
     __shared__ uint32_t warpSum[32];
     const int per = (H + 1023) / 1024, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int r0 = min(H, tid * per), r1 = min(H, r0 + per);
+    auto row_count = [&](int r) {
+        uint32_t c = 0;
+#pragma unroll 8
+        for (int k = 0; k < tiles; k++) c += counts[(size_t)k * H + r];
+        return c;
+    };
     uint32_t s = 0;
-    for (int r = r0; r < r1; r++) s += rowCount[r];
+    for (int r = r0; r < r1; r++) {
+        const uint32_t c = row_count(r);
+        rowStart[r] = c;                                   // its count until the offsets are known
+        s += c;
+    }
     uint32_t inc = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -250,8 +259,9 @@ __global__ void __launch_bounds__(1024) k_fast_scan(int H, const uint32_t *rowCo
     __syncthreads();
     uint32_t run = warpSum[wid] + inc - s;
     for (int r = r0; r < r1; r++) {
+        const uint32_t c = rowStart[r];
         rowStart[r] = run;
-        run += rowCount[r];
+        run += c;
     }
     if (tid == 1023) {
         const uint32_t total = warpSum[wid] + inc;
@@ -298,8 +308,8 @@ size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 struct FastScratch {
     uint8_t *map;
-    uint32_t *bitmap, *rowCount, *rowStart;
-    int mapStride, words;
+    uint32_t *bitmap, *counts, *rowStart;
+    int mapStride, words, tiles;
     size_t bytes;
 };
 
@@ -308,11 +318,12 @@ FastScratch fast_layout(uint32_t W, uint32_t H, void *base)
     FastScratch s{};
     s.mapStride = (int)((W + 15) & ~15u);
     s.words = (int)((W + 31) / 32);
+    s.tiles = (int)((W + kFtX - 1) / kFtX);
     uint8_t *p = (uint8_t *)base;
     size_t o = 0;
     s.map = p + o; o += align256((size_t)s.mapStride * H);
     s.bitmap = (uint32_t *)(p + o); o += align256((size_t)s.words * H * 4);
-    s.rowCount = (uint32_t *)(p + o); o += align256((size_t)H * 4);
+    s.counts = (uint32_t *)(p + o); o += align256((size_t)s.tiles * H * 4);
     s.rowStart = (uint32_t *)(p + o); o += align256((size_t)H * 4);
     s.bytes = o;
     return s;
@@ -338,23 +349,19 @@ extern "C" int agocuda_FastCorners_XY_U8(void *stream, uint32_t W, uint32_t H, c
     if (scratchBytes < s.bytes) return AGOCUDA_INVALID_PARAMS;
     const int t = (int16_t)floorf(strengthThreshold);
     cudaStream_t q = as_stream(stream);
-    const dim3 g1(div_up(W, kFtX), div_up(H, kFtY)), b1(32, kFtY);
+    const dim3 g1(div_up(W, kFtX), div_up(H, kFtY));
     const unsigned g2 = div_up(H, 8);
     vx_keypoint_like *kp = (vx_keypoint_like *)pCorners;
-    if (nonmaxSuppression) {
-        (t >= 0 ? k_fast_map<true, true> : k_fast_map<true, false>)<<<g1, b1, 0, q>>>((int)W, (int)H, pSrc, (int)srcStride, t, s.map, s.mapStride);
-        k_fast_rows<true><<<g2, 256, 0, q>>>((int)W, (int)H, s.map, s.mapStride, s.bitmap, s.words, s.rowCount);
-    } else {
-        (t >= 0 ? k_fast_map<false, true> : k_fast_map<false, false>)<<<g1, b1, 0, q>>>((int)W, (int)H, pSrc, (int)srcStride, t, s.map, s.mapStride);
-        k_fast_rows<false><<<g2, 256, 0, q>>>((int)W, (int)H, s.map, s.mapStride, s.bitmap, s.words, s.rowCount);
-    }
-    k_fast_scan<<<1, 1024, 0, q>>>((int)H, s.rowCount, s.rowStart, cornerCapacity, pCornerCount, pNumCorners);
+    (nonmaxSuppression ? (t >= 0 ? k_fast_tile<true, true> : k_fast_tile<true, false>)
+                       : (t >= 0 ? k_fast_tile<false, true> : k_fast_tile<false, false>))<<<g1, 256, 0, q>>>(
+        (int)W, (int)H, pSrc, (int)srcStride, t, s.map, s.mapStride, s.bitmap, s.words, s.counts);
+    k_fast_scan<<<1, 1024, 0, q>>>((int)H, s.tiles, s.counts, s.rowStart, cornerCapacity, pCornerCount, pNumCorners);
     if (nonmaxSuppression)
         k_fast_emit<true><<<g2, 256, 0, q>>>((int)W, (int)H, s.map, s.mapStride, s.bitmap, s.words, s.rowStart,
                                              cornerCapacity, kp, strengthThreshold);
     else
         k_fast_emit<false><<<g2, 256, 0, q>>>((int)W, (int)H, s.map, s.mapStride, s.bitmap, s.words, s.rowStart,
                                               cornerCapacity, kp, strengthThreshold);
-    agocuda_count_launch(4);
+    agocuda_count_launch(3);
     return agocuda_launch_status();
 }
