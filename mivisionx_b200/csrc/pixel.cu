@@ -1157,13 +1157,21 @@ constexpr int kIiCols = 128, kIiRows = 32, kIiWarps = 4;
 // scratch: column sums [tile row][W], row sums and left sums [tile column][H]
 struct IiScratch { uint32_t *cols, *rows, *left; int tx, ty; };
 
-// the four pixels from column x on (zeros from W on)
-__device__ __forceinline__ uint32_t ii_word(const uint8_t *row, int x, int W, bool words)
+// the four pixels from column x on (zeros from W on) of `ROWS` rows; rows from n on read 0.  Whole
+// words are loaded before any is used: a lane's rows are one dependent chain otherwise.
+template <int ROWS>
+__device__ __forceinline__ void ii_words(const uint8_t *p, int stride, int n, int x, int W, bool words, uint32_t w[ROWS])
 {
-    if (words && x + 4 <= W) return __ldg((const uint32_t *)(row + x));
-    uint32_t w = 0;
-    for (int k = 0; k < 4 && x + k < W; k++) w |= (uint32_t)row[x + k] << (8 * k);
-    return w;
+    if (words && x + 4 <= W) {
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) w[r] = r < n ? __ldg((const uint32_t *)(p + (size_t)r * stride + x)) : 0u;
+    } else {
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            w[r] = 0;
+            for (int k = 0; k < 4 && x + k < W && r < n; k++) w[r] |= (uint32_t)p[(size_t)r * stride + x + k] << (8 * k);
+        }
+    }
 }
 
 __global__ void __launch_bounds__(kIiWarps * 32)
@@ -1174,13 +1182,16 @@ k_integral_sums(int W, int H, const uint8_t *src, int srcStride, IiScratch S, bo
     const int tx = t % S.tx, ty = t / S.tx, x = tx * kIiCols + 4 * lane, y0 = ty * kIiRows, n = min(kIiRows, H - y0);
     const uint8_t *p = src + (size_t)y0 * srcStride;
     uint32_t e = 0, o = 0, mine = 0;                       // 32 bytes of 255 fit a 16-bit lane
-#pragma unroll 8
-    for (int r = 0; r < kIiRows; r++) {
-        const uint32_t w = r < n ? ii_word(p + (size_t)r * srcStride, x, W, words) : 0u;
-        e += w & 0x00ff00ffu;
-        o += (w >> 8) & 0x00ff00ffu;
-        const uint32_t s = __reduce_add_sync(0xffffffffu, __dp4a(w, 0x01010101u, 0u));
-        if (lane == r) mine = s;
+    for (int r0 = 0; r0 < kIiRows; r0 += 8) {
+        uint32_t w[8];
+        ii_words<8>(p + (size_t)r0 * srcStride, srcStride, n - r0, x, W, words, w);
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            e += w[r] & 0x00ff00ffu;
+            o += (w[r] >> 8) & 0x00ff00ffu;
+            const uint32_t s = __reduce_add_sync(0xffffffffu, __dp4a(w[r], 0x01010101u, 0u));
+            if (lane == r0 + r) mine = s;
+        }
     }
     if (lane < n) S.rows[(size_t)tx * H + y0 + lane] = mine;
     const uint32_t c[4] = {e & 0xffff, o & 0xffff, e >> 16, o >> 16};
@@ -1193,14 +1204,18 @@ __global__ void __launch_bounds__(1024) k_integral_scan(int W, int H, IiScratch 
 {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if ((int)blockIdx.x >= S.tx) {
-        const int x = ((int)blockIdx.x - S.tx) * 1024 + tid;
-        if (x >= W) return;
+        const int x = ((int)blockIdx.x - S.tx) * 128 + tid;
+        if (x >= W || tid >= 128) return;                  // a few threads per SM: one chain of loads each
         uint32_t run = 0;
-#pragma unroll 4
-        for (int t = 0; t < S.ty; t++) {
-            const uint32_t v = S.cols[(size_t)t * W + x];
-            S.cols[(size_t)t * W + x] = run;
-            run += v;
+        for (int t0 = 0; t0 < S.ty; t0 += 16) {            // loads first: they may not pass the stores
+            uint32_t v[16];
+#pragma unroll
+            for (int t = 0; t < 16; t++) v[t] = t0 + t < S.ty ? S.cols[(size_t)(t0 + t) * W + x] : 0u;
+#pragma unroll
+            for (int t = 0; t < 16; t++) {
+                if (t0 + t < S.ty) S.cols[(size_t)(t0 + t) * W + x] = run;
+                run += v[t];
+            }
         }
         return;
     }
@@ -1210,7 +1225,7 @@ __global__ void __launch_bounds__(1024) k_integral_scan(int W, int H, IiScratch 
         const int y = y0 + tid;
         uint32_t v = 0;
         if (y < H)
-#pragma unroll 4
+#pragma unroll 8
             for (int t = 0; t < (int)blockIdx.x; t++) v += S.rows[(size_t)t * H + y];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1243,9 +1258,14 @@ k_integral_tiles(int W, int H, uint32_t *dst, int dstStride, const uint8_t *src,
     for (int k = 0; k < 4 && x + k < W; k++) c[k] = S.cols[(size_t)ty * W + x + k];
     const uint32_t left = lane < n ? S.left[(size_t)tx * H + y0 + lane] : 0;
     const bool vec = (((uintptr_t)dst | (uintptr_t)dstStride) & 15) == 0 && x + 4 <= W;
-#pragma unroll 4
-    for (int r = 0; r < n; r++) {
-        const uint32_t w = ii_word(p + (size_t)r * srcStride, x, W, words);
+    for (int r0 = 0; r0 < n; r0 += 8) {
+      uint32_t ws[8];
+      ii_words<8>(p + (size_t)r0 * srcStride, srcStride, n - r0, x, W, words, ws);
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int r = r0 + q;
+        if (r >= n) break;
+        const uint32_t w = ws[q];
         c[0] += w & 0xff;
         c[1] += (w >> 8) & 0xff;
         c[2] += (w >> 16) & 0xff;
@@ -1263,6 +1283,7 @@ k_integral_tiles(int W, int H, uint32_t *dst, int dstStride, const uint8_t *src,
         if (vec) *(uint4 *)d = make_uint4(v[0], v[1], v[2], v[3]);
         else
             for (int k = 0; k < 4 && x + k < W; k++) d[k] = v[k];
+      }
     }
 }
 
@@ -1291,7 +1312,7 @@ extern "C" int agocuda_IntegralImage_U32_U8(void *stream, uint32_t dstWidth, uin
     const bool words = (((uintptr_t)pSrc | srcStride) & 3) == 0;
     const unsigned tiles = div_up((unsigned)(S.tx * S.ty), kIiWarps);
     k_integral_sums<<<tiles, kIiWarps * 32, 0, s>>>((int)W, (int)H, pSrc, (int)srcStride, S, words);
-    k_integral_scan<<<S.tx + div_up(W, 1024), 1024, 0, s>>>((int)W, (int)H, S);
+    k_integral_scan<<<S.tx + div_up(W, 128), 1024, 0, s>>>((int)W, (int)H, S);
     k_integral_tiles<<<tiles, kIiWarps * 32, 0, s>>>((int)W, (int)H, pDst, (int)dstStride, pSrc, (int)srcStride, S, words);
     agocuda_count_launch(3);
     return agocuda_launch_status();

@@ -205,3 +205,35 @@ def test_adjoint_at_strip_edges(cuda, H, W, kind):
         gs, gf = D.remap_adjoint(img[i].astype(np.float64), f, tgt[i].astype(np.float64))
         assert np.abs(src.grad[i].cpu().numpy() - gs).max() <= 1e-5 * max(np.abs(gs).max(), 1.0)
         assert np.abs(field.grad[i].cpu().numpy() - gf).max() <= 1e-5 * max(np.abs(gf).max(), 1.0)
+
+
+def test_source_beyond_int_indexes(cuda):
+    """A source whose element indexes pass 2^31 (two rows 2^30 elements apart)."""
+    import ctypes as CT
+    import torch
+
+    from devbuf import stream_ptr
+    from mivisionx_b200 import diffwarp
+    W, H, stride = 40, 2, 1 << 30
+    rng = np.random.default_rng(3)
+    img, g = rng.random((H, W)).astype(np.float32), rng.random((H, W)).astype(np.float32)
+    big = torch.empty(stride + W, dtype=torch.float32, device="cuda")
+    rows = torch.as_strided(big, (H, W), (stride, 1))
+    rows.copy_(torch.from_numpy(img))
+    theta = np.array([1.02, 0.01, -0.01, 0.97, 0.3, 0.2], np.float32)
+    th, gout = torch.from_numpy(theta).cuda(), torch.from_numpy(g).cuda()
+    out, gth = torch.zeros(H, W, device="cuda"), torch.zeros(6, dtype=torch.float64, device="cuda")
+    L = diffwarp._L()
+    assert L.agocuda_WarpAffine_F32_Bilinear_Constant_batch(stream_ptr(), 1, W, H, out.data_ptr(), H * W, W, W, H, big.data_ptr(),
+                                                            0, stride, th.data_ptr(), 0.0) == 0
+    gbig = torch.empty(stride + W, dtype=torch.float32, device="cuda")
+    grows = torch.as_strided(gbig, (H, W), (stride, 1))
+    grows.zero_()
+    assert L.agocuda_WarpAffine_F32_Bilinear_Constant_adjoint_batch(
+        stream_ptr(), 1, W, H, gout.data_ptr(), H * W, W, W, H, big.data_ptr(), 0, stride, th.data_ptr(), 0.0, gbig.data_ptr(),
+        gth.data_ptr()) == 0
+    t64 = theta.astype(np.float64)
+    assert np.abs(out.cpu().numpy() - D.warp_affine(img.astype(np.float64), t64)).max() <= 2e-5
+    gs, gt = D.warp_affine_adjoint(img.astype(np.float64), t64, g.astype(np.float64))
+    close_grad(grows.cpu().numpy(), gs, "gsrc")
+    assert np.abs(gth.cpu().numpy() - gt).max() <= 1e-6 * 4 * H * W * W
