@@ -508,22 +508,6 @@ struct CannyTiles {
     int tilesX, tilesY;
 };
 
-// global node of the open component at pixel (x, y), which lies on its tile's border ring;
-// -1 where that pixel is not an edge candidate
-__device__ __forceinline__ int ring_node(const CannyTiles &T, int x, int y)
-{
-    const int tx = x / kTW, ty = y / kTH, lx = x - tx * kTW, ly = y - ty * kTH;
-    const int tile = ty * T.tilesX + tx;
-    int idx;
-    if (ly == 0) idx = lx;
-    else if (ly == kTH - 1) idx = kTW + lx;
-    else if (lx == 0) idx = 2 * kTW + ly;
-    else if (lx == kTW - 1) idx = 2 * kTW + kTH + ly;
-    else return -1;
-    const int s = __ldg(T.blab + (size_t)tile * kBorder + idx);
-    return s < 0 ? -1 : tile * kOpenMax + s;
-}
-
 // union-find over the tile's runs in shared memory
 __device__ __forceinline__ int sfind(const int *lab, int x)
 {
@@ -923,44 +907,67 @@ k_canny_ccl_front(int W, int H, const uint8_t *__restrict__ src, int srcStride, 
     }
 }
 
-// unions across tile borders: the W / NW / N / NE neighbours of a tile's left column, top
-// row and right column that lie in another tile (both ends are ring pixels of their tiles)
-__global__ void k_canny_ccl_border(int W, int H, CannyTiles T, uint32_t *err)
+// Unions across tile borders, three warps per tile: the halves of its top row with the row above,
+// and its left column with the column before and its right column with the upper right ones.
+// A pixel joins its N (W) neighbour, or else NW and NE (NW): those touch the N (W) one, so it
+// has them already.  A warp loads all its labels at once, and a pixel whose left (upper)
+// neighbour makes the same join leaves it out; with a thread per ring pixel, its neighbours
+// loaded one after another, the pass took 14 us per 4K frame for a few thousand joins.
+__global__ void __launch_bounds__(192) k_canny_ccl_border(int tiles, CannyTiles T, uint32_t *err)
 {
-    constexpr int kPer = kTH + kTW + kTH;
-    const int tile = blockIdx.y, b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= kPer) return;
-    const int x0 = (tile % T.tilesX) * kTW, y0 = (tile / T.tilesX) * kTH;
-    int x, y;
-    if (b < kTH) { x = x0; y = y0 + b; }
-    else if (b < kTH + kTW) { x = x0 + b - kTH; y = y0; }
-    else { x = x0 + kTW - 1; y = y0 + b - kTH - kTW; }
-    if (x >= W || y >= H) return;
-    const int sp = ring_node(T, x, y);
-    if (sp < 0) return;
-    const int dx[4] = {-1, -1, 0, 1}, dy[4] = {0, -1, -1, -1};
-    for (int k = 0; k < 4; k++) {
-        const int nx = x + dx[k], ny = y + dy[k];
-        if (nx < 0 || ny < 0 || nx >= W) continue;
-        if (nx >= x0 && nx < x0 + kTW && ny >= y0) continue;     // same tile: done locally
-        const int sq = ring_node(T, nx, ny);
-        if (sq >= 0) uf_union(T.uf, sp, sq, err);
+    const int warp = threadIdx.x >> 5, tile = blockIdx.x * 2 + warp / 3, part = warp % 3, lane = threadIdx.x & 31;
+    if (tile >= tiles) return;
+    const unsigned kAll = 0xffffffffu;
+    const int tx = tile % T.tilesX, above = tile - T.tilesX;
+    const bool hasL = tx > 0, hasR = tx + 1 < T.tilesX, hasA = above >= 0;
+    auto node = [&](bool has, int t, int i) {
+        const int l = has ? (int)__ldg(T.blab + (size_t)t * kBorder + i) : -1;
+        return l < 0 ? -1 : t * kOpenMax + l;
+    };
+    // joins nodes p and q of every lane that has both, once per run of equal joins
+    auto join = [&](int p, int q) {
+        const bool has = p >= 0 && q >= 0;
+        const int pu = __shfl_up_sync(kAll, has ? p : -1, 1), qu = __shfl_up_sync(kAll, has ? q : -1, 1);
+        if (has && !(lane > 0 && pu == p && qu == q)) uf_union(T.uf, p, q, err);
+        __syncwarp();
+    };
+    if (part < 2) {                                        // 32 columns of the top row
+        if (!hasA) return;
+        const int at = part * 32 + lane, p = node(true, tile, at), n = node(true, above, kTW + at);
+        // what lies outside the 32 columns: lane 0 loads the NW, lane 31 the NE one
+        int side = -1;
+        if (lane == 0) side = part ? node(true, above, kTW + 31) : node(hasL, above - 1, 2 * kTW - 1);
+        if (lane == 31) side = part ? node(hasR, above + 1, kTW) : node(true, above, kTW + 32);
+        int nw = __shfl_up_sync(kAll, n, 1), ne = __shfl_down_sync(kAll, n, 1);
+        if (lane == 0) nw = side;
+        if (lane == 31) ne = side;
+        join(p, n >= 0 ? n : nw);
+        join(p, n >= 0 ? -1 : ne);
+    } else {
+        const int p = node(hasL, tile, 2 * kTW + lane), w = node(hasL, tile - 1, 2 * kTW + kTH + lane);
+        const int q = node(hasR, tile, 2 * kTW + kTH + lane), e = node(hasR, tile + 1, 2 * kTW + lane);
+        // lane 0's upper neighbours are the top row's; a pixel's SW is the NE of the tile on the left
+        int nw = __shfl_up_sync(kAll, w, 1), ne = __shfl_up_sync(kAll, e, 1);
+        if (lane == 0) nw = ne = -1;
+        join(p, w >= 0 ? w : nw);
+        join(q, ne);
     }
 }
 
 // after the unions: every open node points straight at its component's root (path
 // compression; concurrent readers see the old parent or the root, both lead to the root),
-// and a node holding a strong pixel sets its root's strong bit.  One thread per node.
-__global__ void k_canny_ccl_flatten(CannyTiles T, int nodes)
+// and a node holding a strong pixel sets its root's strong bit.  A warp per tile.
+__global__ void __launch_bounds__(256) k_canny_ccl_flatten(int tiles, CannyTiles T)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nodes) return;
-    const int tile = i / kOpenMax, o = i - tile * kOpenMax;
-    if (o >= (int)__ldg(T.nOpen + tile)) return;
-    const int rt = uf_find(T.uf, i);
-    if (rt != i) {
-        T.uf[i] = rt;
-        if ((__ldcg(T.sbits + (i >> 5)) >> (i & 31)) & 1) atomicOr(T.sbits + (rt >> 5), 1u << (rt & 31));
+    const int tile = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (tile >= tiles) return;
+    const int n = (int)__ldg(T.nOpen + tile);
+    for (int o = lane; o < n; o += 32) {
+        const int i = tile * kOpenMax + o, rt = uf_find(T.uf, i);
+        if (rt != i) {
+            T.uf[i] = rt;
+            if ((__ldcg(T.sbits + (i >> 5)) >> (i & 31)) & 1) atomicOr(T.sbits + (rt >> 5), 1u << (rt & 31));
+        }
     }
 }
 
@@ -1992,12 +1999,11 @@ static size_t canny_tiles_layout(uint32_t W, uint32_t H, void *base, CannyTiles 
 }
 
 // what follows the front: unions across tile borders, flatten, patch
-static void canny_ccl_tail(cudaStream_t s, int W, int H, uint8_t *dst, int dstStride, const CannyTiles &T, uint32_t *status)
+static void canny_ccl_tail(cudaStream_t s, uint8_t *dst, int dstStride, const CannyTiles &T, uint32_t *status)
 {
-    const int tiles = T.tilesX * T.tilesY, nodes = tiles * kOpenMax;
-    constexpr int kPer = kTH + kTW + kTH;
-    k_canny_ccl_border<<<dim3(div_up(kPer, 128), tiles), 128, 0, s>>>(W, H, T, status);
-    k_canny_ccl_flatten<<<div_up(nodes, 256), 256, 0, s>>>(T, nodes);
+    const int tiles = T.tilesX * T.tilesY;
+    k_canny_ccl_border<<<div_up(tiles, 2), 192, 0, s>>>(tiles, T, status);
+    k_canny_ccl_flatten<<<div_up(tiles, 8), 256, 0, s>>>(tiles, T);
     k_canny_ccl_patch<<<div_up(tiles, 8), 256, 0, s>>>(tiles, T, dst, dstStride);
     agocuda_count_launch(3);
 }
@@ -2023,7 +2029,7 @@ extern "C" int agocuda_fused_CannyEdgeDetector_3x3_L1(void *stream, uint32_t W, 
         k_canny_ccl_front<kCannyWords><<<dim3(T.tilesX, T.tilesY), 256, 0, s>>>(
             (int)W, (int)H, pSrc, (int)srcStride, hystLower, hystUpper, pDst, (int)dstStride, T, pStatus, map);
     agocuda_count_launch(1);
-    canny_ccl_tail(s, (int)W, (int)H, pDst, (int)dstStride, T, pStatus);
+    canny_ccl_tail(s, pDst, (int)dstStride, T, pStatus);
     return agocuda_launch_status();
 }
 
@@ -2059,7 +2065,7 @@ extern "C" int agocuda_fused_CannyEdgeDetector_NxN(void *stream, uint32_t W, uin
     k_canny_ccl_front<kCannyPlane><<<dim3(T.tilesX, T.tilesY), 256, 0, s>>>(
         (int)W, (int)H, (const uint8_t *)plane, (int)pitch, hystLower, hystUpper, pDst, (int)dstStride, T, pStatus, map);
     agocuda_count_launch(1);
-    canny_ccl_tail(s, (int)W, (int)H, pDst, (int)dstStride, T, pStatus);
+    canny_ccl_tail(s, pDst, (int)dstStride, T, pStatus);
     return agocuda_launch_status();
 }
 
