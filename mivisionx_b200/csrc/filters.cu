@@ -7,6 +7,7 @@
 // loaded once per thread (the neighbouring words come from L1).  A warp covers 128
 // contiguous bytes per row, so every global access is a full coalesced line.
 #include "agocuda_internal.cuh"
+#include <cuda_fp16.h>
 #include <math.h>
 #include <string.h>
 
@@ -393,15 +394,17 @@ k_fused_c1_persistent(const agocuda_frame *frames, const uint32_t *tilePrefix, u
 // elements, so a single 72-element box spans the 264 columns the tile reads (a box
 // dimension holds at most 256 elements); TMA writes zeros outside the plane.
 //
-// Each thread owns 8 columns and walks down kC1tRows rows.  The Gaussian stays in 16-bit
-// lanes as in the register form; the Sobel and the threshold test run in exact fp32 on the
-// FMA pipe instead of in lanes:
-//   t  = 6144 + G * 2^-7       the masked 16G lane dropped into the mantissa of 6144 (one permute)
-//   gx = [1 2 1]^T (t[c+1] - t[c-1]),  gy = [1 2 1] (t[r+1] - t[r-1])   = k * 2^-7, |k| <= 1020
-//   r  = T - gx^2 - gy^2,  T = (n_min - 1/2) * 2^-14                   multiples of 2^-15, |r| < 2^8
-// Every value is exact (t in [4096, 8192) has ulp 2^-11), so r < 0 <=> gx^2 + gy^2 >= n_min
-// in integers, r is never 0, and the sign byte of r replicated by one permute is the
+// Each thread owns 8 columns and walks down kC1tRows rows.  The Gaussian's sums run in 16-bit
+// lanes as in the register form; its result G becomes the half 1024 + G (one and-or), and the
+// Sobel runs two columns per instruction on the FMA pipe:
+//   gx = [1 2 1]^T (t[c+1] - t[c-1]),  gy = [1 2 1] (t[r+1] - t[r-1])   integers, |.| <= 1020
+//   r  = gx^2 + gy^2 + T,  T = 1/2 - n_min                             multiples of 1/2, |r| < 2^23
+// Every value is exact: the halves are integers below 2048, the squares are taken by the fused
+// multiply-add that reads halves and adds in fp32.  So r < 0 <=> gx^2 + gy^2 < n_min in
+// integers, r is never 0, and the sign byte of r replicated by one permute and inverted is the
 // output byte (255 where the chain's threshold passes).
+// The bound is instruction issue: 64 1080p frames (265 MB) take 74 us on the device,
+// 3.6 TB/s; with the Sobel in fp32, one column per instruction, they took 88 us.
 // ---------------------------------------------------------------------------------
 constexpr int kC1tRows = 36, kC1tBY = 2;              // default shape (rows per warp, warps per block)
 constexpr int kC1tBoxW = 72;                            // 32-bit elements: 288 bytes per row
@@ -410,15 +413,29 @@ __host__ __device__ constexpr int c1t_box_h(int rows, int by) { return by * rows
 __host__ __device__ constexpr int c1t_min_blocks(int by) { return 65536 / (32 * by * 80); }
 constexpr int kC1tWaitLimit = 1 << 20;                  // bounded mbarrier waits
 
-// t of the lo / hi 16-bit lane of a masked Gaussian word
-__device__ __forceinline__ float c1_tlo(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x45C00000u, 0x7610)); }
-__device__ __forceinline__ float c1_thi(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x45C00000u, 0x7632)); }
-
-// t at columns x-1 .. x+8 from the lane words (x, x+2), (x+1, x+3), (x+4, x+6), (x+5, x+7), (x-1, x+8)
-__device__ __forceinline__ void c1_tcols(const C1Row &g, float *t)
+// A Gaussian row of a thread as halves 1024 + G, in the lane pairs of C1Row, and the pairs one
+// column to the left of e1, e2 (m1, m2) and to the right of o1, o2 (p1, p2)
+struct C1G { __half2 e1, o1, e2, o2, b, m1, p1, m2, p2; };
+__device__ __forceinline__ __half2 c1_as_h2(uint32_t w) { return *(const __half2 *)&w; }
+__device__ __forceinline__ uint32_t c1_gh(uint32_t a, uint32_t b, uint32_t c)
 {
-    t[0] = c1_tlo(g.b);  t[1] = c1_tlo(g.e1); t[2] = c1_tlo(g.o1); t[3] = c1_thi(g.e1); t[4] = c1_thi(g.o1);
-    t[5] = c1_tlo(g.e2); t[6] = c1_tlo(g.o2); t[7] = c1_thi(g.e2); t[8] = c1_thi(g.o2); t[9] = c1_thi(g.b);
+    return (((a + 2 * b + c) >> 4) & 0x00FF00FFu) | 0x64006400u;
+}
+__device__ __forceinline__ C1G c1_gauss_halves(const C1Row &a, const C1Row &b, const C1Row &c)
+{
+    const uint32_t e1 = c1_gh(a.e1, b.e1, c.e1), o1 = c1_gh(a.o1, b.o1, c.o1), e2 = c1_gh(a.e2, b.e2, c.e2);
+    const uint32_t o2 = c1_gh(a.o2, b.o2, c.o2), bb = c1_gh(a.b, b.b, c.b);
+    return C1G{c1_as_h2(e1), c1_as_h2(o1), c1_as_h2(e2), c1_as_h2(o2), c1_as_h2(bb),
+               c1_as_h2(__byte_perm(bb, o1, 0x5410)), c1_as_h2(__byte_perm(e1, e2, 0x5432)),
+               c1_as_h2(__byte_perm(o1, o2, 0x5432)), c1_as_h2(__byte_perm(e2, bb, 0x7632))};
+}
+
+// a * a + c of a half, exact in fp32
+__device__ __forceinline__ float c1_sq(__half a, float c)
+{
+    float r;
+    asm("fma.rn.f32.f16 %0, %1, %1, %2;" : "=f"(r) : "h"(__half_as_ushort(a)), "f"(c));
+    return r;
 }
 
 // bytes 0 and 1: 0xFF where a (resp. b) is negative, else 0 (prmt sign-replicate selectors)
@@ -437,36 +454,44 @@ __device__ __forceinline__ void c1t_rows(HROW &hrow, int ys, int ye, int x, int 
 {
     // rolling rows of output row y: h of input rows y, y+1; t of rows y-1, y; d = t[c+1] - t[c-1]
     // of row y; D = d(y-1) + d(y); all rotated by the 6-way unrolled loop
+    struct C1D { __half2 v[4]; };
+    auto diff = [](const C1G &t) {
+        return C1D{__hsub2(t.o1, t.m1), __hsub2(t.p1, t.e1), __hsub2(t.o2, t.m2), __hsub2(t.p2, t.e2)};
+    };
     C1Row h0, h1, h2;
-    float t0[10], t1[10], t2[10], d0[8], d1[8], D0[8], D1[8];
+    C1G t0, t1, t2;
+    C1D d0, d1, D0, D1;
     {
         const C1Row a = hrow(ys - 2), c = hrow(ys - 1);
         h0 = hrow(ys);
         h1 = hrow(ys + 1);
-        c1_tcols(c1_gauss(a, c, h0), t0);
-        c1_tcols(c1_gauss(c, h0, h1), t1);
+        t0 = c1_gauss_halves(a, c, h0);
+        t1 = c1_gauss_halves(c, h0, h1);
+        d0 = diff(t1);
+        const C1D z = diff(t0);
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            d0[j] = t1[j + 2] - t1[j];
-            D0[j] = (t0[j + 2] - t0[j]) + d0[j];
-        }
+        for (int j = 0; j < 4; j++) D0.v[j] = __hadd2(z.v[j], d0.v[j]);
     }
-    auto step = [&](int y, const C1Row &hA, const C1Row &hB, C1Row &hC, const float *tA, float *tC, const float *dB,
-                    float *dC, const float *DA, float *DB) {
+    const __half2 two = __float2half2_rn(2.f);
+    auto step = [&](int y, const C1Row &hA, const C1Row &hB, C1Row &hC, const C1G &tA, C1G &tC, const C1D &dB,
+                    C1D &dC, const C1D &DA, C1D &DB) {
         hC = hrow(y + 2);
-        c1_tcols(c1_gauss(hA, hB, hC), tC);               // t of row y+1
-        float r[8];
+        tC = c1_gauss_halves(hA, hB, hC);                 // t of row y+1
+        dC = diff(tC);
+        const __half2 e1 = __hsub2(tC.e1, tA.e1), o1 = __hsub2(tC.o1, tA.o1), e2 = __hsub2(tC.e2, tA.e2), o2 = __hsub2(tC.o2, tA.o2);
+        const __half2 m1 = __hsub2(tC.m1, tA.m1), p1 = __hsub2(tC.p1, tA.p1), m2 = __hsub2(tC.m2, tA.m2), p2 = __hsub2(tC.p2, tA.p2);
+        const __half2 gy[4] = {__hadd2(__hfma2(two, e1, m1), o1), __hadd2(__hfma2(two, o1, e1), p1),
+                               __hadd2(__hfma2(two, e2, m2), o2), __hadd2(__hfma2(two, o2, e2), p2)};
+        float lo4[4], hi4[4];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            dC[j] = tC[j + 2] - tC[j];
-            DB[j] = dB[j] + dC[j];
-            const float gx = DA[j] + DB[j];
-            const float e0 = tC[j] - tA[j], e1 = tC[j + 1] - tA[j + 1], e2 = tC[j + 2] - tA[j + 2];
-            const float gy = __fmaf_rn(e1, 2.0f, e0) + e2;
-            r[j] = __fmaf_rn(-gx, gx, __fmaf_rn(-gy, gy, T));
+        for (int j = 0; j < 4; j++) {
+            DB.v[j] = __hadd2(dB.v[j], dC.v[j]);
+            const __half2 gx = __hadd2(DA.v[j], DB.v[j]);
+            lo4[j] = c1_sq(__low2half(gx), c1_sq(__low2half(gy[j]), T));
+            hi4[j] = c1_sq(__high2half(gx), c1_sq(__high2half(gy[j]), T));
         }
-        const uint32_t lo = __byte_perm(c1_sign_pair(r[0], r[1]), c1_sign_pair(r[2], r[3]), 0x5410);
-        const uint32_t hi = __byte_perm(c1_sign_pair(r[4], r[5]), c1_sign_pair(r[6], r[7]), 0x5410);
+        const uint32_t lo = ~__byte_perm(c1_sign_pair(lo4[0], lo4[1]), c1_sign_pair(hi4[0], hi4[1]), 0x5410);
+        const uint32_t hi = ~__byte_perm(c1_sign_pair(lo4[2], lo4[3]), c1_sign_pair(hi4[2], hi4[3]), 0x5410);
         uint8_t *o = dst + (size_t)y * dstStride + x;
         if (x < W) *(uint32_t *)o = lo;
         if (x + 4 < W) *(uint32_t *)(o + 4) = hi;
@@ -638,15 +663,15 @@ extern "C" int agocuda_fused_GaussSobelMagDepthThresh(void *stream, const agocud
 // ---- TMA-staged form
 static void c1_thresholds(int32_t shift, int32_t threshold, float &tRound, float &tTrunc)
 {
-    // T = (n_min - 1/2) * 2^-14 (exact: n_min <= 2^22); never-passing thresholds get a T
-    // above the largest gx^2 + gy^2 (2 * 1020^2 * 2^-14 < 128)
+    // T = 1/2 - n_min (exact: n_min <= 2^22); never-passing thresholds get a T below minus the
+    // largest gx^2 + gy^2 (2 * 1020^2 < 2^21)
     const int t = (int)(uint8_t)threshold;
-    tRound = tTrunc = 1024.0f;
+    tRound = tTrunc = -8388608.0f;
     if (t < 255) {
         const long long M = (long long)(t + 1) << shift;
         if (M <= 2048) {
-            tRound = (float)(((double)(M * M - M + 1) - 0.5) / 16384.0);
-            tTrunc = (float)(((double)(M * M) - 0.5) / 16384.0);
+            tRound = (float)(0.5 - (double)(M * M - M + 1));
+            tTrunc = (float)(0.5 - (double)(M * M));
         }
     }
 }

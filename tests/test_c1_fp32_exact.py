@@ -1,9 +1,9 @@
-"""The exact-fp32 Sobel / threshold arithmetic of the TMA-staged configuration-1 kernel
-(k_fused_c1_tma, mivisionx_b200/csrc/filters.cu), restated in numpy float32 step by step and
-compared with the oracle chain (Gaussian3x3 -> SobelMagnitude -> ConvertDepth(SAT) ->
+"""An exact-fp32 form of the Sobel / threshold arithmetic of the configuration-1 chain (the
+kernel itself, k_fused_c1_tma in mivisionx_b200/csrc/filters.cu, takes the differences in
+half lanes: test_c1_half_exact.py), restated in numpy float32 step by step and compared with the oracle chain (Gaussian3x3 -> SobelMagnitude -> ConvertDepth(SAT) ->
 Threshold(BINARY)) for every threshold and shift on noise and on high-contrast frames.
 
-The kernel's claim is that no step rounds: t = 6144 + G/128 is built by dropping the masked
+The claim is that no step rounds: t = 6144 + G/128 is built by dropping the masked
 16G lane into the mantissa of 6144, gx / gy are sums of differences of t, and
 r = (n_min - 1/2)/16384 - gx^2 - gy^2 is exact, so r < 0 exactly when gx^2 + gy^2 >= n_min.
 Each fused multiply-add is checked here to be exact (its float64 value is a float32)."""
