@@ -538,21 +538,10 @@ __device__ __forceinline__ void sunion(int *lab, int a, int b)
 constexpr int kInWords = (kTW + 8) / 4, kGC = kTW + 8;
 
 // One row's 6 pixels X[-1..4] around a 4-pixel word C (L, R: the words either side) as
-// 16-bit lane pairs: E = (X0, X2), O = (X1, X3), Om = (X-1, X1), Ep = (X2, X4).
-struct Lanes4 { uint32_t E, O, Om, Ep; };
-__device__ __forceinline__ Lanes4 lanes4(uint32_t L, uint32_t C, uint32_t R)
-{
-    Lanes4 v;
-    v.E = __byte_perm(C, 0, 0x4240);
-    v.O = __byte_perm(C, 0, 0x4341);
-    v.Om = __byte_perm(L, v.O, 0x5453);
-    v.Ep = __byte_perm(v.E, R, 0x3432);
-    return v;
-}
-
-// The same lanes as halves 1024 + v (bits 0x6400 | v): differences of two such lanes, and sums
-// of differences up to 2048, are exact, so Sobel sums and |gx| + |gy| run two pixels per
-// instruction on the FMA pipe (the front's integer form kept the ALU pipe 75 % busy).
+// lane pairs: E = (X0, X2), O = (X1, X3), Om = (X-1, X1), Ep = (X2, X4).  The lanes are halves
+// 1024 + v (bits 0x6400 | v): differences of two such lanes, and sums of differences up to 2048,
+// are exact, so Sobel sums and |gx| + |gy| run two pixels per instruction on the FMA pipe (in
+// integer lanes the Canny front kept the ALU pipe 75 % busy).
 struct HalfLanes4 { __half2 E, O, Om, Ep; };
 __device__ __forceinline__ HalfLanes4 half_lanes4(uint32_t L, uint32_t C, uint32_t R)
 {
@@ -1091,11 +1080,12 @@ __global__ void k_harris_nms(int W, int H, const float *sc, int scStride, uint64
 // Harris front end as column strips: a warp owns 120 output columns (lanes 1..30, four
 // columns each; lanes 0 and 31 carry the halo) and walks down `rows` output rows with rolling
 // registers (64 where the frames in flight fill the device with such strips, fewer where they
-// do not: harris_rows).  Per input row a lane loads one word; the Sobel sums run in 16-bit lanes
-// (four columns in four registers), the products and window sums in float -- integers
-// below 2^24, i.e. exactly the float sums the reference forms in any order.  The score
-// keeps the reference's float operation order, and its division is skipped only where the
-// result cannot exceed the threshold.
+// do not: harris_rows).  Per input row a lane loads one word; the Sobel sums run in half lanes
+// (four columns in four registers, integers up to 1020), the products, straight from halves, and
+// the window sums in float -- integers below 2^24, i.e. exactly the float sums the reference
+// forms in any order.  The score keeps the reference's float operation order; its division is
+// skipped only where the result cannot exceed the threshold, and the suppression of a row of
+// zero scores altogether.  The bound is instruction issue.
 constexpr int kHRows = 64, kHCols = 120;
 
 __device__ __forceinline__ uint32_t harris_word(const uint8_t *src, int stride, int W, int H, int x, int y, bool fast)
@@ -1105,10 +1095,6 @@ __device__ __forceinline__ uint32_t harris_word(const uint8_t *src, int stride, 
     for (int k = 0; k < 4; k++) w |= (uint32_t)ago_px(src, stride, W, H, x + k, y) << (8 * k);
     return w;
 }
-
-// biased 16-bit lane (value + 1024) as an exact float
-__device__ __forceinline__ float lane_lo(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7610)) - 8389632.0f; }
-__device__ __forceinline__ float lane_hi(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7632)) - 8389632.0f; }
 
 // TMA form: each warp copies its source rows ys-3 .. ys+rows+2, columns from (xs-4) rounded
 // down to 16 bytes, 144 bytes wide, into shared memory with one tensor copy on its own
@@ -1168,112 +1154,135 @@ k_harris_rows(int W, int H, int rows, const uint8_t *__restrict__ src, int srcSt
         else return harris_word(src, srcStride, W, H, xl, y, fast);
     };
     const bool outLane = lane >= 1 && lane <= 30;
-    bool gradCol[4], scoreCol[4];
+    // columns (0, 2) and (1, 3) that have a gradient as lane masks; columns that have a score as bits
+    uint32_t grad02 = 0, grad13 = 0, scoreCol = 0;
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-        gradCol[c] = xl + c >= 0 && xl + c < W;
-        scoreCol[c] = xl + c >= 1 && xl + c < W - 1;
+        const uint32_t m = xl + c >= 0 && xl + c < W ? 0xffffu << (c & 2 ? 16 : 0) : 0u;
+        if (c & 1) grad13 |= m; else grad02 |= m;
+        if (xl + c >= 1 && xl + c < W - 1) scoreCol |= 1u << c;
     }
-    // the score is 0 without the division where Mc < zLess or Mc <= zLessEq:
-    // Tc > 0: Mc < 0.999 Tc norm (the quotient cannot exceed Tc); Tc == 0: Mc <= 0
-    const float cut = Tc > 0.f ? __fmul_rn(0.999f, __fmul_rn(Tc, norm)) : 0.f;
-    const float zLess = Tc > 0.f ? cut : -INFINITY, zLessEq = Tc == 0.f ? 0.f : -INFINITY;
-    // rolling state, rotated by the unrolled loop: input rows as 16-bit lanes, products of
-    // gradient rows, scores (columns -1 .. 4) of score rows
-    Lanes4 X[3] = {};
+    // the score is 0 without the division unless Mc >= least:
+    // Tc > 0: 0.999 Tc norm (below it the quotient cannot exceed Tc); Tc == 0: anything above 0
+    const float least = Tc > 0.f ? __fmul_rn(0.999f, __fmul_rn(Tc, norm)) : Tc == 0.f ? __uint_as_float(1u) : -INFINITY;
+    // rolling state, rotated by the unrolled loop: input rows as half lanes with their horizontal
+    // differences, products of gradient rows, scores (columns -1 .. 4) of score rows
+    struct Row { HalfLanes4 v; __half2 d02, d13; };
+    Row X[3] = {};
     float P[3][3][4] = {};
     float S[3][6] = {};
+    bool some[3] = {};                                     // a score row of the warp holds a non-zero score
     uint32_t next = word(ys - 3);
     const int rLast = yEnd + 2;
+    const __half2 two = __float2half2_rn(2.f);
+    auto masked = [](__half2 v, uint32_t m) {
+        const uint32_t w = *(const uint32_t *)&v & m;
+        return *(const __half2 *)&w;
+    };
+    // a * b of halves, exact in fp32
+    auto product = [](__half a, __half b) {
+        float r;
+        asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(r) : "h"(__half_as_ushort(a)), "h"(__half_as_ushort(b)), "f"(0.f));
+        return r;
+    };
 
     // one input row r: t, m = rows r-2, r-1 (b receives row r); v0, v1 = products at
     // gradient rows g-2, g-1 (p receives g = r-1); sA, sB = scores at rows s-2, s-1 (sc
     // receives s = g-1); suppression at n = s-1
-    auto step = [&](int r, const Lanes4 &t, const Lanes4 &m, Lanes4 &b, const float (&v0)[3][4],
+    auto step = [&](int r, const Row &t, const Row &m, Row &b, const float (&v0)[3][4],
                     const float (&v1)[3][4], float (&p)[3][4], const float (&sA)[6], const float (&sB)[6],
-                    float (&sc)[6]) {
+                    float (&sc)[6], bool someB, bool &someC) {
         const uint32_t cur = next;
         if (r + 1 <= rLast) next = word(r + 1);
-        b = lanes4(__shfl_up_sync(0xffffffffu, cur, 1), cur, __shfl_down_sync(0xffffffffu, cur, 1));
+        b.v = half_lanes4(__shfl_up_sync(0xffffffffu, cur, 1), cur, __shfl_down_sync(0xffffffffu, cur, 1));
+        b.d02 = __hsub2(b.v.O, b.v.Om);
+        b.d13 = __hsub2(b.v.Ep, b.v.E);
         // gradient at g = r - 1 (HafCpu_HarrisSobel_HG3_U8_3x3, harris.cpp:85)
         const int g = r - 1;
         {
-            const uint32_t bias = 0x04000400u;
-            const uint32_t vE = t.E + 2 * m.E + b.E, vO = t.O + 2 * m.O + b.O;
-            const uint32_t vOm = t.Om + 2 * m.Om + b.Om, vEp = t.Ep + 2 * m.Ep + b.Ep;
-            const uint32_t gx02 = vO + bias - vOm, gx13 = vEp + bias - vE;
-            const uint32_t gy02 = (b.Om + 2 * b.E + b.O) + bias - (t.Om + 2 * t.E + t.O);
-            const uint32_t gy13 = (b.E + 2 * b.O + b.Ep) + bias - (t.E + 2 * t.O + t.Ep);
-            const float gx[4] = {lane_lo(gx02), lane_lo(gx13), lane_hi(gx02), lane_hi(gx13)};
-            const float gy[4] = {lane_lo(gy02), lane_lo(gy13), lane_hi(gy02), lane_hi(gy13)};
             const bool rowOk = g >= 1 && g < H - 1;
+            const uint32_t k02 = rowOk ? grad02 : 0u, k13 = rowOk ? grad13 : 0u;
+            const __half2 dOm = __hsub2(b.v.Om, t.v.Om), dE = __hsub2(b.v.E, t.v.E);
+            const __half2 dO = __hsub2(b.v.O, t.v.O), dEp = __hsub2(b.v.Ep, t.v.Ep);
+            const __half2 gx02 = masked(__hfma2(two, m.d02, __hadd2(t.d02, b.d02)), k02);
+            const __half2 gx13 = masked(__hfma2(two, m.d13, __hadd2(t.d13, b.d13)), k13);
+            const __half2 gy02 = masked(__hfma2(two, dE, __hadd2(dOm, dO)), k02);
+            const __half2 gy13 = masked(__hfma2(two, dO, __hadd2(dE, dEp)), k13);
+            const __half gx[4] = {__low2half(gx02), __low2half(gx13), __high2half(gx02), __high2half(gx13)};
+            const __half gy[4] = {__low2half(gy02), __low2half(gy13), __high2half(gy02), __high2half(gy13)};
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                const bool ok = rowOk && gradCol[c];
-                p[0][c] = ok ? __fmul_rn(gx[c], gx[c]) : 0.f;
-                p[1][c] = ok ? __fmul_rn(gx[c], gy[c]) : 0.f;
-                p[2][c] = ok ? __fmul_rn(gy[c], gy[c]) : 0.f;
+                p[0][c] = product(gx[c], gx[c]);
+                p[1][c] = product(gx[c], gy[c]);
+                p[2][c] = product(gy[c], gy[c]);
             }
         }
         // window sums at s = g - 1 over gradient rows g-2 .. g (HafCpu_HarrisScore_HVC_HG3_3x3)
-        float vs[3][6];
+        float sum[3][4];
 #pragma unroll
         for (int q = 0; q < 3; q++) {
+            float vs[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) vs[q][c + 1] = __fadd_rn(__fadd_rn(v0[q][c], v1[q][c]), p[q][c]);
-            vs[q][0] = __shfl_up_sync(0xffffffffu, vs[q][4], 1);
-            vs[q][5] = __shfl_down_sync(0xffffffffu, vs[q][1], 1);
+            for (int c = 0; c < 4; c++) vs[c] = __fadd_rn(__fadd_rn(v0[q][c], v1[q][c]), p[q][c]);
+            const float vl = __shfl_up_sync(0xffffffffu, vs[3], 1), vr = __shfl_down_sync(0xffffffffu, vs[0], 1);
+            const float mid0 = __fadd_rn(vs[0], vs[1]), mid1 = __fadd_rn(vs[2], vs[3]);
+            sum[q][0] = __fadd_rn(vl, mid0);
+            sum[q][1] = __fadd_rn(mid0, vs[2]);
+            sum[q][2] = __fadd_rn(vs[1], mid1);
+            sum[q][3] = __fadd_rn(mid1, vr);
         }
         const int srow = g - 1;
-        const bool sRowOk = srow >= 1 && srow < H - 1;
+        const uint32_t scoreNow = srow >= 1 && srow < H - 1 ? scoreCol : 0u;
+        bool nonzero = false;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            const float gx2 = __fadd_rn(__fadd_rn(vs[0][c], vs[0][c + 1]), vs[0][c + 2]);
-            const float gxy2 = __fadd_rn(__fadd_rn(vs[1][c], vs[1][c + 1]), vs[1][c + 2]);
-            const float gy2 = __fadd_rn(__fadd_rn(vs[2][c], vs[2][c + 1]), vs[2][c + 2]);
+            const float gx2 = sum[0][c], gxy2 = sum[1][c], gy2 = sum[2][c];
             const float traceA = __fadd_rn(gx2, gy2);
             const float detA = __fsub_rn(__fmul_rn(gx2, gy2), __fmul_rn(gxy2, gxy2));
             const float Mc = __fsub_rn(detA, __fmul_rn(__fmul_rn(k, traceA), traceA));
             float v = 0.f;
-            if (sRowOk && scoreCol[c] && !(Mc < zLess || Mc <= zLessEq)) {
+            if (Mc >= least && ((scoreNow >> c) & 1)) {
                 const float q = __fdiv_rn(Mc, norm);
                 v = q > Tc ? q : 0.f;
+                nonzero |= v != 0.f;
             }
             sc[c + 1] = v;
         }
-        sc[0] = __shfl_up_sync(0xffffffffu, sc[4], 1);
-        sc[5] = __shfl_down_sync(0xffffffffu, sc[1], 1);
-        // non-maximum suppression at n = s - 1 (HafCpu_NonMaxSupp_XY_ANY_3x3, harris.cpp:882):
-        // >= the row above and the left neighbour, > the right neighbour and the row below
-        const int n = srow - 1;
-        const bool rowOut = n >= ys && n < yEnd && n >= 1 && n < H - 1;
-        uint32_t keep = 0;
-        if (outLane && rowOut) {
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const float v = sB[c + 1];
-                const float above = fmaxf(fmaxf(sA[c], sA[c + 1]), sA[c + 2]);
-                const float below = fmaxf(fmaxf(sc[c], sc[c + 1]), sc[c + 2]);
-                const bool kc = scoreCol[c] && v >= above && v >= sB[c] && v > sB[c + 2] && v > below;
-                keep |= (uint32_t)kc << c;
-            }
+        someC = __any_sync(0xffffffffu, nonzero);
+        sc[0] = sc[5] = 0.f;
+        if (someC) {
+            sc[0] = __shfl_up_sync(0xffffffffu, sc[4], 1);
+            sc[5] = __shfl_down_sync(0xffffffffu, sc[1], 1);
         }
-        if (rowOut && __any_sync(0xffffffffu, keep != 0)) {
+        // non-maximum suppression at n = s - 1 (HafCpu_NonMaxSupp_XY_ANY_3x3, harris.cpp:882):
+        // >= the row above and the left neighbour, > the right neighbour and the row below.  In a
+        // row of zeros no score is above its right neighbour.
+        const int n = srow - 1;
+        if (!someB || !(n >= ys && n < yEnd && n >= 1 && n < H - 1)) return;
+        uint32_t keep = 0;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const float v = sB[c + 1];
+            const float before = fmaxf(fmaxf(fmaxf(sA[c], sA[c + 1]), sA[c + 2]), sB[c]);
+            const float after = fmaxf(fmaxf(fmaxf(sc[c], sc[c + 1]), sc[c + 2]), sB[c + 2]);
+            if (v >= before && v > after) keep |= 1u << c;
+        }
+        keep = outLane ? keep & scoreCol : 0u;
+        if (__any_sync(0xffffffffu, keep != 0)) {
 #pragma unroll
             for (int c = 0; c < 4; c++)
                 xys_append(list, count, capacity, xys_pack(xl + c, n, sB[c + 1]), (keep >> c) & 1);
         }
     };
     for (int r = ys - 3; r <= rLast; r += 3) {             // r is warp-uniform
-        step(r, X[0], X[1], X[2], P[0], P[1], P[2], S[0], S[1], S[2]);
+        step(r, X[0], X[1], X[2], P[0], P[1], P[2], S[0], S[1], S[2], some[1], some[2]);
         if (r + 1 > rLast) break;
-        step(r + 1, X[1], X[2], X[0], P[1], P[2], P[0], S[1], S[2], S[0]);
+        step(r + 1, X[1], X[2], X[0], P[1], P[2], P[0], S[1], S[2], S[0], some[2], some[0]);
         if (r + 2 > rLast) break;
-        step(r + 2, X[2], X[0], X[1], P[2], P[0], P[1], S[2], S[0], S[1]);
+        step(r + 2, X[2], X[0], X[1], P[2], P[0], P[1], S[2], S[0], S[1], some[0], some[1]);
     }
 }
 
-// ---------------------------------------------------------------------------------
 // Corner pick (HafCpu_HarrisMergeSortAndPick_XY_XYS, harris.cpp:923).  Reference: sort the
 // candidates descending as int64, then walk them in order keeping a point when its grid cell
 // is empty and no kept point in the 5x5 cells around is closer than min_dist2.  That is the
