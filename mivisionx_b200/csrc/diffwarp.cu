@@ -21,18 +21,27 @@ uint64_t agocuda_count_launch(unsigned n);
 
 namespace {
 
-struct Taps {
-    int x0, y0;
+// One sample: the fractions, the four taps, and in `key` the element index of the first tap where
+// all four lie inside a source of fewer than 2^31 elements (`wide` is false), else kNoKey.
+constexpr int kNoKey = INT_MIN;
+struct Sample {
+    int key;
     float fx, fy;
     float p00, p01, p10, p11;
+};
+
+// Where the taps of a sample lie that has no key: each on its own inside the source or not
+struct Place {
+    int x0, y0;
+    float fx, fy;
     bool k00, k01, k10, k11;
 };
 
 // Positions are formed in double: a float position near x = 1000 is only good to ~6e-5 px,
 // and the theta gradient is a strongly cancelling sum over every pixel.
-__device__ __forceinline__ Taps taps(const float *src, int stride, int W, int H, double xs, double ys, float border)
+__device__ __forceinline__ Place place(int W, int H, double xs, double ys)
 {
-    Taps t;
+    Place t;
     const double fx0 = floor(xs), fy0 = floor(ys);
     t.fx = (float)(xs - fx0);
     t.fy = (float)(ys - fy0);
@@ -44,10 +53,6 @@ __device__ __forceinline__ Taps taps(const float *src, int stride, int W, int H,
     const int x1 = t.x0 + 1, y1 = t.y0 + 1;
     const bool cx0 = t.x0 >= 0 && t.x0 < W, cx1 = x1 >= 0 && x1 < W, cy0 = t.y0 >= 0 && t.y0 < H, cy1 = y1 >= 0 && y1 < H;
     t.k00 = cx0 && cy0; t.k01 = cx1 && cy0; t.k10 = cx0 && cy1; t.k11 = cx1 && cy1;
-    t.p00 = t.k00 ? __ldg(src + (size_t)t.y0 * stride + t.x0) : border;
-    t.p01 = t.k01 ? __ldg(src + (size_t)t.y0 * stride + x1) : border;
-    t.p10 = t.k10 ? __ldg(src + (size_t)y1 * stride + t.x0) : border;
-    t.p11 = t.k11 ? __ldg(src + (size_t)y1 * stride + x1) : border;
     return t;
 }
 
@@ -64,25 +69,26 @@ __device__ __forceinline__ bool floor_inside(double v, int n, int &i, float &f)
     return __double2hiint(t) == 0x43380000 && (unsigned)i < (unsigned)(n - 1);
 }
 
-// One sample: the taps, and in `key` the element index of the first tap where all four lie
-// inside a source of fewer than 2^31 elements (`wide` is false), else kNoKey with the tap
-// flags in t.
-constexpr int kNoKey = INT_MIN;
-struct Sample { Taps t; int key; };
-
 __device__ __forceinline__ Sample sample(const float *src, int stride, int W, int H, double xs, double ys, float border,
                                          bool wide)
 {
     Sample s;
-    const bool inx = floor_inside(xs, W, s.t.x0, s.t.fx), iny = floor_inside(ys, H, s.t.y0, s.t.fy);
+    int x0, y0;
+    const bool inx = floor_inside(xs, W, x0, s.fx), iny = floor_inside(ys, H, y0, s.fy);
     if (inx && iny && !wide) {
-        s.key = s.t.y0 * stride + s.t.x0;
+        s.key = y0 * stride + x0;
         const float *p = src + s.key;
-        s.t.p00 = __ldg(p); s.t.p01 = __ldg(p + 1);
-        s.t.p10 = __ldg(p + stride); s.t.p11 = __ldg(p + stride + 1);
-        s.t.k00 = s.t.k01 = s.t.k10 = s.t.k11 = true;
+        s.p00 = __ldg(p); s.p01 = __ldg(p + 1);
+        s.p10 = __ldg(p + stride); s.p11 = __ldg(p + stride + 1);
     } else {
-        s.t = taps(src, stride, W, H, xs, ys, border);
+        const Place t = place(W, H, xs, ys);
+        const float *p = src + (long long)t.y0 * stride + t.x0;
+        s.p00 = t.k00 ? __ldg(p) : border;
+        s.p01 = t.k01 ? __ldg(p + 1) : border;
+        s.p10 = t.k10 ? __ldg(p + stride) : border;
+        s.p11 = t.k11 ? __ldg(p + stride + 1) : border;
+        s.fx = t.fx;
+        s.fy = t.fy;
         s.key = kNoKey;
     }
     return s;
@@ -98,14 +104,15 @@ struct Scatter {
     int key = kNoKey;          // address of the contributions kept from the row above
     float v0 = 0.f, v1 = 0.f;
 
-    // all lanes of the warp take part; a lane without a sample passes key kNoKey and g 0
-    __device__ __forceinline__ void row(float *gsrc, int stride, const Sample &s, float g, bool has)
+    // all lanes of the warp take part; a lane without a sample passes key kNoKey and g 0.  where()
+    // is the Place of a sample without a key, which few have: it is found again, not carried.
+    template <class WHERE>
+    __device__ __forceinline__ void row(float *gsrc, int stride, const Sample &t, float g, bool has, WHERE where)
     {
-        const Taps &t = s.t;
         const float gu = g * (1.f - t.fx), gr = g * t.fx;
         float c00 = gu * (1.f - t.fy), c01 = gr * (1.f - t.fy);
         const float c10 = gu * t.fy, c11 = gr * t.fy;
-        const int k = s.key;
+        const int k = t.key;
         if (key != kNoKey) {
             if (key == k) {
                 c00 += v0;
@@ -127,11 +134,12 @@ struct Scatter {
             v0 = c10;
             v1 = c11;
         } else if (has) {
-            float *p = gsrc + (long long)t.y0 * stride + t.x0;
-            if (t.k00) atomicAdd(p, c00);
-            if (t.k01) atomicAdd(p + 1, c01);
-            if (t.k10) atomicAdd(p + stride, c10);
-            if (t.k11) atomicAdd(p + stride + 1, c11);
+            const Place w = where();
+            float *p = gsrc + (long long)w.y0 * stride + w.x0;
+            if (w.k00) atomicAdd(p, c00);
+            if (w.k01) atomicAdd(p + 1, c01);
+            if (w.k10) atomicAdd(p + stride, c10);
+            if (w.k11) atomicAdd(p + stride + 1, c11);
         }
     }
     __device__ __forceinline__ void flush(float *gsrc)
@@ -145,13 +153,11 @@ struct Scatter {
     }
 };
 
-__device__ __forceinline__ float interp(const Taps &t)
-{
-    return (t.p00 * (1.f - t.fx) + t.p01 * t.fx) * (1.f - t.fy) + (t.p10 * (1.f - t.fx) + t.p11 * t.fx) * t.fy;
-}
-
-__device__ __forceinline__ float dout_dxs(const Taps &t) { return (1.f - t.fy) * (t.p01 - t.p00) + t.fy * (t.p11 - t.p10); }
-__device__ __forceinline__ float dout_dys(const Taps &t) { return (1.f - t.fx) * (t.p10 - t.p00) + t.fx * (t.p11 - t.p01); }
+// a (1 - f) + b f
+__device__ __forceinline__ float mix(float a, float b, float f) { return __fmaf_rn(b, f, a * (1.f - f)); }
+__device__ __forceinline__ float interp(const Sample &t) { return mix(mix(t.p00, t.p01, t.fx), mix(t.p10, t.p11, t.fx), t.fy); }
+__device__ __forceinline__ float dout_dxs(const Sample &t) { return mix(t.p01 - t.p00, t.p11 - t.p10, t.fy); }
+__device__ __forceinline__ float dout_dys(const Sample &t) { return mix(t.p10 - t.p00, t.p11 - t.p01, t.fx); }
 
 // block reduction of N per-thread double sums into double atomics at dst[0..N)
 template <int N>
@@ -191,9 +197,11 @@ enum Mode { kForward = 0, kAdjoint = 1, kFusedL2 = 2 };
 // row loaded while a row is worked on.  Per pixel a thread adds 2 (affine) or 6 terms to
 // double sums of its own; x is fixed per thread, so sum(g x) is x sum(g), and the sums meet
 // across lanes once per strip instead of once per pixel (7 double butterflies per pixel were
-// the larger half of the fused step).  Affine L2 step of 32 x 1024^2: 573 us with one pixel per
-// thread, 278 us so; issue-bound (77 % of the issue slots).  `rows` is 16 where the batch fills the device with
-// such strips and less where it does not (warp_rows).
+// the larger half of the fused step).  Products with y are fused into their sums, and a sample
+// carries no place of its own, only a key.  Affine L2 step of 32 x 1024^2: 573 us with one pixel
+// per thread, 264 us so; issue-bound, and larger bodies (two rows unrolled) are slower, 338 us.
+// `rows` is 32 where the batch fills the device with such strips and less where it does not
+// (warp_rows): 16 rows, with twice as many sums across lanes, took 267 us.
 template <int MODE, int NT>
 __global__ void __launch_bounds__(256)
 k_warp_f32(int W, int H, int rows, Img32 src, Img32 out, Img32 aux, const float *par, long long parBatch, int parStride,
@@ -220,14 +228,15 @@ k_warp_f32(int W, int H, int rows, Img32 src, Img32 out, Img32 aux, const float 
         }
     }
     struct Pos { double xs, ys, iz; };
-    auto position = [&](int y) -> Pos {
+    // yd = y; the sums my y + mx round once, like the sum of the exact product and mx
+    auto position = [&](int y, double yd) -> Pos {
         if (NT == 2) {
             const float2 d = act ? field[(size_t)y * parStride + x] : make_float2(0.f, 0.f);
             return {(double)x + d.x, (double)y + d.y, 1.0};
         }
-        const double xn = mx[0] + my[0] * y + m0[0], yn = mx[1] + my[1] * y + m0[1];
+        const double xn = __fma_rn(my[0], yd, mx[0]) + m0[0], yn = __fma_rn(my[1], yd, mx[1]) + m0[1];
         if (NT == 6) return {xn, yn, 1.0};
-        const double z = mx[2] + my[2] * y + m0[2];
+        const double z = __fma_rn(my[2], yd, mx[2]) + m0[2];
         if (z == 0.0) { const double nan = __longlong_as_double(0x7ff8000000000000ll); return {nan, nan, 0.0}; }
         const double iz = 1.0 / z;
         return {xn * iz, yn * iz, iz};
@@ -236,11 +245,12 @@ k_warp_f32(int W, int H, int rows, Img32 src, Img32 out, Img32 aux, const float 
         if (!act) return;
         float *o = out.p + out.batch * n + x;
         for (int y = yA; y < yB; y += 2) {                 // two rows at a time: their loads overlap
-            const Pos p = position(y), q = position(min(y + 1, yB - 1));
+            const int y1 = min(y + 1, yB - 1);
+            const Pos p = position(y, y), q = position(y1, y1);
             const Sample a = sample(sp, src.stride, src.W, src.H, p.xs, p.ys, border, wide);
             const Sample b = sample(sp, src.stride, src.W, src.H, q.xs, q.ys, border, wide);
-            o[(size_t)y * out.stride] = interp(a.t);
-            if (y + 1 < yB) o[(size_t)(y + 1) * out.stride] = interp(b.t);
+            o[(size_t)y * out.stride] = interp(a);
+            if (y + 1 < yB) o[(size_t)(y + 1) * out.stride] = interp(b);
         }
         return;
     }
@@ -248,9 +258,9 @@ k_warp_f32(int W, int H, int rows, Img32 src, Img32 out, Img32 aux, const float 
     double sum[NS] = {};
     Scatter sc;
     const float *ap = aux.p + aux.batch * n + x;
-    auto load = [&](int y, Pos &p, Sample &s, float &a) {
+    auto load = [&](int y, double yd, Pos &p, Sample &s, float &a) {
         if (act && y < yB) {
-            p = position(y);
+            p = position(y, yd);
             a = __ldg(ap + (size_t)y * aux.stride);
             s = sample(sp, src.stride, src.W, src.H, p.xs, p.ys, border, wide);
         } else {
@@ -262,37 +272,41 @@ k_warp_f32(int W, int H, int rows, Img32 src, Img32 out, Img32 aux, const float 
     Pos p, pn;
     Sample s, sn;
     float a, an;
-    load(yA, p, s, a);
+    double yd = yA;
+    load(yA, yd, p, s, a);
     for (int y = yA; y < yB; y++) {
-        load(y + 1, pn, sn, an);
-        const Taps &t = s.t;
+        const double yn = yd + 1.0;
+        load(y + 1, yn, pn, sn, an);
         float g = a;
         if (MODE == kFusedL2) {
-            const float r = act ? interp(t) - a : 0.f;
-            sum[NS - 1] += (double)r * r;
+            const float r = act ? interp(s) - a : 0.f;
+            sum[NS - 1] = __fma_rn((double)r, (double)r, sum[NS - 1]);
             g = 2.f * r;
         }
-        sc.row(gp, gsrc.stride, s, g, act);
-        const float gx = g * dout_dxs(t), gy = g * dout_dys(t);
+        sc.row(gp, gsrc.stride, s, g, act, [&]() {
+            const Pos q = position(y, yd);
+            return place(src.W, src.H, q.xs, q.ys);
+        });
+        const float gx = g * dout_dxs(s), gy = g * dout_dys(s);
         if (NT == 2) {
             if (act) gfield[(size_t)y * parStride + x] = make_float2(gx, gy);
         } else if (NT == 6) {
             const double dx = gx, dy = gy;
             sum[4 % NS] += dx;
             sum[5 % NS] += dy;
-            sum[2 % NS] += dx * y;
-            sum[3 % NS] += dy * y;
+            sum[2 % NS] = __fma_rn(dx, yd, sum[2 % NS]);
+            sum[3 % NS] = __fma_rn(dy, yd, sum[3 % NS]);
         } else if (act && p.iz != 0.0 && (gx != 0.f || gy != 0.f)) {   // a sample on the border has no theta term
             // d(xs)/d(m00, m10, m20) = (x, y, 1) / z; d(xs)/d(m02, m12, m22) = -xs (x, y, 1) / z; same for ys
             const double gxz = gx * p.iz, gyz = gy * p.iz, q = -((double)gx * p.xs + (double)gy * p.ys) * p.iz;
             sum[6 % NS] += gxz;
             sum[7 % NS] += gyz;
             sum[8 % NS] += q;
-            sum[3 % NS] += gxz * y;
-            sum[4 % NS] += gyz * y;
-            sum[5 % NS] += q * y;
+            sum[3 % NS] = __fma_rn(gxz, yd, sum[3 % NS]);
+            sum[4 % NS] = __fma_rn(gyz, yd, sum[4 % NS]);
+            sum[5 % NS] = __fma_rn(q, yd, sum[5 % NS]);
         }
-        p = pn; s = sn; a = an;
+        p = pn; s = sn; a = an; yd = yn;
     }
     sc.flush(gp);
     if constexpr (NT != 2) {
@@ -349,7 +363,7 @@ extern "C" int agocuda_WarpAffine_F32_Bilinear_Constant_adjoint_batch(void *stre
     if (!pGradOut || !pSrc || !theta || !pGradSrc || !pGradTheta || !batch_ok(n, W, H, srcW, srcH) || goStride < W ||
         srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const int rows = warp_rows(n, W, H, 16);
+    const int rows = warp_rows(n, W, H, 32);
     k_warp_f32<kAdjoint, 6><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
         W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pGradOut, goBatch, goStride, W, H), theta, 0, 0,
         border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradTheta);
@@ -365,7 +379,7 @@ extern "C" int agocuda_WarpAffine_F32_L2_step_batch(void *stream, int n, int W, 
     if (!pTarget || !pSrc || !theta || !pGradSrc || !pGradThetaLoss || !batch_ok(n, W, H, srcW, srcH) || tStride < W ||
         srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const int rows = warp_rows(n, W, H, 16);
+    const int rows = warp_rows(n, W, H, 32);
     k_warp_f32<kFusedL2, 6><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
         W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pTarget, tBatch, tStride, W, H), theta, 0, 0,
         border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradThetaLoss);
@@ -398,7 +412,7 @@ extern "C" int agocuda_Remap_F32_Bilinear_Constant_adjoint_batch(void *stream, i
     if (!pGradOut || !pSrc || !pField || !pGradSrc || !pGradField || !batch_ok(n, W, H, srcW, srcH) || goStride < W ||
         srcStride < srcW || fieldStride < W || ((uintptr_t)pField & 7) || ((uintptr_t)pGradField & 7))
         return AGOCUDA_INVALID_PARAMS;
-    const int rows = warp_rows(n, W, H, 16);
+    const int rows = warp_rows(n, W, H, 32);
     k_warp_f32<kAdjoint, 2><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
         W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pGradOut, goBatch, goStride, W, H),
         pField, fieldBatch, fieldStride, border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradField);
@@ -431,7 +445,7 @@ extern "C" int agocuda_WarpPerspective_F32_Bilinear_Constant_adjoint_batch(void 
     if (!pGradOut || !pSrc || !theta || !pGradSrc || !pGradTheta || !batch_ok(n, W, H, srcW, srcH) || goStride < W ||
         srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const int rows = warp_rows(n, W, H, 16);
+    const int rows = warp_rows(n, W, H, 32);
     k_warp_f32<kAdjoint, 9><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
         W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pGradOut, goBatch, goStride, W, H), theta, 0, 0,
         border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradTheta);
@@ -447,7 +461,7 @@ extern "C" int agocuda_WarpPerspective_F32_L2_step_batch(void *stream, int n, in
     if (!pTarget || !pSrc || !theta || !pGradSrc || !pGradThetaLoss || !batch_ok(n, W, H, srcW, srcH) || tStride < W ||
         srcStride < srcW)
         return AGOCUDA_INVALID_PARAMS;
-    const int rows = warp_rows(n, W, H, 16);
+    const int rows = warp_rows(n, W, H, 32);
     k_warp_f32<kFusedL2, 9><<<warp_grid(n, W, H, rows), 256, 0, as_stream(stream)>>>(
         W, H, rows, img32(pSrc, srcBatch, srcStride, srcW, srcH), Img32{}, img32(pTarget, tBatch, tStride, W, H), theta, 0, 0,
         border, img32(pGradSrc, srcBatch, srcStride, srcW, srcH), pGradThetaLoss);
