@@ -137,3 +137,13 @@ __device__ __forceinline__ uint32_t ago_byte(const uint8_t *img, size_t stride, 
     const int rr = (int)(f / S), cc = (int)(f - rr * S);
     return cc < W ? img[(size_t)rr * stride + cc] : 0;
 }
+
+// Two float operations in one instruction.  A packed product that feeds a packed sum comes out
+// contracted, explicit rounding or not, so a product that has to round by itself is a fused
+// multiply-add with a zero the compiler does not see (a kernel argument).
+struct F2 { unsigned long long w; };
+__device__ __forceinline__ F2 f2(float a, float b) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.w) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.w) : "l"(a.w), "l"(b.w)); return r; }
+__device__ __forceinline__ F2 f2_add_rz(F2 a, F2 b) { F2 r; asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r.w) : "l"(a.w), "l"(b.w)); return r; }
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.w) : "l"(a.w), "l"(b.w), "l"(c.w)); return r; }
+__device__ __forceinline__ void f2_bits(F2 a, uint32_t (&v)[2]) { asm("mov.b64 {%0, %1}, %2;" : "=r"(v[0]), "=r"(v[1]) : "l"(a.w)); }
