@@ -147,3 +147,5 @@ __device__ __forceinline__ F2 f2_add(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %
 __device__ __forceinline__ F2 f2_add_rz(F2 a, F2 b) { F2 r; asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r.w) : "l"(a.w), "l"(b.w)); return r; }
 __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.w) : "l"(a.w), "l"(b.w), "l"(c.w)); return r; }
 __device__ __forceinline__ void f2_bits(F2 a, uint32_t (&v)[2]) { asm("mov.b64 {%0, %1}, %2;" : "=r"(v[0]), "=r"(v[1]) : "l"(a.w)); }
+__device__ __forceinline__ float f2_lo(F2 a) { return __uint_as_float((uint32_t)a.w); }
+__device__ __forceinline__ float f2_hi(F2 a) { return __uint_as_float((uint32_t)(a.w >> 32)); }

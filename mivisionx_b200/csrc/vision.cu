@@ -1105,7 +1105,7 @@ constexpr int kHBoxSlot = (kHBoxH * kHBoxW + 127) & ~127;   // a TMA destination
 template <bool TMA>
 __global__ void __launch_bounds__(128)
 k_harris_rows(int W, int H, int rows, const uint8_t *__restrict__ src, int srcStride, float k, float Tc, float norm,
-              uint64_t *list, uint32_t *count, uint32_t capacity, uint32_t *pStatus, const __grid_constant__ CUtensorMap map)
+              uint64_t *list, uint32_t *count, uint32_t capacity, uint32_t *pStatus, float zero, const __grid_constant__ CUtensorMap map)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int xs = (blockIdx.x * (blockDim.x >> 5) + wib) * kHCols;
@@ -1169,7 +1169,7 @@ k_harris_rows(int W, int H, int rows, const uint8_t *__restrict__ src, int srcSt
     // differences, products of gradient rows, scores (columns -1 .. 4) of score rows
     struct Row { HalfLanes4 v; __half2 d02, d13; };
     Row X[3] = {};
-    float P[3][3][4] = {};
+    F2 P[3][3][2] = {};                                    // columns (0, 2) and (1, 3)
     float S[3][6] = {};
     bool some[3] = {};                                     // a score row of the warp holds a non-zero score
     uint32_t next = word(ys - 3);
@@ -1185,12 +1185,16 @@ k_harris_rows(int W, int H, int rows, const uint8_t *__restrict__ src, int srcSt
         asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(r) : "h"(__half_as_ushort(a)), "h"(__half_as_ushort(b)), "f"(0.f));
         return r;
     };
+    auto products = [&](__half2 a, __half2 b) {
+        return f2(product(__low2half(a), __low2half(b)), product(__high2half(a), __high2half(b)));
+    };
+    const F2 zero2 = f2(zero, zero), minus = f2(-1.f, -1.f), k2 = f2(k, k);
 
     // one input row r: t, m = rows r-2, r-1 (b receives row r); v0, v1 = products at
     // gradient rows g-2, g-1 (p receives g = r-1); sA, sB = scores at rows s-2, s-1 (sc
     // receives s = g-1); suppression at n = s-1
-    auto step = [&](int r, const Row &t, const Row &m, Row &b, const float (&v0)[3][4],
-                    const float (&v1)[3][4], float (&p)[3][4], const float (&sA)[6], const float (&sB)[6],
+    auto step = [&](int r, const Row &t, const Row &m, Row &b, const F2 (&v0)[3][2],
+                    const F2 (&v1)[3][2], F2 (&p)[3][2], const float (&sA)[6], const float (&sB)[6],
                     float (&sc)[6], bool someB, bool &someC) {
         const uint32_t cur = next;
         if (r + 1 <= rLast) next = word(r + 1);
@@ -1208,45 +1212,41 @@ k_harris_rows(int W, int H, int rows, const uint8_t *__restrict__ src, int srcSt
             const __half2 gx13 = masked(__hfma2(two, m.d13, __hadd2(t.d13, b.d13)), k13);
             const __half2 gy02 = masked(__hfma2(two, dE, __hadd2(dOm, dO)), k02);
             const __half2 gy13 = masked(__hfma2(two, dO, __hadd2(dE, dEp)), k13);
-            const __half gx[4] = {__low2half(gx02), __low2half(gx13), __high2half(gx02), __high2half(gx13)};
-            const __half gy[4] = {__low2half(gy02), __low2half(gy13), __high2half(gy02), __high2half(gy13)};
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                p[0][c] = product(gx[c], gx[c]);
-                p[1][c] = product(gx[c], gy[c]);
-                p[2][c] = product(gy[c], gy[c]);
-            }
+            p[0][0] = products(gx02, gx02); p[0][1] = products(gx13, gx13);
+            p[1][0] = products(gx02, gy02); p[1][1] = products(gx13, gy13);
+            p[2][0] = products(gy02, gy02); p[2][1] = products(gy13, gy13);
         }
         // window sums at s = g - 1 over gradient rows g-2 .. g (HafCpu_HarrisScore_HVC_HG3_3x3)
-        float sum[3][4];
+        F2 s02[3], s13[3];
 #pragma unroll
         for (int q = 0; q < 3; q++) {
-            float vs[4];
-#pragma unroll
-            for (int c = 0; c < 4; c++) vs[c] = __fadd_rn(__fadd_rn(v0[q][c], v1[q][c]), p[q][c]);
-            const float vl = __shfl_up_sync(0xffffffffu, vs[3], 1), vr = __shfl_down_sync(0xffffffffu, vs[0], 1);
-            const float mid0 = __fadd_rn(vs[0], vs[1]), mid1 = __fadd_rn(vs[2], vs[3]);
-            sum[q][0] = __fadd_rn(vl, mid0);
-            sum[q][1] = __fadd_rn(mid0, vs[2]);
-            sum[q][2] = __fadd_rn(vs[1], mid1);
-            sum[q][3] = __fadd_rn(mid1, vr);
+            const F2 vs02 = f2_add(f2_add(v0[q][0], v1[q][0]), p[q][0]), vs13 = f2_add(f2_add(v0[q][1], v1[q][1]), p[q][1]);
+            const F2 mid = f2_add(vs02, vs13);             // columns 0 + 1, 2 + 3
+            const float vl = __shfl_up_sync(0xffffffffu, f2_hi(vs13), 1), vr = __shfl_down_sync(0xffffffffu, f2_lo(vs02), 1);
+            s02[q] = f2_add(mid, f2(vl, f2_lo(vs13)));
+            s13[q] = f2_add(mid, f2(f2_hi(vs02), vr));
         }
         const int srow = g - 1;
         const uint32_t scoreNow = srow >= 1 && srow < H - 1 ? scoreCol : 0u;
         bool nonzero = false;
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const float gx2 = sum[0][c], gxy2 = sum[1][c], gy2 = sum[2][c];
-            const float traceA = __fadd_rn(gx2, gy2);
-            const float detA = __fsub_rn(__fmul_rn(gx2, gy2), __fmul_rn(gxy2, gxy2));
-            const float Mc = __fsub_rn(detA, __fmul_rn(__fmul_rn(k, traceA), traceA));
-            float v = 0.f;
-            if (Mc >= least && ((scoreNow >> c) & 1)) {
-                const float q = __fdiv_rn(Mc, norm);
-                v = q > Tc ? q : 0.f;
-                nonzero |= v != 0.f;
+        for (int h = 0; h < 2; h++) {
+            const F2 gx2 = h ? s13[0] : s02[0], gxy2 = h ? s13[1] : s02[1], gy2 = h ? s13[2] : s02[2];
+            const F2 traceA = f2_add(gx2, gy2);
+            // differences as sums with the exact product by -1
+            const F2 detA = f2_fma(f2_fma(gxy2, gxy2, zero2), minus, f2_fma(gx2, gy2, zero2));
+            const F2 M = f2_fma(f2_fma(f2_fma(k2, traceA, zero2), traceA, zero2), minus, detA);
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const float Mc = e ? f2_hi(M) : f2_lo(M);
+                float v = 0.f;
+                if (Mc >= least && ((scoreNow >> (h + 2 * e)) & 1)) {
+                    const float q = __fdiv_rn(Mc, norm);
+                    v = q > Tc ? q : 0.f;
+                    nonzero |= v != 0.f;
+                }
+                sc[1 + h + 2 * e] = v;
             }
-            sc[c + 1] = v;
         }
         someC = __any_sync(0xffffffffu, nonzero);
         sc[0] = sc[5] = 0.f;
@@ -2198,10 +2198,10 @@ static int harris_3x3(void *stream, uint32_t W, uint32_t H, const uint8_t *pSrc,
     const dim3 grd(div_up(strips, 4), div_up(H, rows));
     if (agocuda_u8_tensor_map(&map, pSrc, W, H, srcStride, kHBoxW, rows + 6))
         k_harris_rows<true><<<grd, 128, 0, s>>>((int)W, (int)H, rows, pSrc, (int)srcStride, sensitivity, strengthThreshold,
-                                                normFactor, list, cnt, cap, pStatus, map);
+                                                normFactor, list, cnt, cap, pStatus, 0.f, map);
     else
         k_harris_rows<false><<<grd, 128, 0, s>>>((int)W, (int)H, rows, pSrc, (int)srcStride, sensitivity, strengthThreshold,
-                                                 normFactor, list, cnt, cap, pStatus, map);
+                                                 normFactor, list, cnt, cap, pStatus, 0.f, map);
     agocuda_count_launch(1);
     int rc = agocuda_launch_status();
     if (rc) return rc;
