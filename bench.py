@@ -10,7 +10,7 @@ between steps.  Default workload: Canny (3x3, L1, 80/100) + Harris (3, 3, k 0.04
 min distance 5) on 3840x2160 U8 synthetic scenes.
 
 * value  -- Mpixels/s with the inputs already resident in HBM: the device time of each
-            graph launch (CUDA events the engine records on its own stream), summed over
+            graph launch (clock readings at both ends of the captured graph), summed over
             K steps.  Mpixels counts the pixels of every input image of the graph (one
             per frame; both frames of a pair for the pyramid/LK workload).
 * e2e    -- the same metric through the public OpenVX API with host buffers: per step,
