@@ -81,9 +81,11 @@ __device__ __forceinline__ int best_arc_min(const int d[16])
 // Corner flags of the four pixels of tile word q (columns x0-4+4q ..) of tested row tr (image row
 // y0-1+tr): bit 7 of each byte of `plus` (brighter arc) and `minus`.
 //
-// PACKED (t >= 0): the tests c + t < p and p < c - t in byte lanes, with saturated bounds (a
-// bound of 255 or 0 is never passed, as the unsaturated one); the arcs by ANDs of the 16 circle
-// words.  One pixel at a time takes 16 byte loads and 32 compares each; negative thresholds do.
+// PACKED (0 <= t <= kFtPackedMax): the tests c + t < p and p < c - t in byte lanes, with saturated
+// bounds (a bound of 255 or 0 is never passed, as the unsaturated one); the arcs by ANDs of the 16
+// circle words.  One pixel at a time takes 16 byte loads and 32 compares each; the thresholds that do
+// are negative, or so large that the 16-bit sum c + t can wrap, below every pixel.
+constexpr int kFtPackedMax = 32767 - 255;
 template <bool PACKED>
 __device__ __forceinline__ void fast_flags(const uint8_t (*tile)[kFtSW], int tr, int q, int t, uint32_t &plus, uint32_t &minus)
 {
@@ -352,8 +354,9 @@ extern "C" int agocuda_FastCorners_XY_U8(void *stream, uint32_t W, uint32_t H, c
     const dim3 g1(div_up(W, kFtX), div_up(H, kFtY));
     const unsigned g2 = div_up(H, 8);
     vx_keypoint_like *kp = (vx_keypoint_like *)pCorners;
-    (nonmaxSuppression ? (t >= 0 ? k_fast_tile<true, true> : k_fast_tile<true, false>)
-                       : (t >= 0 ? k_fast_tile<false, true> : k_fast_tile<false, false>))<<<g1, 256, 0, q>>>(
+    const bool packed = t >= 0 && t <= kFtPackedMax;
+    (nonmaxSuppression ? (packed ? k_fast_tile<true, true> : k_fast_tile<true, false>)
+                       : (packed ? k_fast_tile<false, true> : k_fast_tile<false, false>))<<<g1, 256, 0, q>>>(
         (int)W, (int)H, pSrc, (int)srcStride, t, s.map, s.mapStride, s.bitmap, s.words, s.counts);
     k_fast_scan<<<1, 1024, 0, q>>>((int)H, s.tiles, s.counts, s.rowStart, cornerCapacity, pCornerCount, pNumCorners);
     if (nonmaxSuppression)

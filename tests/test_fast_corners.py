@@ -157,16 +157,39 @@ def test_engine_fast_graph(cuda, kind, thr, suppress, W, H):
     _check(V.OpenVX(), kind, W, H, thr, suppress, capacity=1 << 18)
 
 
+def _contrast_image(W, H):
+    img = np.random.default_rng(W + H).choice(np.array([0, 1, 127, 128, 254, 255], np.uint8), (H, W), p=[.35, .05, .1, .1, .05, .35])
+    img[2:H - 2, 4:W - 4:9] = 255
+    return img
+
+
 # the byte-lane circle test at the ends of its saturated bounds, on full-contrast pixels, at sizes
-# around the 128x8 tiles and the 1024-pixel steps of a row
+# around the 128x13 tiles: one tile, its first remainders, and a tile that touches no image edge
+TILE_SIZES = [(128, 8), (128, 13), (129, 17), (1040, 23), (400, 45)]
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("W,H", [(128, 8), (129, 17), (1040, 23)])
+@pytest.mark.parametrize("W,H", TILE_SIZES)
 @pytest.mark.parametrize("suppress", [False, True])
 @pytest.mark.parametrize("thr", [0.0, 1.0, 127.0, 254.0, 255.0, 300.0])
 def test_fast_threshold_ends(cuda, agocuda, thr, suppress, W, H):
-    img = np.random.default_rng(W + H).choice(np.array([0, 1, 127, 128, 254, 255], np.uint8), (H, W), p=[.35, .05, .1, .1, .05, .35])
-    img[2:H - 2, 4:W - 4:9] = 255
+    img = _contrast_image(W, H)
     want, want_n = oracle_fast(img, thr, suppress, 1 << 16)
+    got, _, n = _kernel(agocuda, img, thr, suppress, 1 << 16)
+    assert n == want_n
+    np.testing.assert_array_equal(got, want)
+
+
+# thresholds that the byte lanes cannot hold: negative ones, and those from 32513 on, where the 16-bit
+# sum of pixel and threshold wraps and every circle pixel counts as brighter
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", TILE_SIZES)
+@pytest.mark.parametrize("suppress,thr", [(False, -1.0), (False, -300.0), (False, 32512.0), (False, 32513.0), (False, 32600.0),
+                                          (False, 32767.0), (True, -1.0), (True, -300.0), (True, 32512.0)])
+def test_fast_thresholds_of_16_bits(cuda, agocuda, thr, suppress, W, H):
+    img = _contrast_image(W, H)
+    want, want_n = oracle_fast(img, thr, suppress, 1 << 16)
+    assert (want_n > 0) == (thr != 32512.0)
     got, _, n = _kernel(agocuda, img, thr, suppress, 1 << 16)
     assert n == want_n
     np.testing.assert_array_equal(got, want)
