@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) k_fast_tile(int W, int H, const uint8_t *
             if (e & 0x4000) {
 #pragma unroll
                 for (int k = 0; k < 16; k++) d[k] = (int)tile[3 + tr + kCircleDy[k]][c + kCircleDx[k]] - v;
-                sp = best_arc_min(d) - 1;
+                sp = max(best_arc_min(d) - 1, t);          // t: the search's lower end, reached where c + t wraps
             }
             if (e & 0x8000) {
 #pragma unroll

@@ -185,7 +185,8 @@ def test_fast_threshold_ends(cuda, agocuda, thr, suppress, W, H):
 @pytest.mark.gpu
 @pytest.mark.parametrize("W,H", TILE_SIZES)
 @pytest.mark.parametrize("suppress,thr", [(False, -1.0), (False, -300.0), (False, 32512.0), (False, 32513.0), (False, 32600.0),
-                                          (False, 32767.0), (True, -1.0), (True, -300.0), (True, 32512.0)])
+                                          (False, 32767.0), (True, -1.0), (True, -300.0), (True, 32512.0), (True, 32513.0),
+                                          (True, 32600.0), (True, 32767.0)])
 def test_fast_thresholds_of_16_bits(cuda, agocuda, thr, suppress, W, H):
     img = _contrast_image(W, H)
     want, want_n = oracle_fast(img, thr, suppress, 1 << 16)
