@@ -99,6 +99,7 @@ static uint64_t param_signature(Graph *g)
         case VX_TYPE_IMAGE: {
             Image *img = IMG(r);
             h = mix(h, &img->valid, sizeof(img->valid));
+            for (const Image *i = img; i; i = i->parent) h = mix(h, &i->handle_version, 8);
             for (int i = 0; i < img->num_planes; i++) h = mix(h, &img->planes[i].dev, sizeof(void *));
             break;
         }

@@ -73,6 +73,7 @@ struct Image : Ref {
     bool uniform = false;
     vx_pixel_value_t uniform_value{};
     vx_enum import_type = VX_MEMORY_TYPE_NONE;  // HOST / HIP(device) for images from handle
+    uint64_t handle_version = 0;      // counts vxSwapImageHandle calls: captured copies hold the pointers of one
     Image *parent = nullptr;          // pyramid/channel parent (shares memory)
     Image *view_of = nullptr;         // image this ROI / channel view holds an internal reference on
     std::vector<Image *> views;       // ROI views of this image (vxCreateImageFromROI): share its storage

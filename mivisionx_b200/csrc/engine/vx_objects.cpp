@@ -770,8 +770,8 @@ vx_status vxSwapImageHandle(vx_image image, void *const new_ptrs[], void *prev_p
     image_refresh_views(img);
     if (img->import_type == VX_MEMORY_TYPE_HOST) { img->host_valid = new_ptrs != nullptr; img->dev_valid = false; }
     else img->dev_valid = new_ptrs != nullptr;
-    // pointers are baked into captured launches: graphs using this image re-capture
-    for (Ref *r : img->ctx->refs) if (r->type == VX_TYPE_GRAPH && r->magic == kMagic) static_cast<Graph *>(r)->param_signature ^= 1;
+    // pointers are baked into captured launches: no plan made before is used again with this image
+    img->handle_version++;
     return VX_SUCCESS;
 }
 

@@ -73,6 +73,60 @@ def test_swap_handle_recaptures(cuda):
     _check_cfg2(out.numpy(), api.array_items(g.corners[0]), api.read_scalar(g.num[0]), fb)
 
 
+def _swap(api, img, t):
+    new, prev = (C.c_void_p * 1)(t.data_ptr()), (C.c_void_p * 1)()
+    api.ok(api.vxSwapImageHandle(img, new, prev, 1), "swap")
+
+
+@pytest.mark.parametrize("swaps", ["input and output", "input twice"])
+def test_two_swaps_before_an_execution(cuda, swaps):
+    """Every swap counts, an even number of them too.  All buffers outlive the graph."""
+    api = V.OpenVX()
+    ctx = api.obj(api.vxCreateContext(), "context")
+    w, h = 640, 480
+    ins, outs = [pinned(h, w) for _ in range(3)], [pinned(h, w) for _ in range(2)]
+    scenes = [_scene(20 + i, w, h) for i in range(3)]
+    for t, s in zip(ins, scenes):
+        t.numpy()[:] = s
+    g = WL.Cfg2Graph(api, ctx, [(w, h)], host_io={"src": [ins[0].numpy()], "edge": [outs[0].numpy()]})
+    g.run()
+    _swap(api, g.inputs[0], ins[1])
+    if swaps == "input and output":
+        _swap(api, g.edges[0], outs[1])
+        out, scene = outs[1], scenes[1]
+    else:
+        _swap(api, g.inputs[0], ins[2])
+        out, scene = outs[0], scenes[2]
+    for t in outs:
+        t.zero_()
+    g.run()
+    _check_cfg2(out.numpy(), api.array_items(g.corners[0]), api.read_scalar(g.num[0]), scene)
+
+
+def test_swap_reaches_plans_made_before(cuda):
+    """A graph over a delay has a plan per ageing phase at hand; after a swap it must not go back
+    to one that holds the old buffer."""
+    api = V.OpenVX()
+    ctx = api.obj(api.vxCreateContext(), "context")
+    w, h = 160, 64
+    ins, out = [pinned(h, w) for _ in range(2)], pinned(h, w)
+    for i, t in enumerate(ins):
+        t.fill_(10 + i)
+    src, dst = api.image_from_host(ctx, ins[0].numpy()), api.image_from_host(ctx, out.numpy())
+    d = api.obj(api.vxCreateDelay(ctx, api.obj(api.vxCreateImage(ctx, w, h, V.VX_DF_IMAGE_U8), "image"), 2), "delay")
+    for k in range(2):
+        api.write_plane(api.vxGetReferenceFromDelay(d, -k), np.full((h, w), k, np.uint8))
+    g = api.obj(api.vxCreateGraph(ctx), "graph")
+    api.obj(api.vxAbsDiffNode(g, src, api.vxGetReferenceFromDelay(d, 0), dst), "node")
+    api.ok(api.vxVerifyGraph(g), "verify")
+    for want in (10, 9, 11):
+        if want == 11:
+            _swap(api, src, ins[1])
+        api.ok(api.vxProcessGraph(g), "process")
+        assert (out.numpy() == want).all()
+        api.ok(api.vxAgeDelay(d), "age")
+
+
 def test_cfg1_host_buffers_and_pageable_fallback(cuda):
     """Batched chain (one launch for all frames) with page-locked buffers, and the same graph
     over pageable numpy buffers, which take the synchronous copy path."""
