@@ -73,6 +73,27 @@ def test_swap_handle_recaptures(cuda):
     _check_cfg2(out.numpy(), api.array_items(g.corners[0]), api.read_scalar(g.num[0]), fb)
 
 
+def test_cfg2_large_host_buffers(cuda):
+    """Frames above 6 MB: uploads follow one another and each download waits for an upload that it
+    does not need.  Six frames, and six again with other inputs in the same buffers."""
+    api = V.OpenVX()
+    ctx = api.obj(api.vxCreateContext(), "context")
+    w, h = 2560, 2560
+    scenes = [WL.cfg2_scene(seed=40 + i, width=w, height=h) for i in range(3)]
+    want = [(OC.canny(s)[0], *OC.harris(s, capacity=32768)) for s in scenes]
+    ins, outs = [pinned(h, w) for _ in range(6)], [pinned(h, w) for _ in range(6)]
+    g = WL.Cfg2Graph(api, ctx, [(w, h)] * 6, host_io={"src": [t.numpy() for t in ins], "edge": [t.numpy() for t in outs]})
+    for rnd in range(2):
+        for i, t in enumerate(ins):
+            t.numpy()[:] = scenes[(i + rnd) % 3]
+        g.run()
+        for i, t in enumerate(outs):
+            edges, corners, num = want[(i + rnd) % 3]
+            np.testing.assert_array_equal(t.numpy()[1:h - 1, 1:w - 1], edges[1:h - 1, 1:w - 1])
+            assert api.read_scalar(g.num[i]) == num
+            np.testing.assert_array_equal(api.array_items(g.corners[i]).view(OC.KP), corners)
+
+
 def _swap(api, img, t):
     new, prev = (C.c_void_p * 1)(t.data_ptr()), (C.c_void_p * 1)()
     api.ok(api.vxSwapImageHandle(img, new, prev, 1), "swap")
