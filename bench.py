@@ -10,7 +10,7 @@ between steps.  Default workload: Canny (3x3, L1, 80/100) + Harris (3, 3, k 0.04
 min distance 5) on 3840x2160 U8 synthetic scenes.
 
 * value  -- Mpixels/s with the inputs already resident in HBM: the device time of each
-            graph launch (clock readings at both ends of the captured graph), summed over
+            graph launch (CUDA events on the graph's stream, one on each side of it), summed over
             K steps.  Mpixels counts the pixels of every input image of the graph (one
             per frame; both frames of a pair for the pyramid/LK workload).
 * e2e    -- the same metric through the public OpenVX API with host buffers: per step,
@@ -393,6 +393,20 @@ def run_reference_arm(a, wl_name):
 
 
 # ------------------------------------------------------------------------------------------
+def device_steps(api, g, steps):
+    """Device milliseconds of each of `steps` executions of a graph: CUDA events on its stream."""
+    import torch
+    stream = torch.cuda.ExternalStream(api.node_stream(g.node))
+    events = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(steps)]
+    for e0, e1 in events:
+        e0.record(stream)
+        api.ok(api.vxScheduleGraph(g.graph), "schedule")
+        e1.record(stream)
+        api.ok(api.vxWaitGraph(g.graph), "wait")
+    torch.cuda.synchronize()
+    return [e0.elapsed_time(e1) for e0, e1 in events]
+
+
 def device_value(api, wl, B, plain, steps, warmup, ws, rank, local):
     """Device-resident Mpixels/s of `B` frames of workload `wl` in one graph (fused+batched,
     or the plain one-launch-per-node form), in a context of its own that is released after:
@@ -413,11 +427,7 @@ def device_value(api, wl, B, plain, steps, warmup, ws, rank, local):
             g.run()
         torch.cuda.synchronize()
         _barrier(ws)
-        ms = []
-        for _ in range(steps):
-            g.run()
-            ms.append(api.gpu_ms_last(g.graph))
-        torch.cuda.synchronize()
+        ms = device_steps(api, g, steps)
         _barrier(ws)
         ms_step = _max_over_ranks(sum(ms), ws) / steps
         px = sum(int(f.shape[0] * f.shape[1]) for f in frames)
@@ -518,12 +528,8 @@ def run_ours(a, wl_name):
         g.run()
     torch.cuda.synchronize()
     _barrier(ws)
-    gpu_ms = []
     with ClockSampler(local) as clk:
-        for _ in range(a.steps):
-            g.run()
-            gpu_ms.append(api.gpu_ms_last(g.graph))
-        torch.cuda.synchronize()
+        gpu_ms = device_steps(api, g, a.steps)
     _barrier(ws)
     ms_step = _max_over_ranks(sum(gpu_ms), ws) / a.steps
     px_step = sum(int(f.shape[0] * f.shape[1]) for f in frames)   # input pixels of the first node

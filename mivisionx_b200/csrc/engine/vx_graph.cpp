@@ -967,8 +967,9 @@ vx_status vxQueryGraph(vx_graph graph, vx_enum attribute, void *ptr, vx_size siz
         memset(ptr, 0, size); ((AgoTargetAffinityInfo *)ptr)->device_type = AGO_TARGET_AFFINITY_GPU; return VX_SUCCESS;
     case VX_GRAPH_ATTRIBUTE_AMD_PERFORMANCE_INTERNAL_LAST: case VX_GRAPH_ATTRIBUTE_AMD_PERFORMANCE_INTERNAL_AVG: {
         // vx_api.cpp:3106: AgoGraphPerfInternalInfo in nanoseconds; kernel_wait is the device
-        // time of the launch (CUDA events around the captured graph), last or averaged; the
-        // host<->device copies happen inside that launch, so the buffer times stay 0
+        // time of the execution from its first node to its last (clock readings inside the captured
+        // graph; without one, CUDA events around the steps), last or averaged; the host<->device
+        // copies happen inside, so the buffer times stay 0
         if (size != sizeof(AgoGraphPerfInternalInfo) || !ptr) return VX_ERROR_INVALID_PARAMETERS;
         AgoGraphPerfInternalInfo p{};
         if (attribute == VX_GRAPH_ATTRIBUTE_AMD_PERFORMANCE_INTERNAL_LAST) p.kernel_wait = (vx_uint64)(g->gpu_ms_last * 1e6);
@@ -978,7 +979,7 @@ vx_status vxQueryGraph(vx_graph graph, vx_enum attribute, void *ptr, vx_size siz
     case VX_GRAPH_ATTRIBUTE_AMD_PERFORMANCE_INTERNAL_PROFILE: {
         // ago_interface.cpp:2740 layout: a header and one line per timed object; the nodes of
         // this target run inside one captured CUDA graph, so the lines are the graph's host
-        // time (vxProcessGraph) and its device time (CUDA events around the launch)
+        // time (vxProcessGraph) and its device time (as kernel_wait above)
         const char *file = (const char *)ptr;
         FILE *fp = (!file || !strcmp(file, "stdout")) ? stdout : fopen(file, "w");
         if (!fp) return VX_FAILURE;

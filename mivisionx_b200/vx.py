@@ -371,6 +371,12 @@ class OpenVX:
         self.lib.vxSetContextAttribute.argtypes = [vp, i32, vp, sz]
         self.ok(self.lib.vxSetContextAttribute(ctx, attr, C.byref(v), 4), "set device")
 
+    def node_stream(self, node) -> int:
+        """The CUDA stream that the node's verified graph launches on."""
+        s = C.c_void_p()
+        self.ok(self.vxQueryNode(node, VX_NODE_ATTRIBUTE_AMD_HIP_STREAM, C.byref(s), C.sizeof(s)), "stream")
+        return s.value
+
     def gpu_ms_last(self, graph) -> float:
         """Device time of the graph's last launch (CUDA events on its stream), in ms."""
         p = AgoGraphPerfInternalInfo()

@@ -222,7 +222,7 @@ class Cfg1Graph:
                       a.vxMagnitudeNode(g, gx, gy, mag),
                       a.vxConvertDepthNode(g, mag, dep, V.VX_CONVERT_POLICY_SATURATE, self.shift),
                       a.vxThresholdNode(g, dep, self.thr, dst)):
-                a.obj(n, "node")
+                self.node = a.obj(n, "node")
             self.inputs.append(src)
             self.outputs.append(dst)
         a.ok(a.vxVerifyGraph(g), "vxVerifyGraph")
@@ -284,7 +284,7 @@ class MotionGraph:
             for n in (a.vxAbsDiffNode(g, cur, prev, v[0]), a.vxGaussian3x3Node(g, v[0], v[1]),
                       a.vxThresholdNode(g, v[1], self.thr, v[2]), a.vxDilate3x3Node(g, v[2], v[3]),
                       a.vxErode3x3Node(g, v[3], v[4]), a.vxMedian3x3Node(g, v[4], dst)):
-                a.obj(n, "node")
+                self.node = a.obj(n, "node")
             self.inputs += [prev, cur]
             self.outputs.append(dst)
         a.ok(a.vxVerifyGraph(g), "vxVerifyGraph")
@@ -343,6 +343,7 @@ class Cfg3Graph:
             n2 = a.obj(a.vxWarpAffineNode(g, sb, mat, V.VX_INTERPOLATION_BILINEAR, wb), "node")
             a.set_border(n1, V.VX_BORDER_CONSTANT, 0)
             a.set_border(n2, V.VX_BORDER_CONSTANT, 0)
+            self.node = n2
             self.inputs.append(rgb); self.nv12.append(nv12); self.iyuv.append(iyuv)
             self.scaled.append((sb, sa)); self.warped.append((wn, wb)); self.matrices.append(m)
         a.ok(a.vxVerifyGraph(g), "vxVerifyGraph")
@@ -397,7 +398,7 @@ class Cfg2Graph:
             arr = a.obj(a.vxCreateArray(ctx, V.VX_TYPE_KEYPOINT, capacity), "array")
             num = a.scalar(ctx, V.VX_TYPE_SIZE, 0)
             a.obj(a.vxCannyEdgeDetectorNode(g, src, self.hyst, 3, V.VX_NORM_L1, edge), "canny node")
-            a.obj(a.vxHarrisCornersNode(g, src, self.s_strength, self.s_mind, self.s_k, 3, 3, arr, num), "harris node")
+            self.node = a.obj(a.vxHarrisCornersNode(g, src, self.s_strength, self.s_mind, self.s_k, 3, 3, arr, num), "harris node")
             self.inputs.append(src); self.edges.append(edge); self.corners.append(arr); self.num.append(num)
         a.ok(a.vxVerifyGraph(g), "vxVerifyGraph")
 
@@ -450,8 +451,8 @@ class Cfg4Graph:
             out = a.obj(a.vxCreateArray(ctx, V.VX_TYPE_KEYPOINT, capacity), "array")
             a.obj(a.vxGaussianPyramidNode(g, i0, p0), "pyramid node")
             a.obj(a.vxGaussianPyramidNode(g, i1, p1), "pyramid node")
-            a.obj(a.vxOpticalFlowPyrLKNode(g, p0, p1, pts, pts, out, term, self.s_eps, self.s_iter, self.s_est, window),
-                  "optical flow node")
+            self.node = a.obj(a.vxOpticalFlowPyrLKNode(g, p0, p1, pts, pts, out, term, self.s_eps, self.s_iter, self.s_est, window),
+                              "optical flow node")
             self.old.append(i0); self.new.append(i1); self.pts.append(pts); self.out.append(out)
             self.pyr.append((p0, p1))
         a.ok(a.vxVerifyGraph(g), "vxVerifyGraph")
