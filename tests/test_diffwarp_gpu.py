@@ -174,9 +174,18 @@ def test_perspective_degenerate_rows(cuda):
     assert torch.isfinite(tht.grad).all() and torch.isfinite(src.grad).all()
 
 
-# sizes around the 32-column, 1..16-row strips of a warp; maps whose neighbouring samples share
-# taps (unit scale), skip columns (2.5), sit on one cell (0.2), run backwards or leave the source
-@pytest.mark.parametrize("kind", ["shift", "wide", "tight", "mirror", "off"])
+# maps whose neighbouring samples share taps (unit scale), skip columns (2.5), sit on one cell (0.2),
+# run backwards or leave the source
+STRIP_MAPS = ["shift", "wide", "tight", "mirror", "off"]
+
+
+def _strip_map(kind, H, W):
+    return {"shift": [1, 0, 0, 1, 0.3, -0.4], "wide": [2.5, 0.1, -0.1, 2.5, -3.2, 1.1], "tight": [0.2, 0, 0, 0.2, 1.1, 0.6],
+            "mirror": [-1, 0, 0, -1, W - 1.25, H - 1.75], "off": [1, 0, 0, 1, W - 2.5, -H + 1.5]}[kind]
+
+
+# sizes around the 32 columns of a warp's strip; batches this small have strips of one row
+@pytest.mark.parametrize("kind", STRIP_MAPS)
 @pytest.mark.parametrize("H,W", [(1, 1), (1, 40), (2, 33), (17, 31), (67, 130)])
 def test_adjoint_at_strip_edges(cuda, H, W, kind):
     import torch
@@ -186,8 +195,7 @@ def test_adjoint_at_strip_edges(cuda, H, W, kind):
     n = 3
     img = rng.random((n, H, W)).astype(np.float32)
     tgt = rng.random((n, H, W)).astype(np.float32)
-    base = {"shift": [1, 0, 0, 1, 0.3, -0.4], "wide": [2.5, 0.1, -0.1, 2.5, -3.2, 1.1], "tight": [0.2, 0, 0, 0.2, 1.1, 0.6],
-            "mirror": [-1, 0, 0, -1, W - 1.25, H - 1.75], "off": [1, 0, 0, 1, W - 2.5, -H + 1.5]}[kind]
+    base = _strip_map(kind, H, W)
     theta = np.array([base, base, [1.01, 0.02, -0.02, 0.99, 0.1, 0.2]], np.float32)
     d = [torch.from_numpy(a).cuda() for a in (img, theta, tgt)]
     loss, gsrc, gth = diffwarp.warp_affine_l2_step(*d)
@@ -205,6 +213,48 @@ def test_adjoint_at_strip_edges(cuda, H, W, kind):
         gs, gf = D.remap_adjoint(img[i].astype(np.float64), f, tgt[i].astype(np.float64))
         assert np.abs(src.grad[i].cpu().numpy() - gs).max() <= 1e-5 * max(np.abs(gs).max(), 1.0)
         assert np.abs(field.grad[i].cpu().numpy() - gf).max() <= 1e-5 * max(np.abs(gf).max(), 1.0)
+
+
+# strips of several rows, where the lower contributions of a row join the upper ones of the next.  A
+# strip has the most rows (up to 32) that leave 32 warps for every SM: the batch sets them.  The rows
+# of each size end in a part strip.
+@pytest.mark.parametrize("kind", STRIP_MAPS)
+@pytest.mark.parametrize("rows", [8, 32])
+@pytest.mark.parametrize("H,W", [(67, 130), (40, 33)])
+def test_adjoint_in_strips_of_many_rows(cuda, H, W, rows, kind):
+    import torch
+
+    from mivisionx_b200 import diffwarp
+    warps = 32 * torch.cuda.get_device_properties(0).multi_processor_count
+    strips = lambda r: -(-W // 32) * -(-H // r)
+    n = -(-warps // strips(rows))
+    assert rows == 32 or n * strips(2 * rows) < warps
+    rng = np.random.default_rng(H + rows)
+    img, tgt = rng.random((n, H, W)).astype(np.float32), rng.random((n, H, W)).astype(np.float32)
+    theta = np.array([_strip_map(kind, H, W)] * n, np.float32)
+    d = [torch.from_numpy(a).cuda() for a in (img, theta, tgt)]
+    loss, gsrc, gth = diffwarp.warp_affine_l2_step(*d)
+    src, th = d[0].clone().requires_grad_(True), d[1].clone().requires_grad_(True)
+    (diffwarp.warp_affine(src, th) * d[2]).sum().backward()
+    ys, xs = np.meshgrid(np.arange(H), np.arange(W), indexing="ij")
+    m = theta[0]
+    at = np.stack([m[0] * xs + m[2] * ys + m[4] - xs, m[1] * xs + m[3] * ys + m[5] - ys], -1).astype(np.float32)
+    field = torch.from_numpy(np.broadcast_to(at, (n, H, W, 2)).copy()).cuda().requires_grad_(True)
+    fsrc = d[0].clone().requires_grad_(True)
+    (diffwarp.remap(fsrc, field) * d[2]).sum().backward()
+    scale = 4 * H * W * max(H, W)          # as above: 1e-6 of each term, terms at most the size of the sum's scale
+    near = lambda a, b: np.abs(a - b).max() <= 1e-5 * max(np.abs(b).max(), 1.0)
+    for i in (0, n // 2, n - 1):
+        _, l, gs, gt = fp64(img, theta, tgt, i)
+        assert abs(float(loss[i]) - l) <= 1e-5 * max(l, 1e-6)
+        assert np.abs(gth[i].cpu().numpy() - gt).max() <= 1e-6 * scale
+        assert near(gsrc[i].cpu().numpy(), gs)
+        gs, gt = D.warp_affine_adjoint(img[i].astype(np.float64), theta[i].astype(np.float64), tgt[i].astype(np.float64))
+        assert near(src.grad[i].cpu().numpy(), gs)
+        assert np.abs(th.grad[i].cpu().numpy() - gt).max() <= 1e-6 * scale
+        gs, gf = D.remap_adjoint(img[i].astype(np.float64), at.astype(np.float64), tgt[i].astype(np.float64))
+        assert near(fsrc.grad[i].cpu().numpy(), gs)
+        assert near(field.grad[i].cpu().numpy(), gf)
 
 
 def test_source_beyond_int_indexes(cuda):
