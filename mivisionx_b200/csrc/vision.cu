@@ -2163,13 +2163,17 @@ static uint32_t harris_list_capacity(uint32_t W, uint32_t H) { return ((W + 1) /
 
 // Rows per strip.  A strip repeats 6 halo rows (three extra steps each end), so 64 rows cost the
 // least work; but each strip is one warp's serial walk (35 us for 64 rows), and one 720p frame
-// has only 132 of them.  The most rows that still give `kHMinWarps` warps over the frames in
-// flight: one 720p frame 8 rows, one 1080p frame 16, 4K frames and batches 64.
-constexpr int kHMinWarps = 888;      // 6 per SM
+// has only 132 of them.  The most rows that still give `kHMinWarps` warps per SM over the frames in
+// flight: one 720p frame 8 rows, one 1080p frame 16, 4K frames and batches 64.  Eight frames count
+// at most: of a larger batch the strips of some meet the other kernels of the rest (12 and 16 frames of
+// 640x480: 125 and 165 us so, 130 and 171 us with 16 counted; no difference at 320x240, 720p, 1080p).
+constexpr int kHMinWarps = 6;
+constexpr uint32_t kHMaxFrames = 8;
 static int harris_rows(int strips, int H, uint32_t framesInFlight)
 {
+    const long long frames = min(framesInFlight, kHMaxFrames), least = (long long)kHMinWarps * agocuda_sm_count();
     int rows = kHRows;
-    while (rows > 8 && (long long)strips * div_up(H, rows) * min(framesInFlight, 8u) < kHMinWarps) rows >>= 1;
+    while (rows > 8 && strips * frames * div_up(H, rows) < least) rows >>= 1;
     return rows;
 }
 
