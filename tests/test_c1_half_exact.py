@@ -51,13 +51,23 @@ def fused_c1_half(img, shift, thr):
     return out
 
 
-@pytest.mark.parametrize("W,H", [(64, 40), (37, 21)])
-def test_half_chain_every_threshold(rng, W, H):
+@pytest.mark.parametrize("W,H", [(64, 40), (37, 21), (130, 66)])
+def test_half_chain_matches_oracle(rng, W, H):
     yy, xx = np.indices((H, W))
     for img in (rng.integers(0, 256, (H, W), dtype=np.uint8), (rng.integers(0, 2, (H, W)) * 255).astype(np.uint8),
+                ((yy + xx) % 2 * 255).astype(np.uint8),          # checkerboard: largest |gx|, |gy|
                 (xx % 2 * 255).astype(np.uint8), ((yy % 3 == 0) * 255).astype(np.uint8)):
-        for shift in range(5):
+        for shift in range(6):
             for thr in range(0, 256, 3):
+                ref, (sx, sy, ex, ey) = OC.cfg1_chain(img, shift, thr)
+                got = fused_c1_half(img, shift, thr)
+                assert np.array_equal(got[sy:ey, sx:ex], ref[sy:ey, sx:ex]), (shift, thr)
+
+
+def test_half_chain_every_threshold_and_shift(rng):
+    for img in (rng.integers(0, 256, (20, 40), dtype=np.uint8), (rng.integers(0, 2, (20, 40)) * 255).astype(np.uint8)):
+        for shift in range(6):
+            for thr in range(256):
                 ref, (sx, sy, ex, ey) = OC.cfg1_chain(img, shift, thr)
                 got = fused_c1_half(img, shift, thr)
                 assert np.array_equal(got[sy:ey, sx:ex], ref[sy:ey, sx:ex]), (shift, thr)
